@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -167,6 +168,16 @@ struct DeviceGlobals {
     void* prog = nullptr;
     std::vector<CoopClassDev> coop;
     std::vector<int> coop_prim_flops, coop_post_flops;
+    // resident blocks per SM of the compiled classes' kernels, plain and
+    // extended (0: not asked yet; every thread finds the same value)
+    std::atomic<int> occupancy[2][vlx::kNumQuartetClasses] = {};
+
+    int resident_blocks(int cls, bool ext)
+    {
+        std::atomic<int>& o = occupancy[ext ? 1 : 0][cls];
+        if (o.load() == 0) o.store(std::max(1, vlx::kQuartetClasses[cls].occupancy(ext ? 1 : 0)));
+        return o.load();
+    }
 };
 
 std::mutex g_dev_mutex;
@@ -444,6 +455,42 @@ struct TaskSet {
     long long quartets = 0, prim_quartets = 0;
 };
 
+// Streams beside a build's own for the class launches that cannot fill the
+// chip (enqueue_ctx), made on first use and owned by a screener or a batch.
+struct SideStreams {
+    static constexpr int kCount = 8;
+    cudaStream_t s[kCount] = {};
+    cudaEvent_t fork = nullptr, join[kCount] = {};
+    bool ready = false;
+
+    int open()
+    {
+        if (ready) return VLX_B200_OK;
+        int least = 0, greatest = 0;
+        VLX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        if (!fork) VLX_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        for (int i = 0; i < kCount; i++) {
+            if (!s[i]) VLX_CUDA(cudaStreamCreateWithPriority(&s[i], cudaStreamNonBlocking, greatest));
+            if (!join[i]) VLX_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
+        }
+        ready = true;
+        return VLX_B200_OK;
+    }
+
+    void close()
+    {
+        for (int i = 0; i < kCount; i++) {
+            if (s[i]) cudaStreamDestroy(s[i]);
+            if (join[i]) cudaEventDestroy(join[i]);
+            s[i] = nullptr;
+            join[i] = nullptr;
+        }
+        if (fork) cudaEventDestroy(fork);
+        fork = nullptr;
+        ready = false;
+    }
+};
+
 int pair_key(int la, int lb) { return (la + lb) * 16 + lb; }
 
 // ket pairs per work item of a warp-cooperative class
@@ -499,6 +546,7 @@ struct vlx_b200_screener {
     float* d_F32 = nullptr;
     std::vector<TaskSet> tasksets;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    SideStreams side;
 };
 
 namespace {
@@ -846,7 +894,8 @@ int ensure_buffers(vlx_b200_screener* s)
     if (!s->d_D) VLX_CUDA(cudaMalloc(&s->d_D, std::max<size_t>(bytes, 8)));
     if (!s->d_F) VLX_CUDA(cudaMalloc(&s->d_F, std::max<size_t>(bytes, 8)));
     if (s->permuted && !s->d_Dint) VLX_CUDA(cudaMalloc(&s->d_Dint, std::max<size_t>(bytes, 8)));
-    return VLX_B200_OK;
+    // with the buffers, so that a later build under stream capture creates nothing
+    return s->side.open();
 }
 
 // The density the class kernels read: the caller's dD (caller's AO order)
@@ -913,6 +962,7 @@ struct LaunchCtx {
     float* F32 = nullptr;
     const std::map<int, int>* bps = nullptr;  // per-class caps of resident blocks per SM (compiled classes)
     int bps_try = 0;                          // a cap for every compiled class (autotuning; 0: off)
+    SideStreams* side = nullptr;              // launches that cannot fill the chip run beside the others (null: in turn)
 };
 
 // Enqueues all class kernels of a task set on `st`; the accumulators must be
@@ -950,41 +1000,91 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
     const int nprec = (L.dsh ? L.tau32 > 0.0f : ith32 >= 0) ? 2 : 1;
     const int warps_per_block = vlx::kWarpsPerBlock;
     const int nsm = L.glob->nsm;
+    // One launch per class and precision.  The kernels of a class have one grid
+    // of at most one wave, and a single step of the large classes takes 0.1 to
+    // 1 ms, so a class with fewer items than the chip holds warps lasts that
+    // long however few they are, with most SMs idle: such launches go to the
+    // side streams, the slowest steps (highest angular momentum) first, and
+    // run beside each other and beside the full launches, which stay in turn on
+    // `st` (full launches side by side only share the caches).
+    struct Launch {
+        size_t c;
+        int f, grid, side;
+    };
+    std::vector<Launch> list;
     for (size_t c = 0; c < ts->classes.size(); c++) {
-        ClassTasks& ct = ts->classes[c];
+        const ClassTasks& ct = ts->classes[c];
         if (ct.items.empty()) continue;
-        a.items = ts->d_items + ct.offset;
-        a.nitems = (int)ct.items.size();
-        if (events) VLX_CUDA(cudaEventRecord((*events)[c].first, st));
         for (int f = 0; f < nprec; f++) {
-            FockArgs af = a;
-            af.counter = L.counters + (f ? ts->classes.size() : 0) + c;
-            af.qstat = L.qstat ? L.qstat + (c * 2 + f) * 2 : nullptr;
-            const int fmode = f ? (mode | vlx::MODE_F32) : mode;
+            int wpb = warps_per_block, most = 0;
             if (ct.compiled >= 0) {
-                const auto& e = vlx::kQuartetClasses[ct.compiled];
-                int occ = std::max(1, e.occupancy(vlx::needs_ext(af) ? 1 : 0));
+                int occ = L.glob->resident_blocks(ct.compiled, vlx::needs_ext(a) || L.qstat);
                 if (L.bps_try > 0) {
                     occ = std::min(occ, L.bps_try);
                 } else if (L.bps) {
                     const auto cap = L.bps->find(ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12));
                     if (cap != L.bps->end()) occ = std::min(occ, cap->second);
                 }
-                const int want = (int)((ct.items.size() + warps_per_block - 1) / warps_per_block);
-                e.launch(fmode, af, std::max(1, std::min(want, occ * nsm)), st);
+                most = occ * nsm;
             } else {
                 const CoopClassDev& cc = L.glob->coop[ct.coop];
-                const int wpb = vlx::coop_warps_per_block(cc, f != 0);
-                const int cap = vlx::coop_blocks_per_sm(cc, f != 0) * nsm;
-                const int grid = std::max(1, std::min((int)((ct.items.size() + wpb - 1) / wpb), cap));
-                VLX_CUDA(vlx::launch_coop_quartet(fmode, af, cc, grid, st));
+                wpb = vlx::coop_warps_per_block(cc, f != 0);
+                most = vlx::coop_blocks_per_sm(cc, f != 0) * nsm;
             }
-            if (launches) (*launches)++;
+            const int want = (int)((ct.items.size() + wpb - 1) / wpb);
+            list.push_back({c, f, std::max(1, std::min(want, most)), (L.side && !events && want <= most) ? 0 : -1});
         }
-        VLX_CUDA(cudaGetLastError());
-        if (events) VLX_CUDA(cudaEventRecord((*events)[c].second, st));
     }
-    return VLX_B200_OK;
+    const auto momentum = [&](const Launch& l) {
+        const ClassTasks& ct = ts->classes[l.c];
+        return ct.la + ct.lb + ct.lc + ct.ld;
+    };
+    int nside = 0;
+    for (const Launch& l : list) nside += l.side >= 0;
+    if (nside > 0 && list.size() > 1) {
+        std::stable_sort(list.begin(), list.end(), [&](const Launch& x, const Launch& y) {
+            if ((x.side >= 0) != (y.side >= 0)) return x.side >= 0;
+            return x.side >= 0 && momentum(x) > momentum(y);
+        });
+        const int rc = L.side->open();
+        if (rc) return rc;
+        nside = std::min(nside, SideStreams::kCount);
+        VLX_CUDA(cudaEventRecord(L.side->fork, st));
+        for (int i = 0; i < nside; i++) VLX_CUDA(cudaStreamWaitEvent(L.side->s[i], L.side->fork, 0));
+        for (size_t i = 0; i < list.size() && list[i].side >= 0; i++) list[i].side = (int)(i % nside);
+    } else {
+        nside = 0;
+        for (Launch& l : list) l.side = -1;
+    }
+    int rc = VLX_B200_OK;
+    for (const Launch& l : list) {
+        const ClassTasks& ct = ts->classes[l.c];
+        cudaStream_t ls = l.side >= 0 ? L.side->s[l.side] : st;
+        FockArgs af = a;
+        af.items = ts->d_items + ct.offset;
+        af.nitems = (int)ct.items.size();
+        af.counter = L.counters + (l.f ? ts->classes.size() : 0) + l.c;
+        af.qstat = L.qstat ? L.qstat + (l.c * 2 + l.f) * 2 : nullptr;
+        const int fmode = l.f ? (mode | vlx::MODE_F32) : mode;
+        if (events && l.f == 0) VLX_CUDA(cudaEventRecord((*events)[l.c].first, st));
+        if (ct.compiled >= 0) {
+            vlx::kQuartetClasses[ct.compiled].launch(fmode, af, l.grid, ls);
+        } else {
+            const cudaError_t e = vlx::launch_coop_quartet(fmode, af, L.glob->coop[ct.coop], l.grid, ls);
+            if (e != cudaSuccess && !rc) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
+        }
+        if (launches) (*launches)++;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess && !rc) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
+        if (events && l.f == nprec - 1) VLX_CUDA(cudaEventRecord((*events)[l.c].second, st));
+        if (rc) break;
+    }
+    // `st` waits for the side streams also after a failed launch
+    for (int i = 0; i < nside; i++) {
+        VLX_CUDA(cudaEventRecord(L.side->join[i], L.side->s[i]));
+        VLX_CUDA(cudaStreamWaitEvent(st, L.side->join[i], 0));
+    }
+    return rc;
 }
 
 bool dscr_active(const vlx_b200_screener* s) { return s->dscr_fp32 > 0.0 || s->dscr_skip > 0.0; }
@@ -1030,6 +1130,7 @@ int enqueue_classes(vlx_b200_screener* s, TaskSet* ts, int mode, const double* d
     L.qstat = qstat;
     L.bps = &s->class_bps;
     L.bps_try = s->bps_try;
+    L.side = &s->side;
     if (mode != vlx::MODE_ERI && dscr_active(s)) {
         const int rc = prepare_dscr(s, dD, st);
         if (rc) return rc;
@@ -1384,6 +1485,7 @@ int vlx_b200_screener_destroy(vlx_b200_screener* s)
     if (s->d_Dint) cudaFree(s->d_Dint);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
+    s->side.close();
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return VLX_B200_OK;
@@ -1505,6 +1607,7 @@ int vlx_b200_fock_build_multi(vlx_b200_screener* s, int rank, int nodes, int nde
         L.mol.nao = s->nao;
         for (int l = 0; l <= VLX_LMAX; l++) L.mol.nl[l] = s->nl[l];
         L.dens.n = nd;
+        L.side = &s->side;
         bool chunk_any = false;
         for (int d = 0; d < nd; d++) {
             if (s->permuted) {
@@ -2134,6 +2237,7 @@ struct vlx_b200_batch {
     int run_ith = 0;  // threshold of the build being enqueued
     const double* mols_D = nullptr;  // D of the uploaded per-molecule records
     long long launches = 0;          // kernel launches of one build
+    SideStreams side;
 };
 
 namespace {
@@ -2234,6 +2338,7 @@ int batch_enqueue(vlx_b200_batch* b, TaskSet* ts, bool known, int symmetric, dou
         L.glob = b->glob;
         L.counters = b->d_counters;
         L.mols = b->d_mols;
+        L.side = &b->side;
         const int rc = enqueue_ctx(L, ts, symmetric ? vlx::MODE_FOCK_SYM : vlx::MODE_FOCK_GEN, nullptr, cj, ck,
                                    omega2, b->run_ith, -1, st, launches);
         if (rc) return rc;
@@ -2350,6 +2455,7 @@ int vlx_b200_batch_destroy(vlx_b200_batch* b)
     if (b->d_perm) cudaFree(b->d_perm);
     if (b->d_dint) cudaFree(b->d_dint);
     if (b->d_counters) cudaFree(b->d_counters);
+    b->side.close();
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return VLX_B200_OK;
