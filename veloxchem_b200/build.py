@@ -25,7 +25,9 @@ LIB = PKG / 'lib' / 'libvlx_b200.so'
 INCLUDE = PKG.parent / 'include'
 
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
-NVCC_FLAGS = ARCH + ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC', '--expt-relaxed-constexpr',
+# no -lineinfo: with the recursions inlined into several kernels per class the
+# line tables alone are 300 MB of the library
+NVCC_FLAGS = ARCH + ['-O3', '-std=c++17', '-Xcompiler', '-fPIC', '--expt-relaxed-constexpr',
                      '-I' + str(CSRC), '-I' + str(GEN), '-I' + str(INCLUDE)]
 
 
@@ -55,7 +57,11 @@ def _headers_digest(abi=False):
 
 def _compile(src, obj, hdr):
     stamp = obj.with_suffix('.stamp')
-    key = hdr + hashlib.sha256(src.read_bytes()).hexdigest()[:16]
+    text = src.read_bytes()
+    recursion = src.with_name(src.stem.rsplit('_', 1)[0] + '.inc')  # a class unit includes its recursion
+    if src.parent == GEN and recursion.exists():
+        text += recursion.read_bytes()
+    key = hdr + hashlib.sha256(text).hexdigest()[:16]
     if obj.exists() and stamp.exists() and stamp.read_text() == key:
         return src.name, 0.0, False
     cmd = [nvcc()] + NVCC_FLAGS + ['-c', str(src), '-o', str(obj)]
@@ -90,7 +96,11 @@ def build(jobs=None, lmax=3, verbose=True):
     objs = [OBJ / (s.stem + '.o') for s in sources]
     jobs = jobs or os.cpu_count() or 4
     # the longest units first, so that they do not finish last on one core
-    order = sorted(range(len(sources)), key=lambda k: -sources[k].stat().st_size)
+    def size(src):
+        recursion = src.with_name(src.stem.rsplit('_', 1)[0] + '.inc')
+        return (recursion if recursion.exists() else src).stat().st_size
+
+    order = sorted(range(len(sources)), key=lambda k: -size(sources[k]))
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
         futs = [ex.submit(_compile, sources[k], objs[k], hdr_abi if sources[k].stem in abi_units else hdr)
                 for k in order]

@@ -264,15 +264,18 @@ class ClassGen:
                 w('        double c_%d_%d = 0.0;' % (ie, jf))
         # ket primitives outer: the ket data is per lane (loaded once per ket
         # primitive), the bra data is warp-uniform (broadcast loads)
+        w('#pragma unroll 1')
         w('        for (int pk = 0; pk < kk; pk++) {')
         w('            const double eta = ket.zeta(pk), hie = ket.hiz(pk), kcd = ket.kfac(pk);')
         w('            const double QDx = ket.pbx(pk), QDy = ket.pby(pk), QDz = ket.pbz(pk);')
         w('            const double Qx = ket.px(pk), Qy = ket.py(pk), Qz = ket.pz(pk);')
+        w('#pragma unroll 1')
         w('            for (int pb = 0; pb < kb; pb++) {')
-        w('                const double zeta = bra.zeta(pb), hiz = bra.hiz(pb), kab = bra.kfac(pb);')
-        w('                const double PBx = bra.pbx(pb), PBy = bra.pby(pb), PBz = bra.pbz(pb);')
-        w('                const double PQx = bra.px(pb) - Qx, PQy = bra.py(pb) - Qy, PQz = bra.pz(pb) - Qz;')
-        w('                const double r = rsqrt(zeta + eta);')
+        w('                const auto br = bra.rec(pb);')
+        w('                const double zeta = br.zeta, hiz = br.hiz, kab = br.kfac;')
+        w('                const double PBx = br.pbx, PBy = br.pby, PBz = br.pbz;')
+        w('                const double PQx = br.px - Qx, PQy = br.py - Qy, PQz = br.pz - Qz;')
+        w('                const double r = rsqrt_pos(zeta + eta);')
         w('                const double inv = r * r;')
         w('                const double rz = eta * inv, rh = zeta * inv;')
         w('                const double rho = zeta * rz;')
@@ -581,7 +584,7 @@ def to_f32(method_lines):
         t = t.replace('double* __restrict__ out', 'float* __restrict__ out')
         t = t.replace('const double ', 'const float ').replace('double c_', 'float c_').replace('double F[', 'float F[')
         t = t.replace('double h_', 'float h_')
-        t = t.replace('boys_scaled<', 'boys_scaled_f<').replace('rsqrt(', 'rsqrtf(')
+        t = t.replace('boys_scaled<', 'boys_scaled_f<').replace('rsqrt_pos(', 'rsqrtf(')
         t = re.sub(r'(?<![r\w])sqrt\(', 'sqrtf(', t)
         t = re.sub(r'\bdouble (Tb|sc|s2|sm)\b', r'float \1', t)
         if not t.lstrip().startswith('//'):
@@ -623,7 +626,15 @@ def class_name(c):
     return '%d%d%d%d' % c
 
 
+def write_if_changed(path, text):
+    if not path.exists() or path.read_text() != text:
+        path.write_text(text)
+
+
 def emit_class_file(cls, outdir):
+    """class_<name>.inc (traits and recursion) and one translation unit per
+    kernel variant (KernelVariant in vlx_kernels.cuh), compiled in parallel."""
+    cls = tuple(cls)
     g = ClassGen(*cls)
     la, lb, lc, ld = cls
     nm = class_name(cls)
@@ -632,43 +643,38 @@ def emit_class_file(cls, outdir):
     w('// Generated by gen_eri.py -- do not edit.')
     w('#include "vlx_kernels.cuh"')
     w('namespace vlx {')
-    w('template <> struct BlocksHint<%d, %d, %d, %d> { static constexpr int value = %d; };'
-      % (cls + (BLOCKS_HINT.get(tuple(cls), 0),)))
+    for v in range(NUM_VARIANTS):
+        w('template <> struct BlocksHint<%d, %d, %d, %d, %d> { static constexpr int value = %d; };'
+          % (cls + (v, BLOCKS_HINT[v].get(cls, 0))))
     w('template <> struct StageBra<%d, %d, %d, %d> { static constexpr bool value = %s; };'
-      % (cls + ('true' if tuple(cls) in STAGE_BRA else 'false',)))
-    w('template <> struct AccumulateJ<%d, %d, %d, %d> { static constexpr int value = %d; };'
-      % (cls + (ACCUM_J.get(tuple(cls), 0),)))
+      % (cls + ('true' if cls in STAGE_BRA else 'false',)))
+    for gen in (0, 1):
+        w('template <> struct RowStore<%d, %d, %d, %d, %s> { static constexpr int acc = %d, dc = %d; };'
+          % (cls + ('true' if gen else 'false',) + row_store(cls, gen)))
     w(g.emit(parts=class_parts(cls)))
-    w('')
-    w('void launch_quartet_%s(int mode, const FockArgs& a, int grid, cudaStream_t st)' % nm)
-    w('{')
-    w('    const dim3 blk(32 * kWarpsPerBlock);')
-    w('    if (needs_ext(a))')
-    w('        quartet_kernel_of<%d, %d, %d, %d, true>()<<<grid, blk, 0, st>>>(a, mode);' % cls)
-    w('    else')
-    w('        quartet_kernel_of<%d, %d, %d, %d, false>()<<<grid, blk, 0, st>>>(a, mode);' % cls)
-    w('}')
-    w('int occupancy_quartet_%s(int ext)' % nm)
-    w('{')
-    w('    int n = 0;')
-    w('    if (ext)')
-    w('        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, quartet_kernel_of<%d, %d, %d, %d, true>(), 32 * kWarpsPerBlock, 0);' % cls)
-    w('    else')
-    w('        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, quartet_kernel_of<%d, %d, %d, %d, false>(), 32 * kWarpsPerBlock, 0);' % cls)
-    w('    return n;')
-    w('}')
-    if (la, lb) == (lc, ld):
-        w('void launch_schwarz_%d%d(const PairBlockDev* blocks, int bid, int npairs, const double* boys, double* maxv, cudaStream_t st)' % (la, lb))
-        w('{')
-        w('    if (npairs > 0) schwarz_kernel<%d, %d><<<(npairs + 63) / 64, 64, 0, st>>>(blocks, bid, boys, maxv);' % (la, lb))
-        w('}')
     w('}  // namespace vlx')
-    text = '\n'.join(body) + '\n'
-    path = outdir / ('class_%s.cu' % nm)
-    if not path.exists() or path.read_text() != text:
-        path.write_text(text)
-    return path, g.stats()
+    write_if_changed(outdir / ('class_%s.inc' % nm), '\n'.join(body) + '\n')
+    for v in range(NUM_VARIANTS):
+        unit = ['// Generated by gen_eri.py -- do not edit.', '#include "class_%s.inc"' % nm, 'namespace vlx {',
+                'void launch_quartet_%s_%d(int mode, const FockArgs& a, int grid, cudaStream_t st)' % (nm, v),
+                '{',
+                '    launch_quartet<%d, %d, %d, %d, %d>(mode, a, grid, st);' % (cls + (v,)),
+                '}',
+                'int occupancy_quartet_%s_%d(bool f32) { return occupancy_quartet<%d, %d, %d, %d, %d>(f32); }'
+                % ((nm, v) + cls + (v,))]
+        if (la, lb) == (lc, ld) and v == 0:
+            unit += ['void launch_schwarz_%d%d(const PairBlockDev* blocks, int bid, int npairs, const double* boys, '
+                     'double* maxv, cudaStream_t st)' % (la, lb), '{',
+                     '    if (npairs > 0) schwarz_kernel<%d, %d><<<(npairs + 63) / 64, 64, 0, st>>>(blocks, bid, boys, '
+                     'maxv);' % (la, lb), '}']
+        unit.append('}  // namespace vlx')
+        write_if_changed(outdir / ('class_%s_%d.cu' % (nm, v)), '\n'.join(unit) + '\n')
+    return g.stats()
 
+
+# kernel variants of a class (KernelVariant): row items and pair items, each
+# for symmetric and general densities
+NUM_VARIANTS = 4
 
 VRR_COMPILED_MAX = 2400
 ACC_COMPILED_MAX = 180
@@ -698,7 +704,8 @@ GROUPED = {(1, 2, 1, 2): 5, (1, 3, 0, 3): 5, (1, 3, 1, 1): 5, (1, 3, 1, 2): 6, (
 # returned value, (pp|ss) 6, (sd|ss) 8 and (sp|sp) 6 measured 1-13% faster
 # than 4, 5 and 5; higher minimums for (sp|ss), (pp|sp) and (sd|sp) were
 # slower (up to 1.8x).
-BLOCKS_HINT = {(1, 1, 0, 0): 6, (0, 1, 0, 1): 6, (0, 2, 0, 0): 8, (0, 1, 0, 0): 8, (1, 1, 0, 1): 4, (0, 2, 0, 1): 4}
+PAIRS_BLOCKS = {(1, 1, 0, 0): 6, (0, 1, 0, 1): 6, (0, 2, 0, 0): 8, (0, 1, 0, 0): 8, (1, 1, 0, 1): 4, (0, 2, 0, 1): 4}
+BLOCKS_HINT = ({}, {}, PAIRS_BLOCKS, PAIRS_BLOCKS)
 
 # Classes whose bra primitive records are staged in shared memory per work
 # item: measured faster staged on the (H2O)32 / def2-SVP build ((ss|ss)
@@ -707,16 +714,18 @@ BLOCKS_HINT = {(1, 1, 0, 0): 6, (0, 1, 0, 1): 6, (0, 2, 0, 0): 8, (0, 1, 0, 0): 
 STAGE_BRA = {(0, 0, 0, 0), (0, 1, 0, 0), (1, 1, 0, 0), (0, 2, 0, 0), (2, 2, 1, 2)}
 
 
-# Classes whose plain kernels sum the J elements of the bra block F_PQ per
-# work item (1: in registers, 2: in a per-warp shared-memory array) instead of
-# one warp sum and atomic add per 32-ket step (absent: per step).  Chosen per
-# class from timings of all three forms on the (H2O)32 / def2-SVP and
-# (H2O)64 / def2-TZVP builds (gains 3-12% per class; (sp|ss), (sp|sp),
-# (ss|ss), (pd|pd), (pd|pp), (sf|sf), (sf|pp) measured neutral or slower and
-# stay per step).
-ACCUM_J = {(1, 1, 0, 1): 1, (1, 2, 0, 1): 2, (1, 1, 0, 0): 2, (0, 2, 0, 1): 2, (0, 2, 1, 1): 2, (0, 2, 0, 0): 2,
-           (1, 1, 1, 1): 2, (1, 2, 0, 2): 2, (1, 2, 0, 0): 1, (0, 3, 0, 1): 2, (0, 3, 1, 2): 1, (0, 3, 0, 0): 2,
-           (0, 3, 0, 2): 2}
+# Where the row-item kernels keep an item's accumulators and elements of D
+# (RowStore in vlx_kernels.cuh) for the classes that differ from row_store's
+# rule: class -> (acc, dc), for symmetric and general densities.
+ROW_STORE = ({(1, 2, 1, 1): (2, 1)}, {})
+
+
+def row_store(cls, gen):
+    if tuple(cls) in ROW_STORE[gen]:
+        return ROW_STORE[gen][tuple(cls)]
+    nb, nc, nd = (2 * l + 1 for l in cls[1:])
+    n = nb * (nc + nd) * (2 if gen else 1) + nc * nd
+    return (2, 2) if n <= 39 else (0, 0)
 
 
 def class_parts(cls):
@@ -736,18 +745,24 @@ def is_compiled(cls):
 def emit_dispatch(compiled, lmax, outdir):
     lines = ['// Generated by gen_eri.py -- do not edit.', '#pragma once', 'namespace vlx {']
     for c in compiled:
-        nm = class_name(c)
-        lines.append('void launch_quartet_%s(int mode, const FockArgs& a, int grid, cudaStream_t st);' % nm)
-        lines.append('int occupancy_quartet_%s(int mode);' % nm)
+        for v in range(NUM_VARIANTS):
+            nm = '%s_%d' % (class_name(c), v)
+            lines.append('void launch_quartet_%s(int mode, const FockArgs& a, int grid, cudaStream_t st);' % nm)
+            lines.append('int occupancy_quartet_%s(bool f32);' % nm)
     schw = [(a, b) for (a, b) in pair_classes(lmax) if (a, b, a, b) in compiled]
     for (a, b) in schw:
         lines.append('void launch_schwarz_%d%d(const PairBlockDev* blocks, int bid, int npairs, const double* boys, double* maxv, cudaStream_t st);' % (a, b))
-    lines.append('struct QuartetClassEntry { int la, lb, lc, ld; void (*launch)(int, const FockArgs&, int, cudaStream_t); int (*occupancy)(int); int prim_flops, post_flops; };')
+    lines.append('struct QuartetClassEntry { int la, lb, lc, ld; '
+                 'void (*launch[%d])(int, const FockArgs&, int, cudaStream_t); int (*occupancy[%d])(bool); '
+                 'int prim_flops, post_flops; };' % (NUM_VARIANTS, NUM_VARIANTS))
     lines.append('static const QuartetClassEntry kQuartetClasses[] = {')
     for c in compiled:
         nm = class_name(c)
         fv, fa, fp = ClassGen(*c).flops()
-        lines.append('    {%d, %d, %d, %d, launch_quartet_%s, occupancy_quartet_%s, %d, %d},' % (c + (nm, nm, fv + fa, fp)))
+        each = range(NUM_VARIANTS)
+        lines.append('    {%d, %d, %d, %d, {%s}, {%s}, %d, %d},'
+                     % (c + (', '.join('launch_quartet_%s_%d' % (nm, v) for v in each),
+                             ', '.join('occupancy_quartet_%s_%d' % (nm, v) for v in each), fv + fa, fp)))
     lines.append('};')
     lines.append('static const int kNumQuartetClasses = %d;' % len(compiled))
     lines.append('struct SchwarzEntry { int la, lb; void (*launch)(const PairBlockDev*, int, int, const double*, double*, cudaStream_t); };')
@@ -930,8 +945,9 @@ def main():
     emit_xforms(outdir, lmax, interp)
     import gen_coop
     gen_coop.emit_blob(interp, outdir / 'coop_programs.bin')
-    for p in outdir.glob('class_*.cu'):
-        if tuple(int(ch) for ch in p.stem[6:]) not in compiled:
+    for p in list(outdir.glob('class_*.cu')) + list(outdir.glob('class_*.inc')):
+        name = p.stem[6:].split('_')
+        if tuple(int(ch) for ch in name[0]) not in compiled or (p.suffix == '.cu' and len(name) != 2):
             p.unlink()
     print('compiled classes:', len(compiled), 'warp-cooperative classes:', len(interp))
 

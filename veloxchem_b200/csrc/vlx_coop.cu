@@ -43,12 +43,14 @@ template <typename R>
 __device__ __forceinline__ R boys_one(const int m, const R T, const R* __restrict__ tab)
 {
     if (T < (R)BOYS_TMAX) {
-        const int it = (int)(T * (R)BOYS_INV_H);
-        const R x = (R)(2.0 * BOYS_INV_H) * T - (R)(2 * it + 1);
-        const R* c = tab + ((size_t)(m * BOYS_NINT + it)) * BOYS_NCOEF;
-        R p = __ldg(c + BOYS_NCOEF - 1);
+        constexpr bool f32 = sizeof(R) == sizeof(float);
+        constexpr int nc = f32 ? BOYS_NCOEF_F : BOYS_NCOEF, stride = f32 ? BOYS_STRIDE_F : BOYS_STRIDE;
+        const int it = (int)(T * (R)BOYS_INV_H + (R)0.5);
+        const R x = (R)(2 * BOYS_INV_H) * T - (R)(2 * it);
+        const R* c = tab + m * stride + it * nc;
+        R p = __ldg(c + nc - 1);
 #pragma unroll
-        for (int j = BOYS_NCOEF - 2; j >= 0; j--) p = p * x + __ldg(c + j);
+        for (int j = nc - 2; j >= 0; j--) p = p * x + __ldg(c + j);
         return p;
     }
     // F_0 = sqrt(pi / T) / 2 (erf(sqrt T) = 1 to working precision), then the

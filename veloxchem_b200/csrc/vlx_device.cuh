@@ -14,54 +14,51 @@
 namespace vlx {
 
 // ---------------------------------------------------------------- pair views
-// Field order inside a pair block's primitive array [field][prim][pair]
-// (primitive pairs of each shell pair sorted by |kfac| descending, the first
-// nuse[pair] of them significant):
+// One primitive pair's fields, as the recursions read them.
+template <typename R>
+struct PrimRec {
+    R zeta, hiz, kfac, px, py, pz, pbx, pby, pbz;
+};
+
+// Field order inside a pair block's primitive array, tiles of 32 pairs
+// [tile][prim][field][pair of the tile] (primitive pairs of each shell pair
+// sorted by |kfac| descending, the first nuse[pair] of them significant):
 //   0 zeta = a + b            1 hiz = 1 / (2 zeta)
 //   2 kfac = Na Nb S_ab sqrt(zeta) sqrt(2 / sqrt(pi))
 //   3..5  P = (a A + b B) / zeta       6..8  P - B
-// and per pair ab[3][pair] = B - A, ao[2][pair] = AO index of m = 0 of A, B.
-struct PairView {
-    const double* __restrict__ prim;
-    const double* __restrict__ ab;
-    int npairs, kprim, kuse, i;
-    __device__ __forceinline__ double fld(int f, int p) const { return __ldg(prim + ((size_t)(f * kprim + p)) * npairs + i); }
+// and per tile ab[3][pair of the tile] = B - A; ao[2][pair] = AO index of m = 0
+// of A, B.  The FP32 view (mixed precision) reads the rounded copies, so its
+// primitive loops load half the bytes and convert nothing.
+template <typename R>
+struct PairViewT {
+    const R* __restrict__ prim;  // the pair's column of its tile
+    const R* __restrict__ ab;
+    int kuse;
+    __device__ __forceinline__ R fld(int f, int p) const { return __ldg(prim + p * 288 + f * 32); }
     __device__ __forceinline__ int nprim() const { return kuse; }
-    __device__ __forceinline__ double zeta(int p) const { return fld(0, p); }
-    __device__ __forceinline__ double hiz(int p) const { return fld(1, p); }
-    __device__ __forceinline__ double kfac(int p) const { return fld(2, p); }
-    __device__ __forceinline__ double px(int p) const { return fld(3, p); }
-    __device__ __forceinline__ double py(int p) const { return fld(4, p); }
-    __device__ __forceinline__ double pz(int p) const { return fld(5, p); }
-    __device__ __forceinline__ double pbx(int p) const { return fld(6, p); }
-    __device__ __forceinline__ double pby(int p) const { return fld(7, p); }
-    __device__ __forceinline__ double pbz(int p) const { return fld(8, p); }
-    __device__ __forceinline__ double abx() const { return __ldg(ab + i); }
-    __device__ __forceinline__ double aby() const { return __ldg(ab + npairs + i); }
-    __device__ __forceinline__ double abz() const { return __ldg(ab + 2 * npairs + i); }
+    __device__ __forceinline__ R zeta(int p) const { return fld(0, p); }
+    __device__ __forceinline__ R hiz(int p) const { return fld(1, p); }
+    __device__ __forceinline__ R kfac(int p) const { return fld(2, p); }
+    __device__ __forceinline__ R px(int p) const { return fld(3, p); }
+    __device__ __forceinline__ R py(int p) const { return fld(4, p); }
+    __device__ __forceinline__ R pz(int p) const { return fld(5, p); }
+    __device__ __forceinline__ R pbx(int p) const { return fld(6, p); }
+    __device__ __forceinline__ R pby(int p) const { return fld(7, p); }
+    __device__ __forceinline__ R pbz(int p) const { return fld(8, p); }
+    __device__ __forceinline__ PrimRec<R> rec(int p) const
+    {
+        return {zeta(p), hiz(p), kfac(p), px(p), py(p), pz(p), pbx(p), pby(p), pbz(p)};
+    }
+    __device__ __forceinline__ R abx() const { return __ldg(ab); }
+    __device__ __forceinline__ R aby() const { return __ldg(ab + 32); }
+    __device__ __forceinline__ R abz() const { return __ldg(ab + 64); }
 };
+using PairView = PairViewT<double>;
+using PairViewF = PairViewT<float>;
 
-// The same fields rounded to FP32 (the mixed-precision path reads these, so
-// its primitive loops load half the bytes and convert nothing).
-struct PairViewF {
-    const float* __restrict__ prim;
-    int npairs, kprim, kuse, i;
-    __device__ __forceinline__ float fld(int f, int p) const { return __ldg(prim + ((size_t)(f * kprim + p)) * npairs + i); }
-    __device__ __forceinline__ int nprim() const { return kuse; }
-    __device__ __forceinline__ float zeta(int p) const { return fld(0, p); }
-    __device__ __forceinline__ float hiz(int p) const { return fld(1, p); }
-    __device__ __forceinline__ float kfac(int p) const { return fld(2, p); }
-    __device__ __forceinline__ float px(int p) const { return fld(3, p); }
-    __device__ __forceinline__ float py(int p) const { return fld(4, p); }
-    __device__ __forceinline__ float pz(int p) const { return fld(5, p); }
-    __device__ __forceinline__ float pbx(int p) const { return fld(6, p); }
-    __device__ __forceinline__ float pby(int p) const { return fld(7, p); }
-    __device__ __forceinline__ float pbz(int p) const { return fld(8, p); }
-    // ab[3][npairs] follows the 9 kprim primitive rows
-    __device__ __forceinline__ float abx() const { return fld(9, 0); }
-    __device__ __forceinline__ float aby() const { return fld(9, 1); }
-    __device__ __forceinline__ float abz() const { return fld(9, 2); }
-};
+// Offset of primitive 0, field 0 of pair i, and of its B - A.
+__host__ __device__ __forceinline__ size_t prim_offset(int kprim, int i) { return (size_t)(i >> 5) * kprim * 288 + (i & 31); }
+__host__ __device__ __forceinline__ size_t ab_offset(int i) { return (size_t)(i >> 5) * 96 + (i & 31); }
 
 // The bra pair's primitive fields staged in shared memory for a work item
 // (record of 10 per primitive: the 9 fields of PairView, padded to 16 bytes),
@@ -70,8 +67,8 @@ struct PairViewF {
 template <typename R>
 struct PairViewS {
     const R* s;
-    const R* ab;  // B - A rows (npairs apart)
-    int npairs, kuse, i;
+    const R* ab;  // the pair's column of its tile's B - A
+    int kuse;
     __device__ __forceinline__ int nprim() const { return kuse; }
     __device__ __forceinline__ R zeta(int p) const { return s[p * 10 + 0]; }
     __device__ __forceinline__ R hiz(int p) const { return s[p * 10 + 1]; }
@@ -82,47 +79,66 @@ struct PairViewS {
     __device__ __forceinline__ R pbx(int p) const { return s[p * 10 + 6]; }
     __device__ __forceinline__ R pby(int p) const { return s[p * 10 + 7]; }
     __device__ __forceinline__ R pbz(int p) const { return s[p * 10 + 8]; }
-    __device__ __forceinline__ R abx() const { return __ldg(ab + i); }
-    __device__ __forceinline__ R aby() const { return __ldg(ab + npairs + i); }
-    __device__ __forceinline__ R abz() const { return __ldg(ab + 2 * npairs + i); }
+    __device__ __forceinline__ PrimRec<R> rec(int p) const
+    {
+        return {zeta(p), hiz(p), kfac(p), px(p), py(p), pz(p), pbx(p), pby(p), pbz(p)};
+    }
+    __device__ __forceinline__ R abx() const { return __ldg(ab); }
+    __device__ __forceinline__ R aby() const { return __ldg(ab + 32); }
+    __device__ __forceinline__ R abz() const { return __ldg(ab + 64); }
+};
+
+// A bra pair of a row item: its records in row order (PairBlockDev::rprim),
+// read as warp-uniform vector loads (5 instead of 9, of contiguous bytes).
+template <typename R>
+struct Vec2;
+template <>
+struct Vec2<double> {
+    using type = double2;
+};
+template <>
+struct Vec2<float> {
+    using type = float2;
+};
+template <typename R>
+struct PairViewR {
+    using Vec = typename Vec2<R>::type;
+    const R* __restrict__ s;   // the pair's first record of 10 values
+    const R* __restrict__ ab;  // its B - A
+    int kuse;
+    __device__ __forceinline__ int nprim() const { return kuse; }
+    __device__ __forceinline__ PrimRec<R> rec(int p) const
+    {
+        const Vec* v = reinterpret_cast<const Vec*>(s + p * 10);
+        const Vec a = __ldg(v), b = __ldg(v + 1), c = __ldg(v + 2), d = __ldg(v + 3), e = __ldg(v + 4);
+        return {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x};
+    }
+    __device__ __forceinline__ R abx() const { return __ldg(ab); }
+    __device__ __forceinline__ R aby() const { return __ldg(ab + 1); }
+    __device__ __forceinline__ R abz() const { return __ldg(ab + 2); }
 };
 
 // Bra primitive pairs a staged record holds at most (36: a pair of two
 // six-primitive shells); pairs with more use the global-memory view.
 constexpr int kStageBraMax = 36;
 
-// Stages the first kuse primitive records of pair i of block b (all lanes of
-// the warp take part; the caller synchronises the warp before reading).
+// Stages the kuse significant primitive records of the pair at `v` (all lanes
+// of the warp take part; the caller synchronises the warp before reading).
 template <typename R>
-__device__ __forceinline__ void stage_bra(R* __restrict__ s, const R* __restrict__ prim, const int npairs,
-                                          const int kprim, const int i, const int kuse, const int lane)
+__device__ __forceinline__ void stage_bra(R* __restrict__ s, const PairViewT<R>& v, const int lane)
 {
-    for (int x = lane; x < kuse * 9; x += 32) {
+    for (int x = lane; x < v.kuse * 9; x += 32) {
         const int p = x / 9, f = x - p * 9;
-        s[p * 10 + f] = __ldg(prim + ((size_t)(f * kprim + p)) * npairs + i);
+        s[p * 10 + f] = v.fld(f, p);
     }
-}
-
-__device__ __forceinline__ PairViewF make_view_f(const PairBlockDev& b, int i, int kuse)
-{
-    PairViewF v;
-    v.prim = b.primf;
-    v.npairs = b.npairs;
-    v.kprim = b.kprim;
-    v.kuse = kuse;
-    v.i = i;
-    return v;
 }
 
 __device__ __forceinline__ PairView make_view(const PairBlockDev& b, int i)
 {
     PairView v;
-    v.prim = b.prim;
-    v.ab = b.ab;
-    v.npairs = b.npairs;
-    v.kprim = b.kprim;
+    v.prim = b.prim + prim_offset(b.kprim, i);
+    v.ab = b.ab + ab_offset(i);
     v.kuse = __ldg(b.nuse + i);
-    v.i = i;
     return v;
 }
 
@@ -137,30 +153,64 @@ __device__ __forceinline__ void red_add(float* p, float v)
     asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v));
 }
 
+// ---------------------------------------------------------------- elementary functions
+// 1 / sqrt(x) for positive normal x: the PTX approximation (about 20 bits) and
+// one third-order Householder step, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2.
+// The arguments here (exponent sums, Boys arguments) are never zero, negative
+// or special, so the checks of the library function are not needed; relative
+// error below 3e-16.
+__device__ __forceinline__ double rsqrt_pos(const double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
 // ---------------------------------------------------------------- Boys function
 // F_m(T) = int_0^1 t^{2m} exp(-T t^2) dt.  For T < BOYS_TMAX the highest order
-// needed is a degree-9 polynomial per unit interval of the table, in the
-// interval's local variable x in [-1, 1) (Chebyshev fit generated on the host
-// from the convergent series in long double, stored in the monomial basis of
-// x, so one Horner chain of 9 FMAs evaluates it), and the lower orders follow
-// by the stable downward recursion F_m = (2 T F_{m+1} + e^{-T}) / (2m + 1).
-// For T >= BOYS_TMAX, F_0 = sqrt(pi / T) / 2 (erf(sqrt T) = 1 to double
-// precision) and the upward recursion F_{m+1} = ((2m + 1) F_m - e^{-T}) / (2T)
-// is stable.  e^{-T} is taken before the branch: lanes of one warp often fall
-// on both sides of BOYS_TMAX.
-// tabM: the BOYS_NINT x BOYS_NCOEF coefficients of order M (global or shared
-// memory: the class kernels stage their order in shared memory).
+// needed is a degree-9 polynomial in the local variable x in [-1, 1] of the
+// interval around the table point nearest to T (Chebyshev fit generated on the
+// host from the convergent series in long double, stored in the monomial basis
+// of x, so one Horner chain of 9 FMAs evaluates it), and the lower orders follow
+// by the stable downward recursion F_m = (2 T F_{m+1} + e^{-T}) / (2m + 1), with
+// e^{-T} = e^{-T_k} e^{-x/4} from the table and a polynomial of degree 10 (its
+// Chebyshev expansion; 6e-18), a third of the instructions of the library's
+// exponential.  For T >= BOYS_TMAX, F_0 = sqrt(pi / T) / 2 (erf(sqrt T) = 1 to
+// double precision) and the upward recursion F_{m+1} = ((2m + 1) F_m - e^{-T}) /
+// (2T) is stable; e^{-T} is below 3e-17 of F_0 and F_1 there.
+// The nearest integer of 2 T comes from adding 1.5 2^52, whose sum holds it in
+// the low word: no conversion instructions.
+// tabM: the BOYS_STRIDE values of order M (global or shared memory: the class
+// kernels stage their order in shared memory).
 // F[m] = sc F_m(T), m = 0..M: the scale enters the highest order (or F_0) and
 // e^{-T} once, and the recursions carry it to the other orders.
+__device__ __forceinline__ double boys_exp(const double x, const int k, const double* __restrict__ tabM)
+{
+    double p = 2.6318062436936905e-13;
+    p = fma(p, x, -1.0528720142264342e-11);
+    p = fma(p, x, 3.7844176871668523e-10);
+    p = fma(p, x, -1.2110133608598948e-08);
+    p = fma(p, x, 3.390842016068632e-07);
+    p = fma(p, x, -8.138020840527125e-06);
+    p = fma(p, x, 0.00016276041666661556);
+    p = fma(p, x, -0.002604166666665382);
+    p = fma(p, x, 0.03125000000000001);
+    p = fma(p, x, -0.25000000000000006);
+    p = fma(p, x, 1.0);
+    return p * tabM[BOYS_NINT * BOYS_NCOEF + k];
+}
+
 template <int M>
 __device__ __forceinline__ void boys_scaled(const double T, const double sc, double* F,
                                             const double* __restrict__ tabM)
 {
-    const double et = (M > 0) ? sc * exp(-T) : 0.0;
+    static_assert(BOYS_INV_H == 2, "the local variable and boys_exp assume half-unit intervals");
     if (T < (double)BOYS_TMAX) {
-        const int it = (int)(T * (double)BOYS_INV_H);
-        const double x = fma(2.0 * BOYS_INV_H, T, -(double)(2 * it + 1));
-        const double2* c2 = reinterpret_cast<const double2*>(tabM + it * BOYS_NCOEF);
+        const double near = fma(T, (double)BOYS_INV_H, 6755399441055744.0);
+        const int k = __double2loint(near);
+        const double x = fma(T, 4.0, -2.0 * (near - 6755399441055744.0));
+        const double2* c2 = reinterpret_cast<const double2*>(tabM + k * BOYS_NCOEF);
         double c[BOYS_NCOEF];
 #pragma unroll
         for (int j = 0; j < BOYS_NCOEF / 2; j++) {
@@ -173,14 +223,17 @@ __device__ __forceinline__ void boys_scaled(const double T, const double sc, dou
         for (int j = BOYS_NCOEF - 2; j >= 0; j--) p = fma(p, x, c[j]);
         F[M] = sc * p;
         if (M > 0) {
-            const double t2 = 2.0 * T;
+            const double t2 = 2.0 * T, et = sc * boys_exp(x, k, tabM);
 #pragma unroll
             for (int m = M - 1; m >= 0; m--) F[m] = fma(t2, F[m + 1], et) * (1.0 / (2 * m + 1));
         }
     } else {
-        F[0] = (sc * 0.88622692545275801365) * rsqrt(T);
+        const double r = rsqrt_pos(T);
+        F[0] = (sc * 0.88622692545275801365) * r;
         if (M > 0) {
-            const double h = 0.5 / T;
+            // 1 / (2T) from the same root, with one correction step
+            const double r2 = r * r, h = 0.5 * fma(r2, fma(-T, r2, 1.0), r2);
+            const double et = (M > 1) ? sc * exp(-T) : 0.0;
 #pragma unroll
             for (int m = 0; m < M; m++) F[m + 1] = fma((double)(2 * m + 1), F[m], -et) * h;
         }
@@ -197,49 +250,51 @@ __device__ __forceinline__ void boys_function_tab(const double T, double* F, con
 template <int M>
 __device__ __forceinline__ void boys_function(const double T, double* F, const double* __restrict__ tab)
 {
-    boys_function_tab<M>(T, F, tab + (size_t)M * BOYS_NINT * BOYS_NCOEF);
+    boys_function_tab<M>(T, F, tab + (size_t)M * BOYS_STRIDE);
 }
 
-// FP32 Boys function for the mixed-precision path: the same polynomials
-// rounded to float, recursions in float (relative error ~1e-7).
+// FP32 Boys function for the mixed-precision path: the same scheme in float
+// (polynomials of degree 7, and 5 for e^{-x/4}; relative error ~1e-7).  e^{-T}
+// beyond BOYS_TMAX is below 3e-8 of F_m up to order 10.
 template <int M>
 __device__ __forceinline__ void boys_scaled_f(const float T, const float sc, float* F, const float* __restrict__ tabM)
 {
-    const float et = (M > 0) ? sc * expf(-T) : 0.0f;
     if (T < (float)BOYS_TMAX) {
-        const int it = (int)(T * (float)BOYS_INV_H);
-        const float x = fmaf(2.0f * BOYS_INV_H, T, -(float)(2 * it + 1));
-        const float2* c2 = reinterpret_cast<const float2*>(tabM + it * BOYS_NCOEF);
-        float c[BOYS_NCOEF];
-#pragma unroll
-        for (int j = 0; j < BOYS_NCOEF / 2; j++) {
-            const float2 v = c2[j];
-            c[2 * j] = v.x;
-            c[2 * j + 1] = v.y;
-        }
-        float p = c[BOYS_NCOEF - 1];
-#pragma unroll
-        for (int j = BOYS_NCOEF - 2; j >= 0; j--) p = fmaf(p, x, c[j]);
+        const float near = fmaf(T, (float)BOYS_INV_H, 12582912.0f);
+        const int k = __float_as_int(near) - 0x4b400000;
+        const float x = fmaf(T, 4.0f, -2.0f * (near - 12582912.0f));
+        const float4* c4 = reinterpret_cast<const float4*>(tabM + k * BOYS_NCOEF_F);
+        const float4 lo = c4[0], hi = c4[1];
+        float p = hi.w;
+        p = fmaf(p, x, hi.z);
+        p = fmaf(p, x, hi.y);
+        p = fmaf(p, x, hi.x);
+        p = fmaf(p, x, lo.w);
+        p = fmaf(p, x, lo.z);
+        p = fmaf(p, x, lo.y);
+        p = fmaf(p, x, lo.x);
         F[M] = sc * p;
         if (M > 0) {
-            const float t2 = 2.0f * T;
+            float q = -8.15923726e-06f;
+            q = fmaf(q, x, 0.000163269706f);
+            q = fmaf(q, x, -0.00260415605f);
+            q = fmaf(q, x, 0.0312498089f);
+            q = fmaf(q, x, -0.250000001f);
+            q = fmaf(q, x, 1.00000001f);
+            const float t2 = 2.0f * T, et = sc * q * tabM[BOYS_NINT * BOYS_NCOEF_F + k];
 #pragma unroll
             for (int m = M - 1; m >= 0; m--) F[m] = fmaf(t2, F[m + 1], et) * (1.0f / (2 * m + 1));
         }
     } else {
-        F[0] = (sc * 0.886226925f) * rsqrtf(T);
+        const float r = rsqrtf(T);
+        F[0] = (sc * 0.886226925f) * r;
         if (M > 0) {
-            const float h = 0.5f / T;
+            const float h = 0.5f * r * r;
+            const float et = (M > 10) ? sc * expf(-T) : 0.0f;
 #pragma unroll
             for (int m = 0; m < M; m++) F[m + 1] = fmaf((float)(2 * m + 1), F[m], -et) * h;
         }
     }
-}
-
-template <int M>
-__device__ __forceinline__ void boys_function_tab_f(const float T, float* F, const float* __restrict__ tabM)
-{
-    boys_scaled_f<M>(T, 1.0f, F, tabM);
 }
 
 // Kets of a work item admitted at run time: the kets of a pair block are

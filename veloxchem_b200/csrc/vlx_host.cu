@@ -113,49 +113,44 @@ long double boys_series(int m, long double t)
     for (int k = 1; k < 1000; k++) {
         term *= 2.0L * t / (2 * m + 2 * k + 1);
         sum += term;
-        if (term < 1e-24L * sum) break;
+        if (std::fabs(term) < 1e-24L * sum) break;
     }
     return std::exp(-t) * sum;
 }
 
-// Per (order, interval): the Chebyshev interpolant of degree BOYS_NCOEF - 1 at
-// the Chebyshev nodes of the interval's local variable x in [-1, 1], rewritten
-// in the monomial basis of x (T_0 = 1, T_1 = x, T_{j+1} = 2x T_j - T_{j-1}) so
-// that the device evaluates it by Horner's rule.  The coefficients decay fast
-// (|c_9| ~ 1e-17 relative), so the monomial form on [-1, 1] stays as well
-// conditioned as the Chebyshev one.
-std::vector<double> make_boys_table()
+// Per (order, interval): the Chebyshev interpolant of N coefficients at the
+// Chebyshev nodes of the interval's local variable x in [-1, 1], rewritten in
+// the monomial basis of x (T_0 = 1, T_1 = x, T_{j+1} = 2x T_j - T_{j-1}) so that
+// the device evaluates it by Horner's rule (the coefficients decay fast, so the
+// monomial form on [-1, 1] stays as well conditioned as the Chebyshev one);
+// behind each order's coefficients e^{-k / BOYS_INV_H} per interval k.
+template <int N>
+std::vector<long double> make_boys_table(int stride)
 {
-    const int N = BOYS_NCOEF;
+    const long double pi = std::acos(-1.0L), h = 1.0L / BOYS_INV_H;
     // monomial coefficients of T_0 .. T_{N-1}
-    long double tj[BOYS_NCOEF][BOYS_NCOEF] = {};
+    long double tj[N][N] = {};
     tj[0][0] = 1.0L;
     if (N > 1) tj[1][1] = 1.0L;
     for (int j = 2; j < N; j++)
         for (int k = 0; k < N; k++)
             tj[j][k] = (k > 0 ? 2.0L * tj[j - 1][k - 1] : 0.0L) - tj[j - 2][k];
-    std::vector<double> tab((size_t)(BOYS_MMAX + 1) * BOYS_NINT * N);
-    for (int m = 0; m <= BOYS_MMAX; m++)
+    std::vector<long double> tab((size_t)(BOYS_MMAX + 1) * stride, 0.0L);
+    for (int m = 0; m <= BOYS_MMAX; m++) {
+        long double* order = tab.data() + (size_t)m * stride;
         for (int it = 0; it < BOYS_NINT; it++) {
-            long double fv[BOYS_NCOEF], cheb[BOYS_NCOEF];
-            for (int k = 0; k < N; k++) {
-                const long double x = std::cos(M_PI * (k + 0.5L) / N);
-                const long double h = 1.0L / BOYS_INV_H;
-                fv[k] = boys_series(m, it * h + 0.5L * h + 0.5L * h * x);
-            }
+            long double fv[N], cheb[N];
+            for (int k = 0; k < N; k++) fv[k] = boys_series(m, h * (it + 0.5L * std::cos(pi * (k + 0.5L) / N)));
             for (int j = 0; j < N; j++) {
                 long double s = 0.0L;
-                for (int k = 0; k < N; k++) s += fv[k] * std::cos(M_PI * j * (k + 0.5L) / N);
-                s *= 2.0L / N;
-                if (j == 0) s *= 0.5L;
-                cheb[j] = s;
+                for (int k = 0; k < N; k++) s += fv[k] * std::cos(pi * j * (k + 0.5L) / N);
+                cheb[j] = s * (j == 0 ? 1.0L : 2.0L) / N;
             }
-            for (int k = 0; k < N; k++) {
-                long double a = 0.0L;
-                for (int j = k; j < N; j++) a += cheb[j] * tj[j][k];
-                tab[((size_t)(m * BOYS_NINT + it)) * N + k] = (double)a;
-            }
+            for (int k = 0; k < N; k++)
+                for (int j = k; j < N; j++) order[it * N + k] += cheb[j] * tj[j][k];
+            order[BOYS_NINT * N + it] = std::exp(-h * it);
         }
+    }
     return tab;
 }
 
@@ -168,14 +163,14 @@ struct DeviceGlobals {
     void* prog = nullptr;
     std::vector<CoopClassDev> coop;
     std::vector<int> coop_prim_flops, coop_post_flops;
-    // resident blocks per SM of the compiled classes' kernels, plain and
-    // extended (0: not asked yet; every thread finds the same value)
-    std::atomic<int> occupancy[2][vlx::kNumQuartetClasses] = {};
+    // resident blocks per SM of the compiled classes' kernel variants
+    // (0: not asked yet; every thread finds the same value)
+    std::atomic<int> occupancy[vlx::kNumVariants][2][vlx::kNumQuartetClasses] = {};
 
-    int resident_blocks(int cls, bool ext)
+    int resident_blocks(int cls, int variant, bool f32)
     {
-        std::atomic<int>& o = occupancy[ext ? 1 : 0][cls];
-        if (o.load() == 0) o.store(std::max(1, vlx::kQuartetClasses[cls].occupancy(ext ? 1 : 0)));
+        std::atomic<int>& o = occupancy[variant][f32 ? 1 : 0][cls];
+        if (o.load() == 0) o.store(std::max(1, vlx::kQuartetClasses[cls].occupancy[variant](f32)));
         return o.load();
     }
 };
@@ -190,10 +185,12 @@ int device_globals(int device, DeviceGlobals** out)
     if (!g.ready) {
         VLX_CUDA(cudaSetDevice(device));
         VLX_CUDA(cudaDeviceGetAttribute(&g.nsm, cudaDevAttrMultiProcessorCount, device));
-        const auto tab = make_boys_table();
+        const auto t64 = make_boys_table<BOYS_NCOEF>(BOYS_STRIDE);
+        const auto t32 = make_boys_table<BOYS_NCOEF_F>(BOYS_STRIDE_F);
+        const std::vector<double> tab(t64.begin(), t64.end());
+        const std::vector<float> tabf(t32.begin(), t32.end());
         VLX_CUDA(cudaMalloc(&g.boys, tab.size() * sizeof(double)));
         VLX_CUDA(cudaMemcpy(g.boys, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
-        const std::vector<float> tabf(tab.begin(), tab.end());
         VLX_CUDA(cudaMalloc(&g.boys_f, tabf.size() * sizeof(float)));
         VLX_CUDA(cudaMemcpy(g.boys_f, tabf.data(), tabf.size() * sizeof(float), cudaMemcpyHostToDevice));
         // warp-cooperative programs (gen_coop.py): magic, count, 16-int headers,
@@ -436,29 +433,61 @@ struct PairBlock {
     std::vector<int> nuse_ref;               // reference order: significant primitive pairs
     std::vector<int> nuse;                   // sorted order: significant primitive pairs
     std::vector<long long> nuse_prefix;      // sorted order: prefix sums of nuse
+    // the sorted pairs by rows of equal second shell (ascending sorted position
+    // within a row): sorted position per row position, row starts, and per row
+    // the number of pairs of bin <= b
+    std::vector<int> row, row_off;
+    std::vector<std::array<int, 16>> row_bins;
 };
+
+// Rows of a screened, bin-sorted pair block.
+void make_rows(PairBlock& pb)
+{
+    const int n = (int)pb.sorted.size();
+    pb.row.resize(n);
+    std::iota(pb.row.begin(), pb.row.end(), 0);
+    std::stable_sort(pb.row.begin(), pb.row.end(), [&pb](int x, int y) {
+        return pb.pairs[pb.sorted[x]].second < pb.pairs[pb.sorted[y]].second;
+    });
+    pb.row_off.clear();
+    pb.row_bins.clear();
+    for (int q = 0; q < n; q++) {
+        if (q == 0 || pb.pairs[pb.sorted[pb.row[q]]].second != pb.pairs[pb.sorted[pb.row[q - 1]]].second) {
+            pb.row_off.push_back(q);
+            pb.row_bins.push_back(std::array<int, 16>{});
+        }
+        for (int b = pb.bin[pb.sorted[pb.row[q]]]; b < 16; b++) pb.row_bins.back()[b]++;
+    }
+    pb.row_off.push_back(n);
+}
 
 struct ClassTasks {
     int compiled = -1;  // index into kQuartetClasses
     int coop = -1;      // index into DeviceGlobals::coop
     int la = 0, lb = 0, lc = 0, ld = 0;
-    std::vector<WorkItem> items;    // FP64 quartets
+    std::vector<WorkItem> items;
+    bool rows = false;                        // row items (else pair items)
+    std::vector<std::pair<int, int>> jobs;    // (bra block, ket block) of the class; complete when nodes == 1
     size_t offset = 0;  // first item in the task set's device array
-    long long quartets = 0, prim_quartets = 0, ref_prim_quartets = 0;  // at the task set's threshold
+    long long quartets = 0, prim_quartets = 0;  // at the task set's threshold
 };
 
 struct TaskSet {
     int ith = 0, rank = 0, nodes = 1, seg = 0, tune_gen = 0;  // ith: the threshold the items were built for
     int part = 0;  // partition of the items over nodes: 0 round-robin, 1 cost-balanced
+    // pair items throughout, for the extended kernels (density screening,
+    // multi-density builds); otherwise the compiled classes have row items
+    bool ext = false;
+    int share = 1;  // molecules whose items share the launches
     std::vector<ClassTasks> classes;
     WorkItem* d_items = nullptr;
     long long quartets = 0, prim_quartets = 0;
 };
 
-// Streams beside a build's own for the class launches that cannot fill the
-// chip (enqueue_ctx), made on first use and owned by a screener or a batch.
+// Streams beside a build's own for its class launches (enqueue_ctx), made on
+// first use and owned by a screener or a batch.
 struct SideStreams {
-    static constexpr int kCount = 8;
+    static constexpr int kCount = 16;
     cudaStream_t s[kCount] = {};
     cudaEvent_t fork = nullptr, join[kCount] = {};
     bool ready = false;
@@ -466,11 +495,9 @@ struct SideStreams {
     int open()
     {
         if (ready) return VLX_B200_OK;
-        int least = 0, greatest = 0;
-        VLX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         if (!fork) VLX_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
         for (int i = 0; i < kCount; i++) {
-            if (!s[i]) VLX_CUDA(cudaStreamCreateWithPriority(&s[i], cudaStreamNonBlocking, greatest));
+            if (!s[i]) VLX_CUDA(cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking));
             if (!join[i]) VLX_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
         }
         ready = true;
@@ -495,6 +522,12 @@ int pair_key(int la, int lb) { return (la + lb) * 16 + lb; }
 
 // ket pairs per work item of a warp-cooperative class
 constexpr int kCoopSegment = 2;
+
+// Steps (bra pairs against 32 kets) of a row item per ket pair of the
+// work-item length: the default length of 256 ket pairs allows rows of 32.
+constexpr int kRowShare = 8;
+// Row items per SM that a class is cut into at least, where it has the steps.
+constexpr int kRowSpread = 64;
 
 }  // namespace
 
@@ -551,135 +584,236 @@ struct vlx_b200_screener {
 
 namespace {
 
-// Byte offset of a pair block's FP32 fields (after its FP64 fields and index
-// arrays, 16-byte aligned).
-size_t fp32_offset(size_t n, size_t kp)
+// Sections of a device arena, 256-byte aligned.
+struct Arena {
+    size_t size = 0;
+    size_t take(size_t bytes)
+    {
+        const size_t at = size;
+        size += (bytes + 255) & ~size_t(255);
+        return at;
+    }
+};
+
+// The pair data of every pair of a block in reference order (FP64 tiles, see
+// PairBlockDev), computed on the host once, from which the Schwarz diagonals are
+// evaluated and the screened pairs gathered (upload_pairs).
+struct RawPairs {
+    char* dev = nullptr;
+    PairBlockDev* d_blocks = nullptr;
+
+    ~RawPairs()
+    {
+        if (dev) cudaFree(dev);
+        if (d_blocks) cudaFree(d_blocks);
+    }
+
+    int upload(vlx_b200_screener* s)
+    {
+        const size_t nb = s->blocks.size();
+        Arena arena;
+        std::vector<std::array<size_t, 3>> at(nb);  // prim, ab, nuse
+        for (size_t b = 0; b < nb; b++) {
+            const PairBlock& pb = s->blocks[b];
+            const size_t n = pb.pairs.size(), tiles = (n + 31) / 32;
+            at[b] = {arena.take(tiles * pb.ka * pb.kb * 288 * sizeof(double)), arena.take(tiles * 96 * sizeof(double)),
+                     arena.take(n * sizeof(int))};
+        }
+        const std::unique_ptr<char[]> host(new char[arena.size + 256]);
+        VLX_CUDA(cudaMalloc(&dev, arena.size + 256));
+        VLX_CUDA(cudaMalloc(&d_blocks, std::max<size_t>(1, nb) * sizeof(PairBlockDev)));
+        std::vector<PairBlockDev> h(nb);
+        const double kconst = std::sqrt(2.0 / std::sqrt(M_PI));
+        for (size_t b = 0; b < nb; b++) {
+            PairBlock& pb = s->blocks[b];
+            const int n = (int)pb.pairs.size(), kp = pb.ka * pb.kb;
+            double* prim = reinterpret_cast<double*>(host.get() + at[b][0]);
+            double* ab = reinterpret_cast<double*>(host.get() + at[b][1]);
+            int* nuse = reinterpret_cast<int*>(host.get() + at[b][2]);
+            pb.nuse_ref.resize(n);
+            std::vector<std::array<double, 9>> vals(kp);
+            for (int i = 0; i < n; i++) {
+                const Shell& A = s->shells[pb.pairs[i].first];
+                const Shell& B = s->shells[pb.pairs[i].second];
+                double r2 = 0.0;
+                double* abi = ab + vlx::ab_offset(i);
+                for (int x = 0; x < 3; x++) {
+                    abi[32 * x] = B.xyz[x] - A.xyz[x];
+                    r2 += (B.xyz[x] - A.xyz[x]) * (B.xyz[x] - A.xyz[x]);
+                }
+                for (int ka = 0; ka < pb.ka; ka++)
+                    for (int kb = 0; kb < pb.kb; kb++) {
+                        const double ea = A.e[ka], eb = B.e[kb], z = ea + eb;
+                        const double fz = M_PI / z;
+                        const double sab = fz * std::sqrt(fz) * std::exp(-ea * eb / z * r2);
+                        const double cab = A.c[ka] * B.c[kb] * sab;
+                        std::array<double, 9>& v = vals[ka * pb.kb + kb];
+                        v[0] = z;
+                        v[1] = 0.5 / z;
+                        v[2] = cab * std::sqrt(z) * kconst;
+                        for (int x = 0; x < 3; x++) {
+                            v[3 + x] = (ea * A.xyz[x] + eb * B.xyz[x]) / z;
+                            v[6 + x] = v[3 + x] - B.xyz[x];
+                        }
+                    }
+                // significant primitive pairs first; the kernels loop over the first nuse
+                if (kp > 1)
+                    std::stable_sort(vals.begin(), vals.end(),
+                                     [](const std::array<double, 9>& x, const std::array<double, 9>& y) {
+                                         return std::fabs(x[2]) > std::fabs(y[2]);
+                                     });
+                int used = 0;
+                while (used < kp && std::fabs(vals[used][2]) >= VLX_PRIM_CUTOFF) used++;
+                nuse[i] = pb.nuse_ref[i] = std::max(used, 1);
+                double* pi = prim + vlx::prim_offset(kp, i);
+                for (int p = 0; p < kp; p++)
+                    for (int f = 0; f < 9; f++) pi[p * 288 + f * 32] = vals[p][f];
+            }
+            PairBlockDev& d = h[b];
+            std::memset(&d, 0, sizeof(d));
+            d.prim = reinterpret_cast<const double*>(dev + at[b][0]);
+            d.ab = reinterpret_cast<const double*>(dev + at[b][1]);
+            d.nuse = reinterpret_cast<const int*>(dev + at[b][2]);
+            d.npairs = n;
+            d.kprim = kp;
+            d.la = pb.la;
+            d.lb = pb.lb;
+        }
+        VLX_CUDA(cudaMemcpy(dev, host.get(), arena.size, cudaMemcpyHostToDevice));
+        VLX_CUDA(cudaMemcpy(d_blocks, h.data(), nb * sizeof(PairBlockDev), cudaMemcpyHostToDevice));
+        return VLX_B200_OK;
+    }
+};
+
+// Fills the screened pairs' fields: blockIdx.y is the block; one thread per
+// position takes the pair src[position] of the raw data into the bin-sorted
+// tiles (FP64 and FP32) and into its row-order records.  pos[]: the row
+// position of each sorted position.
+__global__ void gather_pairs_kernel(const PairBlockDev* __restrict__ raw, const PairBlockDev* __restrict__ blocks,
+                                    const int* const* __restrict__ src, const int* const* __restrict__ pos)
 {
-    const size_t bytes = (9 * kp * n + 3 * n) * sizeof(double) + (6 * n + 17) * sizeof(int);
-    return (bytes + 15) & ~size_t(15);
+    const PairBlockDev b = blocks[blockIdx.y], r = raw[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < b.npairs; i += gridDim.x * blockDim.x) {
+        const int from = src[blockIdx.y][i], q = pos[blockIdx.y][i];
+        const_cast<int4*>(b.rhead)[q] = make_int4(i, b.ao[i], b.ao[b.npairs + i], b.nuse[i] | (b.bin[i] << 16));
+        const double* ab = r.ab + vlx::ab_offset(from);
+        for (int x = 0; x < 4; x++) {
+            const double v = x < 3 ? ab[32 * x] : 0.0;
+            if (x < 3) {
+                const_cast<double*>(b.ab)[vlx::ab_offset(i) + 32 * x] = v;
+                const_cast<float*>(b.abf)[vlx::ab_offset(i) + 32 * x] = (float)v;
+            }
+            const_cast<double*>(b.rab)[4 * (size_t)q + x] = v;
+            const_cast<float*>(b.rabf)[4 * (size_t)q + x] = (float)v;
+        }
+        const double* p0 = r.prim + vlx::prim_offset(b.kprim, from);
+        double* p1 = const_cast<double*>(b.prim) + vlx::prim_offset(b.kprim, i);
+        float* p2 = const_cast<float*>(b.primf) + vlx::prim_offset(b.kprim, i);
+        for (int p = 0; p < b.kprim; p++) {
+            double* rec = const_cast<double*>(b.rprim) + ((size_t)q * b.kprim + p) * 10;
+            float* recf = const_cast<float*>(b.rprimf) + ((size_t)q * b.kprim + p) * 10;
+            for (int f = 0; f < 10; f++) {
+                const double v = f < 9 ? p0[p * 288 + f * 32] : 0.0;
+                if (f < 9) {
+                    p1[p * 288 + f * 32] = v;
+                    p2[p * 288 + f * 32] = (float)v;
+                }
+                rec[f] = v;
+                recf[f] = (float)v;
+            }
+        }
+    }
 }
 
-// Builds device arrays of all pair blocks; `sorted` selects the screened,
-// bin-sorted pair order instead of the reference order.
-int upload_pairs(vlx_b200_screener* s, bool sorted)
+// The device arrays of the screened, bin-sorted pairs: the index arrays from
+// the host, the rest gathered on the device from the raw pair data.
+int upload_pairs(vlx_b200_screener* s, const RawPairs& raw)
 {
     const size_t nb = s->blocks.size();
-    std::vector<size_t> offs(nb + 1, 0);
-    std::vector<int> npairs(nb);
+    Arena idx, data;
+    std::vector<std::array<size_t, 8>> ai(nb);
+    std::vector<std::array<size_t, 9>> ad(nb);
+    int most = 0;
     for (size_t b = 0; b < nb; b++) {
         const PairBlock& pb = s->blocks[b];
-        const size_t n = sorted ? pb.sorted.size() : pb.pairs.size();
-        npairs[b] = (int)n;
-        const size_t k = (size_t)pb.ka * pb.kb;
-        size_t bytes = fp32_offset(n, k) + (9 * k * n + 4 * n) * sizeof(float);
-        bytes = (bytes + 255) & ~size_t(255);
-        offs[b + 1] = offs[b] + bytes;
+        const size_t n = pb.sorted.size(), tiles = (n + 31) / 32, k = (size_t)pb.ka * pb.kb;
+        most = std::max(most, (int)n);
+        ai[b] = {idx.take(2 * n * sizeof(int)), idx.take(n * sizeof(int)),     idx.take(n * sizeof(int)),
+                 idx.take(17 * sizeof(int)),    idx.take(2 * n * sizeof(int)), idx.take(n * sizeof(float)),
+                 idx.take(n * sizeof(int)),     idx.take(n * sizeof(int))};
+        ad[b] = {data.take(tiles * k * 288 * sizeof(double)), data.take(tiles * 96 * sizeof(double)),
+                 data.take(tiles * k * 288 * sizeof(float)),  data.take(tiles * 96 * sizeof(float)),
+                 data.take(n * sizeof(int4)),                 data.take(4 * n * sizeof(double)),
+                 data.take(10 * k * n * sizeof(double)),      data.take(4 * n * sizeof(float)),
+                 data.take(10 * k * n * sizeof(float))};
     }
-    std::vector<char> host(offs[nb] + 256, 0);
+    const size_t ptrs = idx.take(2 * nb * sizeof(int*));
+    const size_t idx_at = data.take(idx.size);
+    VLX_CUDA(cudaMalloc(&s->d_pairs, data.size + 256));
+    char* dev = s->d_pairs;
+    const std::unique_ptr<char[]> host(new char[idx.size]);
     s->h_blocks.assign(nb, PairBlockDev{});
-    const double kconst = std::sqrt(2.0 / std::sqrt(M_PI));
     for (size_t b = 0; b < nb; b++) {
-        if (sorted)
-            s->blocks[b].nuse.assign(npairs[b], 0);
-        else
-            s->blocks[b].nuse_ref.assign(npairs[b], 0);
-        const PairBlock& pb = s->blocks[b];
-        const size_t n = npairs[b];
-        const int kp = pb.ka * pb.kb;
-        double* prim = reinterpret_cast<double*>(host.data() + offs[b]);
-        double* ab = prim + 9 * (size_t)kp * n;
-        int* ao = reinterpret_cast<int*>(ab + 3 * n);
-        int* nuse = ao + 2 * n;
-        int* bins = nuse + n;     // Schwarz bin per pair (sorted order; 0 before screening)
-        int* bin_off = bins + n;  // first pair of bin >= b (17 entries)
-        int* shl = bin_off + 17;  // shell index of A, then of B
-        float* primf = reinterpret_cast<float*>(host.data() + offs[b] + fp32_offset(n, (size_t)kp));
-        float* abf = primf + 9 * (size_t)kp * n;
-        float* qf = abf + 3 * n;  // Schwarz factor, rounded up (0 before screening)
-        for (int k = 0; k <= 16; k++) bin_off[k] = sorted ? pb.bin_off[k] : 0;
+        PairBlock& pb = s->blocks[b];
+        const size_t n = pb.sorted.size();
+        const auto at = [&](int k) { return reinterpret_cast<int*>(host.get() + ai[b][k]); };
+        int *ao = at(0), *nuse = at(1), *bins = at(2), *bin_off = at(3), *shl = at(4), *src = at(6), *pos = at(7);
+        float* qf = reinterpret_cast<float*>(at(5));
+        for (int k = 0; k <= 16; k++) bin_off[k] = pb.bin_off[k];
+        pb.nuse.resize(n);
+        pb.nuse_prefix.assign(n + 1, 0);
         for (size_t i = 0; i < n; i++) {
-            bins[i] = sorted ? pb.bin[pb.sorted[i]] : 0;
-            const int ref = sorted ? pb.sorted[i] : (int)i;
-            const Shell& A = s->shells[pb.pairs[ref].first];
-            const Shell& B = s->shells[pb.pairs[ref].second];
-            double r2 = 0.0;
-            for (int x = 0; x < 3; x++) {
-                ab[x * n + i] = B.xyz[x] - A.xyz[x];
-                abf[x * n + i] = (float)ab[x * n + i];
-                r2 += (B.xyz[x] - A.xyz[x]) * (B.xyz[x] - A.xyz[x]);
-            }
-            ao[i] = A.ao0;
-            ao[n + i] = B.ao0;
+            const int ref = pb.sorted[i];
+            ao[i] = s->shells[pb.pairs[ref].first].ao0;
+            ao[n + i] = s->shells[pb.pairs[ref].second].ao0;
+            nuse[i] = pb.nuse[i] = pb.nuse_ref[ref];
+            pb.nuse_prefix[i + 1] = pb.nuse_prefix[i] + pb.nuse[i];
+            bins[i] = pb.bin[ref];
             shl[i] = pb.pairs[ref].first;
             shl[n + i] = pb.pairs[ref].second;
-            qf[i] = sorted ? std::nextafter((float)std::sqrt(pb.maxv[ref]), INFINITY) : 0.0f;
-            std::vector<std::array<double, 9>> vals(kp);
-            for (int ka = 0; ka < pb.ka; ka++)
-                for (int kb = 0; kb < pb.kb; kb++) {
-                    const int p = ka * pb.kb + kb;
-                    const double ea = A.e[ka], eb = B.e[kb], z = ea + eb;
-                    const double fz = M_PI / z;
-                    const double sab = fz * std::sqrt(fz) * std::exp(-ea * eb / z * r2);
-                    const double cab = A.c[ka] * B.c[kb] * sab;
-                    std::array<double, 9>& v = vals[p];
-                    v[0] = z;
-                    v[1] = 0.5 / z;
-                    v[2] = cab * std::sqrt(z) * kconst;
-                    for (int x = 0; x < 3; x++) {
-                        v[3 + x] = (ea * A.xyz[x] + eb * B.xyz[x]) / z;
-                        v[6 + x] = v[3 + x] - B.xyz[x];
-                    }
-                }
-            // significant primitive pairs first; the kernels loop over the first nuse
-            std::stable_sort(vals.begin(), vals.end(), [](const std::array<double, 9>& x,
-                                                          const std::array<double, 9>& y) {
-                return std::fabs(x[2]) > std::fabs(y[2]);
-            });
-            int used = 0;
-            while (used < kp && std::fabs(vals[used][2]) >= VLX_PRIM_CUTOFF) used++;
-            nuse[i] = std::max(used, 1);
-            if (sorted)
-                s->blocks[b].nuse[i] = nuse[i];
-            else
-                s->blocks[b].nuse_ref[i] = nuse[i];
-            for (int p = 0; p < kp; p++)
-                for (int f = 0; f < 9; f++) {
-                    prim[((size_t)f * kp + p) * n + i] = vals[p][f];
-                    primf[((size_t)f * kp + p) * n + i] = (float)vals[p][f];
-                }
+            qf[i] = std::nextafter((float)std::sqrt(pb.maxv[ref]), INFINITY);
+            src[i] = ref;
+            pos[pb.row[i]] = (int)i;
         }
-    }
-    if (sorted)
-        for (auto& pb : s->blocks) {
-            pb.nuse_prefix.assign(pb.nuse.size() + 1, 0);
-            for (size_t i = 0; i < pb.nuse.size(); i++) pb.nuse_prefix[i + 1] = pb.nuse_prefix[i] + pb.nuse[i];
-        }
-    if (s->d_pairs) cudaFree(s->d_pairs);
-    s->d_pairs = nullptr;
-    VLX_CUDA(cudaMalloc(&s->d_pairs, host.size()));
-    VLX_CUDA(cudaMemcpy(s->d_pairs, host.data(), host.size(), cudaMemcpyHostToDevice));
-    for (size_t b = 0; b < nb; b++) {
-        const PairBlock& pb = s->blocks[b];
-        const size_t n = npairs[b];
-        const int kp = pb.ka * pb.kb;
-        PairBlockDev d;
-        d.prim = reinterpret_cast<const double*>(s->d_pairs + offs[b]);
-        d.ab = d.prim + 9 * (size_t)kp * n;
-        d.primf = reinterpret_cast<const float*>(s->d_pairs + offs[b] + fp32_offset(n, (size_t)kp));
-        d.ao = reinterpret_cast<const int*>(d.ab + 3 * n);
-        d.nuse = d.ao + 2 * n;
-        d.bin = d.nuse + n;
-        d.bin_off = d.bin + n;
-        d.sh = d.bin_off + 17;
-        d.q = d.primf + (9 * (size_t)kp + 3) * n;
+        const auto di = [&](int k) { return reinterpret_cast<const int*>(dev + idx_at + ai[b][k]); };
+        const auto dd = [&](int k) { return reinterpret_cast<const double*>(dev + ad[b][k]); };
+        const auto df = [&](int k) { return reinterpret_cast<const float*>(dev + ad[b][k]); };
+        PairBlockDev& d = s->h_blocks[b];
+        d.prim = dd(0);
+        d.ab = dd(1);
+        d.primf = df(2);
+        d.abf = df(3);
+        d.ao = di(0);
+        d.nuse = di(1);
+        d.bin = di(2);
+        d.bin_off = di(3);
+        d.sh = di(4);
+        d.q = reinterpret_cast<const float*>(di(5));
+        d.rhead = reinterpret_cast<const int4*>(dd(4));
+        d.rab = dd(5);
+        d.rprim = dd(6);
+        d.rabf = df(7);
+        d.rprimf = df(8);
         d.npairs = (int)n;
-        d.kprim = kp;
+        d.kprim = pb.ka * pb.kb;
         d.la = pb.la;
         d.lb = pb.lb;
-        s->h_blocks[b] = d;
+        const int* sp = di(6);
+        const int* pp = di(7);
+        std::memcpy(host.get() + ptrs + b * sizeof(int*), &sp, sizeof(int*));
+        std::memcpy(host.get() + ptrs + (nb + b) * sizeof(int*), &pp, sizeof(int*));
     }
-    if (!s->d_blocks) VLX_CUDA(cudaMalloc(&s->d_blocks, std::max<size_t>(1, nb) * sizeof(PairBlockDev)));
+    VLX_CUDA(cudaMemcpy(dev + idx_at, host.get(), idx.size, cudaMemcpyHostToDevice));
+    VLX_CUDA(cudaMalloc(&s->d_blocks, std::max<size_t>(1, nb) * sizeof(PairBlockDev)));
     VLX_CUDA(cudaMemcpy(s->d_blocks, s->h_blocks.data(), nb * sizeof(PairBlockDev), cudaMemcpyHostToDevice));
+    if (most > 0) {
+        const dim3 grid((unsigned)std::min((most + 127) / 128, 1024), (unsigned)nb);
+        const int* const* lists = reinterpret_cast<const int* const*>(dev + idx_at + ptrs);
+        gather_pairs_kernel<<<grid, 128, 0, s->stream>>>(raw.d_blocks, s->d_blocks, lists, lists + nb);
+        VLX_CUDA(cudaGetLastError());
+        // builds run on the callers' streams
+        VLX_CUDA(cudaStreamSynchronize(s->stream));
+    }
     return VLX_B200_OK;
 }
 
@@ -701,49 +835,122 @@ int find_coop(const DeviceGlobals* g, int la, int lb, int lc, int ld)
     return -1;
 }
 
-int run_schwarz(vlx_b200_screener* s, std::vector<std::vector<double>>& maxv)
+int run_schwarz(vlx_b200_screener* s, const PairBlockDev* d_blocks, std::vector<std::vector<double>>& maxv)
 {
     const size_t nb = s->blocks.size();
-    std::vector<double*> d_max(nb, nullptr);
+    std::vector<size_t> off(nb + 1, 0);
+    for (size_t b = 0; b < nb; b++) off[b + 1] = off[b] + s->blocks[b].pairs.size();
+    double* d_max = nullptr;
+    VLX_CUDA(cudaMalloc(&d_max, std::max<size_t>(1, off[nb]) * sizeof(double)));
+    const std::unique_ptr<double, cudaError_t (*)(void*)> owner(d_max, [](void* p) { return cudaFree(p); });
     for (size_t b = 0; b < nb; b++) {
         const PairBlock& pb = s->blocks[b];
         const int n = (int)pb.pairs.size();
-        VLX_CUDA(cudaMalloc(&d_max[b], std::max(1, n) * sizeof(double)));
         bool done = false;
         for (int c = 0; c < vlx::kNumSchwarzClasses; c++) {
             if (vlx::kSchwarzClasses[c].la == pb.la && vlx::kSchwarzClasses[c].lb == pb.lb) {
-                vlx::kSchwarzClasses[c].launch(s->d_blocks, (int)b, n, s->glob->boys, d_max[b], s->stream);
+                vlx::kSchwarzClasses[c].launch(d_blocks, (int)b, n, s->glob->boys, d_max + off[b], s->stream);
                 done = true;
             }
         }
         if (!done && n > 0) {
             const int ic = find_coop(s->glob, pb.la, pb.lb, pb.la, pb.lb);
             if (ic < 0) return fail(VLX_B200_ERR_UNSUPPORTED, "no kernel for Schwarz class");
-            VLX_CUDA(vlx::launch_coop_schwarz(s->d_blocks, (int)b, n, s->glob->coop[ic], s->glob->boys, d_max[b],
+            VLX_CUDA(vlx::launch_coop_schwarz(d_blocks, (int)b, n, s->glob->coop[ic], s->glob->boys, d_max + off[b],
                                               s->glob->nsm, s->stream));
         }
         VLX_CUDA(cudaGetLastError());
     }
+    std::vector<double> all(off[nb]);
+    VLX_CUDA(cudaMemcpyAsync(all.data(), d_max, off[nb] * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     VLX_CUDA(cudaStreamSynchronize(s->stream));
     maxv.assign(nb, {});
-    for (size_t b = 0; b < nb; b++) {
-        maxv[b].resize(s->blocks[b].pairs.size());
-        if (!maxv[b].empty())
-            VLX_CUDA(cudaMemcpy(maxv[b].data(), d_max[b], maxv[b].size() * sizeof(double), cudaMemcpyDeviceToHost));
-        cudaFree(d_max[b]);
-    }
+    for (size_t b = 0; b < nb; b++) maxv[b].assign(all.begin() + off[b], all.begin() + off[b + 1]);
     return VLX_B200_OK;
 }
 
 double class_flops(const vlx_b200_screener* s, const ClassTasks& ct, long long quartets, long long prim_quartets);
+void count_class(const vlx_b200_screener* s, const ClassTasks& ct, int nodes, int ith, int ith32, long long* q,
+                 long long* q32, long long* prim);
 
-int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, TaskSet** out)
+// Quartets and primitive quartets of one work item at the run-time thresholds,
+// and those in FP32 (the host mirror of the kernels' ket ranges).
+struct ItemCount {
+    long long quartets = 0, fp32 = 0, prim = 0;
+};
+
+void count_pair(const PairBlock& Pb, const PairBlock& Pk, int x, int kbeg, int kend, int ith, int ith32,
+                ItemCount* c)
+{
+    const int bx = Pb.bin[Pb.sorted[x]];
+    const int kmax = ith - bx;
+    const int k1 = (kmax < 0) ? kbeg : std::min(kend, Pk.bin_off[std::min(kmax, 15) + 1]);
+    if (k1 <= kbeg) return;
+    int kmid = k1;
+    if (ith32 >= 0) {
+        const int b32 = ith32 - bx;
+        const int kb32 = (b32 <= 0) ? 0 : Pk.bin_off[std::min(b32, 16)];
+        kmid = std::max(kbeg, std::min(k1, kb32));
+    }
+    c->quartets += k1 - kbeg;
+    c->fp32 += k1 - kmid;
+    c->prim += (long long)Pb.nuse[x] * (Pk.nuse_prefix[k1] - Pk.nuse_prefix[kbeg]);
+}
+
+ItemCount count_item(const vlx_b200_screener* s, const WorkItem& w, bool rows, int ith, int ith32)
+{
+    const int bra = w.blocks & 0xffff, ket = w.blocks >> 16;
+    const PairBlock& Pb = s->blocks[bra];
+    const PairBlock& Pk = s->blocks[ket];
+    ItemCount c;
+    if (!rows) {
+        count_pair(Pb, Pk, w.bra, w.kbeg, w.kend, ith, ith32, &c);
+        return c;
+    }
+    const int kend = std::min(w.kbeg + 32, (int)Pk.sorted.size());
+    for (int q = w.bra; q < w.kend; q++) {
+        const int x = Pb.row[q];
+        count_pair(Pb, Pk, x, bra == ket ? std::max(w.kbeg, x) : w.kbeg, kend, ith, ith32, &c);
+    }
+    return c;
+}
+
+// Row items of one job, each of at most `cap` steps: all bra pairs of a row
+// against 32 kets that pass the threshold with the first of them.
+template <class Emit>
+void row_items(const PairBlock& Pb, const PairBlock& Pk, int blocks, bool diag, int ith, int cap, Emit emit)
+{
+    const int nk = (int)Pk.sorted.size();
+    for (size_t r = 0; r + 1 < Pb.row_off.size(); r++) {
+        const int q0 = Pb.row_off[r], q1 = Pb.row_off[r + 1];
+        for (int k0 = 0; k0 < nk; k0 += 32) {
+            const int left = ith - Pk.bin[Pk.sorted[k0]];
+            if (left < 0) break;
+            int qe = q0 + Pb.row_bins[r][std::min(left, 15)];
+            // each pair of pairs once: kets from the bra pair on
+            if (diag) qe = std::min<int>(qe, (int)(std::upper_bound(Pb.row.begin() + q0, Pb.row.begin() + q1, k0 + 31) -
+                                                   Pb.row.begin()));
+            for (int q = q0; q < qe; q += cap) {
+                WorkItem w;
+                w.blocks = blocks;
+                w.bra = q;
+                w.kbeg = k0;
+                w.kend = std::min(q + cap, qe);
+                emit(w);
+            }
+        }
+    }
+}
+
+// ext: the list of the extended kernels (TaskSet::ext).  share: molecules that
+// share the launches (batched builds), whose items fill the SMs together.
+int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext, TaskSet** out, int share = 1)
 {
     const int ith = std::max(ith_req, s->ith_base);
     const int part = (nodes > 1) ? s->part : 0;
     for (auto& t : s->tasksets)
         if (t.ith == ith && t.rank == rank && t.nodes == nodes && t.seg == s->seg && t.tune_gen == s->tune_gen &&
-            t.part == part) {
+            t.part == part && t.ext == ext && t.share == share) {
             *out = &t;
             return VLX_B200_OK;
         }
@@ -758,6 +965,8 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, TaskSet*
     std::vector<double> load(part ? nodes : 0, 0.0);
     ts.seg = s->seg;
     ts.tune_gen = s->tune_gen;
+    ts.ext = ext;
+    ts.share = share;
     std::map<int, int> cls_index;  // key -> position in ts.classes
     long long g = 0;
     const size_t nb = s->blocks.size();
@@ -786,52 +995,70 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, TaskSet*
                 ts.classes.push_back(ct);
             }
             ClassTasks& ct = ts.classes[it->second];
-            const bool diag = (qi == qj);
-            const int nbra = (int)Pb.sorted.size();
-            const long long kp = (long long)Pb.ka * Pb.kb * Pk.ka * Pk.kb;
-            for (int x = 0; x < nbra; x++) {
-                const int bx = Pb.bin[Pb.sorted[x]];
-                const int kmax = ith - bx;
+            ct.rows = ct.compiled >= 0 && !ext;
+            ct.jobs.push_back({(int)bra, (int)ket});
+        }
+    for (ClassTasks& ct : ts.classes) {
+        // work-item length in ket pairs: a compiled-class item feeds 32 lanes
+        // per step; a cooperative-class item is walked one quartet at a time by
+        // one warp, so it stays short
+        int seg = (ct.coop >= 0) ? kCoopSegment : s->seg;
+        if (s->seg_try_compiled > 0) {
+            seg = (ct.coop >= 0) ? s->seg_try_coop : s->seg_try_compiled;
+        } else {
+            const auto tuned = s->class_seg.find(ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12));
+            if (tuned != s->class_seg.end()) seg = tuned->second;
+        }
+        const auto take = [&](const WorkItem& w) {
+            if (part) {
+                const ItemCount c = count_item(s, w, ct.rows, ith, -1);
+                int owner = 0;
+                for (int r = 1; r < nodes; r++)
+                    if (load[r] < load[owner]) owner = r;
+                load[owner] += class_flops(s, ct, c.quartets, c.prim);
+                if (owner != rank) return;
+            } else if ((g++ % nodes) != rank) {
+                return;
+            }
+            ct.items.push_back(w);
+        };
+        int cap = std::max(1, seg / kRowShare);
+        if (ct.rows) {
+            // short rows where the class has few steps, so that every SM gets
+            // several items
+            long long steps = 0;
+            for (const auto& j : ct.jobs)
+                row_items(s->blocks[j.first], s->blocks[j.second], 0, j.first == j.second, ith, 1 << 30,
+                          [&](const WorkItem& w) { steps += w.kend - w.bra; });
+            cap = (int)std::max<long long>(1, std::min<long long>(cap, steps * share / ((long long)kRowSpread * s->glob->nsm)));
+        }
+        for (const auto& j : ct.jobs) {
+            const PairBlock& Pb = s->blocks[j.first];
+            const PairBlock& Pk = s->blocks[j.second];
+            const int blocks = j.first | (j.second << 16);
+            const bool diag = j.first == j.second;
+            if (ct.rows) {
+                row_items(Pb, Pk, blocks, diag, ith, cap, take);
+                continue;
+            }
+            for (int x = 0; x < (int)Pb.sorted.size(); x++) {
+                const int kmax = ith - Pb.bin[Pb.sorted[x]];
                 if (kmax < 0) break;
                 const int kend = Pk.bin_off[std::min(kmax, 15) + 1];
-                const int kbeg = diag ? x : 0;
-                // a compiled-class item feeds 32 lanes per step; a cooperative-class
-                // item is walked one quartet at a time by one warp, so it stays short
-                int seg = (ct.coop >= 0) ? kCoopSegment : s->seg;
-                if (s->seg_try_compiled > 0) {
-                    seg = (ct.coop >= 0) ? s->seg_try_coop : s->seg_try_compiled;
-                } else {
-                    const auto tuned = s->class_seg.find(ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12));
-                    if (tuned != s->class_seg.end()) seg = tuned->second;
-                }
-                for (int k0 = kbeg; k0 < kend; k0 += seg) {
-                    const int k1 = std::min(kend, k0 + seg);
-                    if (part) {
-                        const long long prim = (long long)Pb.nuse[x] * (Pk.nuse_prefix[k1] - Pk.nuse_prefix[k0]);
-                        int owner = 0;
-                        for (int r = 1; r < nodes; r++)
-                            if (load[r] < load[owner]) owner = r;
-                        load[owner] += class_flops(s, ct, k1 - k0, prim);
-                        if (owner != rank) continue;
-                    } else if ((g++ % nodes) != rank) {
-                        continue;
-                    }
+                for (int k0 = diag ? x : 0; k0 < kend; k0 += seg) {
                     WorkItem w;
-                    w.blocks = (int)bra | ((int)ket << 16);
+                    w.blocks = blocks;
                     w.bra = x;
                     w.kbeg = k0;
-                    w.kend = k1;
-                    ct.items.push_back(w);
-                    const long long evaluated =
-                        (long long)Pb.nuse[x] * (Pk.nuse_prefix[k1] - Pk.nuse_prefix[k0]);
-                    ts.quartets += k1 - k0;
-                    ts.prim_quartets += evaluated;
-                    ct.quartets += k1 - k0;
-                    ct.prim_quartets += evaluated;
-                    ct.ref_prim_quartets += (long long)(k1 - k0) * kp;
+                    w.kend = std::min(kend, k0 + seg);
+                    take(w);
                 }
             }
         }
+        count_class(s, ct, nodes, ith, -1, &ct.quartets, nullptr, &ct.prim_quartets);
+        ts.quartets += ct.quartets;
+        ts.prim_quartets += ct.prim_quartets;
+    }
     size_t total = 0;
     for (auto& ct : ts.classes) {
         ct.offset = total;
@@ -962,7 +1189,7 @@ struct LaunchCtx {
     float* F32 = nullptr;
     const std::map<int, int>* bps = nullptr;  // per-class caps of resident blocks per SM (compiled classes)
     int bps_try = 0;                          // a cap for every compiled class (autotuning; 0: off)
-    SideStreams* side = nullptr;              // launches that cannot fill the chip run beside the others (null: in turn)
+    SideStreams* side = nullptr;              // the launches run beside each other (null: in turn on the build's stream)
 };
 
 // Enqueues all class kernels of a task set on `st`; the accumulators must be
@@ -1000,13 +1227,18 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
     const int nprec = (L.dsh ? L.tau32 > 0.0f : ith32 >= 0) ? 2 : 1;
     const int warps_per_block = vlx::kWarpsPerBlock;
     const int nsm = L.glob->nsm;
-    // One launch per class and precision.  The kernels of a class have one grid
-    // of at most one wave, and a single step of the large classes takes 0.1 to
-    // 1 ms, so a class with fewer items than the chip holds warps lasts that
-    // long however few they are, with most SMs idle: such launches go to the
-    // side streams, the slowest steps (highest angular momentum) first, and
-    // run beside each other and beside the full launches, which stay in turn on
-    // `st` (full launches side by side only share the caches).
+    // One launch per class and precision, spread over the side streams, the
+    // slowest steps (highest angular momentum) first.  A single step of the
+    // large classes takes 0.1 to 0.5 ms, so a class of few quartets lasts that
+    // long with most SMs idle, and every class ends in a nearly empty last wave;
+    // beside each other they fill the chip, and kernels of different register
+    // needs and bounds share the SMs.  One stream against 16: (H2O)1 / def2-SVP
+    // 1.69 -> 0.33 ms, (H2O)32 / def2-SVP 34.2 -> 28.6 ms, (H2O)27 / def2-TZVP
+    // 277 -> 258 ms (8 streams: 0.42 ms for the smallest, 24: the same as 16).
+    const auto variant = [&](const ClassTasks& ct) {
+        const bool sym = mode == vlx::MODE_FOCK_SYM;
+        return ct.rows ? (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN) : (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN);
+    };
     struct Launch {
         size_t c;
         int f, grid, side;
@@ -1018,7 +1250,7 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
         for (int f = 0; f < nprec; f++) {
             int wpb = warps_per_block, most = 0;
             if (ct.compiled >= 0) {
-                int occ = L.glob->resident_blocks(ct.compiled, vlx::needs_ext(a) || L.qstat);
+                int occ = L.glob->resident_blocks(ct.compiled, variant(ct), f != 0);
                 if (L.bps_try > 0) {
                     occ = std::min(occ, L.bps_try);
                 } else if (L.bps) {
@@ -1032,7 +1264,7 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
                 most = vlx::coop_blocks_per_sm(cc, f != 0) * nsm;
             }
             const int want = (int)((ct.items.size() + wpb - 1) / wpb);
-            list.push_back({c, f, std::max(1, std::min(want, most)), (L.side && !events && want <= most) ? 0 : -1});
+            list.push_back({c, f, std::max(1, std::min(want, most)), -1});
         }
     }
     const auto momentum = [&](const Launch& l) {
@@ -1040,21 +1272,15 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
         return ct.la + ct.lb + ct.lc + ct.ld;
     };
     int nside = 0;
-    for (const Launch& l : list) nside += l.side >= 0;
-    if (nside > 0 && list.size() > 1) {
-        std::stable_sort(list.begin(), list.end(), [&](const Launch& x, const Launch& y) {
-            if ((x.side >= 0) != (y.side >= 0)) return x.side >= 0;
-            return x.side >= 0 && momentum(x) > momentum(y);
-        });
+    if (L.side && !events && list.size() > 1) {
+        std::stable_sort(list.begin(), list.end(),
+                         [&](const Launch& x, const Launch& y) { return momentum(x) > momentum(y); });
         const int rc = L.side->open();
         if (rc) return rc;
-        nside = std::min(nside, SideStreams::kCount);
+        nside = std::min<int>((int)list.size(), SideStreams::kCount);
         VLX_CUDA(cudaEventRecord(L.side->fork, st));
         for (int i = 0; i < nside; i++) VLX_CUDA(cudaStreamWaitEvent(L.side->s[i], L.side->fork, 0));
-        for (size_t i = 0; i < list.size() && list[i].side >= 0; i++) list[i].side = (int)(i % nside);
-    } else {
-        nside = 0;
-        for (Launch& l : list) l.side = -1;
+        for (size_t i = 0; i < list.size(); i++) list[i].side = (int)(i % nside);
     }
     int rc = VLX_B200_OK;
     for (const Launch& l : list) {
@@ -1068,7 +1294,7 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
         const int fmode = l.f ? (mode | vlx::MODE_F32) : mode;
         if (events && l.f == 0) VLX_CUDA(cudaEventRecord((*events)[l.c].first, st));
         if (ct.compiled >= 0) {
-            vlx::kQuartetClasses[ct.compiled].launch(fmode, af, l.grid, ls);
+            vlx::kQuartetClasses[ct.compiled].launch[variant(ct)](fmode, af, l.grid, ls);
         } else {
             const cudaError_t e = vlx::launch_coop_quartet(fmode, af, L.glob->coop[ct.coop], l.grid, ls);
             if (e != cudaSuccess && !rc) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
@@ -1160,28 +1386,30 @@ int enqueue_classes(vlx_b200_screener* s, TaskSet* ts, int mode, const double* d
 }
 
 // Quartets (all, FP32 part) and primitive quartets one class evaluates at the
-// run-time thresholds (the host mirror of item_range in vlx_device.cuh).
-void count_class(const vlx_b200_screener* s, const ClassTasks& ct, int ith, int ith32, long long* q,
+// run-time thresholds: from its jobs for a full list, from its items for a
+// rank's share.
+void count_class(const vlx_b200_screener* s, const ClassTasks& ct, int nodes, int ith, int ith32, long long* q,
                  long long* q32, long long* prim)
 {
-    *q = *q32 = *prim = 0;
-    for (const WorkItem& w : ct.items) {
-        const PairBlock& Pb = s->blocks[w.blocks & 0xffff];
-        const PairBlock& Pk = s->blocks[w.blocks >> 16];
-        const int bx = Pb.bin[Pb.sorted[w.bra]];
-        const int kmax = ith - bx;
-        const int kend = (kmax < 0) ? w.kbeg : std::min(w.kend, Pk.bin_off[std::min(kmax, 15) + 1]);
-        if (kend <= w.kbeg) continue;
-        int kmid = kend;
-        if (ith32 >= 0) {
-            const int b32 = ith32 - bx;
-            const int kb32 = (b32 <= 0) ? 0 : Pk.bin_off[std::min(b32, 16)];
-            kmid = std::max(w.kbeg, std::min(kend, kb32));
+    ItemCount c;
+    if (nodes == 1) {
+        for (const auto& j : ct.jobs) {
+            const PairBlock& Pb = s->blocks[j.first];
+            const PairBlock& Pk = s->blocks[j.second];
+            for (int x = 0; x < (int)Pb.sorted.size(); x++)
+                count_pair(Pb, Pk, x, j.first == j.second ? x : 0, (int)Pk.sorted.size(), ith, ith32, &c);
         }
-        *q += kend - w.kbeg;
-        *q32 += kend - kmid;
-        *prim += (long long)Pb.nuse[w.bra] * (Pk.nuse_prefix[kend] - Pk.nuse_prefix[w.kbeg]);
+    } else {
+        for (const WorkItem& w : ct.items) {
+            const ItemCount i = count_item(s, w, ct.rows, ith, ith32);
+            c.quartets += i.quartets;
+            c.fp32 += i.fp32;
+            c.prim += i.prim;
+        }
     }
+    *q = c.quartets;
+    if (q32) *q32 = c.fp32;
+    *prim = c.prim;
 }
 
 // Algorithmic FP64 flops of one class launch: per primitive quartet the
@@ -1219,7 +1447,7 @@ int device_build(vlx_b200_screener* s, int rank, int nodes, const double* dD, in
     const float* acc32 = nullptr;
     if (known) {
         TaskSet* ts = nullptr;
-        rc = build_tasks(s, ith, rank, nodes, &ts);
+        rc = build_tasks(s, ith, rank, nodes, dscr_active(s), &ts);
         if (rc) return rc;
         const double* dI = nullptr;
         rc = internal_density(s, dD, st, &dI, launches);
@@ -1233,7 +1461,7 @@ int device_build(vlx_b200_screener* s, int rank, int nodes, const double* dD, in
                 q = pq = 0;
                 for (const ClassTasks& ct : ts->classes) {
                     long long a = 0, b = 0, c = 0;
-                    count_class(s, ct, ith, s->ith32, &a, &b, &c);
+                    count_class(s, ct, ts->nodes, ith, s->ith32, &a, &b, &c);
                     q += a;
                     pq += c;
                 }
@@ -1425,10 +1653,11 @@ int vlx_b200_screener_create(vlx_b200_screener** out, int device, int natoms, co
             s->blocks.push_back(std::move(pb));
         }
     // Schwarz diagonals on the device, in reference pair order
-    rc = upload_pairs(s, false);
+    RawPairs raw;
+    rc = raw.upload(s);
     if (rc) return cleanup(rc);
     std::vector<std::vector<double>> maxv;
-    rc = run_schwarz(s, maxv);
+    rc = run_schwarz(s, raw.d_blocks, maxv);
     if (rc) return cleanup(rc);
     for (size_t b = 0; b < s->blocks.size(); b++) {
         PairBlock& pb = s->blocks[b];
@@ -1455,8 +1684,9 @@ int vlx_b200_screener_create(vlx_b200_screener** out, int device, int natoms, co
             std::stable_sort(pb.sorted.begin() + first, pb.sorted.end(),
                              [&pb](int x, int y) { return pb.nuse_ref[x] > pb.nuse_ref[y]; });
         }
+        make_rows(pb);
     }
-    rc = upload_pairs(s, true);
+    rc = upload_pairs(s, raw);
     if (rc) return cleanup(rc);
     *out = s;
     return VLX_B200_OK;
@@ -1589,7 +1819,7 @@ int vlx_b200_fock_build_multi(vlx_b200_screener* s, int rank, int nodes, int nde
     }
     TaskSet* ts = nullptr;
     if (any) {
-        const int rc = build_tasks(s, ith, rank, nodes, &ts);
+        const int rc = build_tasks(s, ith, rank, nodes, true, &ts);
         if (rc) return rc;
     }
     vlx_b200_stats acc{};
@@ -1749,8 +1979,8 @@ int vlx_b200_fock_build_noalloc(vlx_b200_screener* s, const double* d_density, i
     TaskSet* ts = nullptr;
     for (auto& t : s->tasksets)
         if (t.ith == std::max(ith, s->ith_base) && t.rank == 0 && t.nodes == 1 && t.seg == s->seg &&
-            t.tune_gen == s->tune_gen)
-            ts = &t;
+            t.tune_gen == s->tune_gen && (!ts || ts->ext))
+            ts = &t;  // either kind of list; the plain builds' one when both exist
     if (known && !ts)
         return fail(VLX_B200_ERR_ARGUMENT,
                     "fock_build_noalloc: no work list for ithreshold " + std::to_string(ith) +
@@ -1965,7 +2195,7 @@ int vlx_b200_compute_eri(vlx_b200_screener* s, int ith, double* eri_out)
     cudaError_t e = cudaMemsetAsync(d_eri, 0, bytes, s->stream);
     if (e != cudaSuccess) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
     if (!rc) rc = ensure_buffers(s);
-    if (!rc) rc = build_tasks(s, ith, 0, 1, &ts);
+    if (!rc) rc = build_tasks(s, ith, 0, 1, true, &ts);
     if (!rc) rc = enqueue_classes(s, ts, vlx::MODE_ERI, s->d_D, s->d_acc, d_eri, 0.0, 0.0, 0.0, ith, -1, s->stream,
                                   nullptr);
     // the kernels scatter in the internal AO order: reorder into the caller's
@@ -2006,7 +2236,7 @@ int vlx_b200_fock_profile(vlx_b200_screener* s, const double* d_density, int sym
     int rc = ensure_buffers(s);
     if (rc) return rc;
     TaskSet* ts = nullptr;
-    rc = build_tasks(s, ith, 0, 1, &ts);
+    rc = build_tasks(s, ith, 0, 1, dscr_active(s), &ts);
     if (rc) return rc;
     const size_t nc = ts->classes.size();
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev(nc);
@@ -2063,7 +2293,7 @@ int vlx_b200_fock_profile(vlx_b200_screener* s, const double* d_density, int sym
             q32 = (long long)c4[2];
             pq = (long long)(c4[1] + c4[3]);
         } else {
-            count_class(s, ct, ith, s->ith32, &q, &q32, &pq);
+            count_class(s, ct, ts->nodes, ith, s->ith32, &q, &q32, &pq);
         }
         p.shell_quartets = q;
         p.prim_quartets = pq;
@@ -2258,7 +2488,7 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
     for (size_t k = 0; k < b->mols.size(); k++) {
         vlx_b200_screener* s = b->mols[k];
         TaskSet* t = nullptr;
-        int rc = build_tasks(s, ith, 0, 1, &t);
+        int rc = build_tasks(s, ith, 0, 1, false, &t, (int)b->mols.size());
         if (rc) return rc;
         for (const ClassTasks& ct : t->classes) {
             const std::array<int, 4> key{ct.la, ct.lb, ct.lc, ct.ld};
@@ -2267,6 +2497,7 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
                 ClassTasks n;
                 n.compiled = ct.compiled;
                 n.coop = ct.coop;
+                n.rows = ct.rows;
                 n.la = ct.la;
                 n.lb = ct.lb;
                 n.lc = ct.lc;
@@ -2282,7 +2513,6 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
             }
             d.quartets += ct.quartets;
             d.prim_quartets += ct.prim_quartets;
-            d.ref_prim_quartets += ct.ref_prim_quartets;
         }
         m.quartets += t->quartets;
         m.prim_quartets += t->prim_quartets;
@@ -2592,7 +2822,7 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
         s->seg_try_coop = kTuneCandidates[k].coop;
         s->tune_gen = gen0 + 1 + (int)k;
         TaskSet* ts = nullptr;
-        rc = build_tasks(s, ith, 0, 1, &ts);
+        rc = build_tasks(s, ith, 0, 1, dscr_active(s), &ts);
         if (rc) break;
         const size_t nc = ts->classes.size();
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev(nc);
@@ -2654,7 +2884,7 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
     s->class_bps.clear();
     s->tune_gen = gen0 + 1 + (int)ncand;
     TaskSet* tsb = nullptr;
-    rc = build_tasks(s, ith, 0, 1, &tsb);
+    rc = build_tasks(s, ith, 0, 1, dscr_active(s), &tsb);
     for (const int cap : kTuneBlockCaps) {
         if (rc) break;
         s->bps_try = cap;

@@ -17,6 +17,43 @@ __device__ __forceinline__ T warp_sum(T v)
     return v;
 }
 
+// Sums of N values (N <= 32) over the warp by recursive halving: at each level
+// a lane hands half of its values to its partner and keeps the other half, so
+// that N values cost about N + 5 exchanges instead of the 5 N of N separate
+// warp sums.  On return v[0] of a lane is the sum of element `e` (one lane
+// for each e in [0, N); e < 0: nothing).
+template <int N, int O, typename T>
+__device__ __forceinline__ void warp_sums_level(T* v, const int lane, int& e, int& cnt, bool& own)
+{
+    if constexpr (O > 0) {
+        const bool up = (lane & O) != 0;
+        if constexpr (N > 1) {
+            constexpr int H = (N + 1) / 2;
+#pragma unroll
+            for (int k = 0; k < H; k++) {
+                const T lo = v[k], hi = (k + H < N) ? v[k + H] : T(0);
+                v[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, O);
+            }
+            e += up ? H : 0;
+            cnt = up ? max(cnt - H, 0) : min(cnt, H);
+            warp_sums_level<H, O / 2>(v, lane, e, cnt, own);
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+            own = own && !up;
+            warp_sums_level<1, O / 2>(v, lane, e, cnt, own);
+        }
+    }
+}
+
+template <int N, typename T>
+__device__ __forceinline__ int warp_sums(T* v, const int lane)
+{
+    int e = 0, cnt = N;
+    bool own = true;
+    warp_sums_level<N, 16>(v, lane, e, cnt, own);
+    return (own && cnt > 0) ? e : -1;
+}
+
 template <typename T>
 __device__ __forceinline__ T ldD(const T* __restrict__ D, int nao, int r, int c)
 {
@@ -36,15 +73,11 @@ __device__ __forceinline__ void addF(T* F, int nao, int r, int c, T v)
 // accumulated in one orientation and the caller adds the transpose at the end.
 // T = double, or float for the FP32 digestion of FP32 quartets into the
 // separate FP32 accumulator of a density-screened build (FP32 copy of D).
-// JS > 0: jacc is the lane's part of the work item's F_PQ accumulator, element
-// e at jacc[JS e] (JS = 1: the lane's registers; JS = 32: the lane's column of
-// a per-warp shared-memory array); F_PQ is then reduced over the lanes once
-// per work item (flush_jpq) instead of once per step.
-template <int NA, int NB, int NC, int ND, int MODE, typename T, int JS = 0>
+template <int NA, int NB, int NC, int ND, int MODE, typename T>
 __device__ __forceinline__ void digest_t(const T* f, const T s, const int lane, const int p0, const int nlp,
                                          const int q0, const int nlq, const int r0, const int nlr, const int s0,
                                          const int nls, const T* __restrict__ D, T* F, const int nao, const T cjw,
-                                         const T ckw, T* jacc = nullptr)
+                                         const T ckw)
 {
     const T cj = cjw * s, ck = ckw * s;
     if (cjw != T(0)) {
@@ -63,14 +96,10 @@ __device__ __forceinline__ void digest_t(const T* f, const T s, const int lane, 
                         v = fma(f[((i * NB + j) * NC + k) * ND + l], d, v);
                     }
                 }
-                if constexpr (JS > 0) {
-                    jacc[JS * (i * NB + j)] = fma(v, cj, jacc[JS * (i * NB + j)]);
-                } else {
-                    v = warp_sum(v * cj);
-                    if (lane == ((i * NB + j) & 31)) {
-                        addF(F, nao, p0 + i * nlp, q0 + j * nlq, v);
-                        if (MODE == MODE_FOCK_GEN) addF(F, nao, q0 + j * nlq, p0 + i * nlp, v);
-                    }
+                v = warp_sum(v * cj);
+                if (lane == ((i * NB + j) & 31)) {
+                    addF(F, nao, p0 + i * nlp, q0 + j * nlq, v);
+                    if (MODE == MODE_FOCK_GEN) addF(F, nao, q0 + j * nlq, p0 + i * nlp, v);
                 }
             }
         }
@@ -176,34 +205,278 @@ __device__ __forceinline__ void digest_t(const T* f, const T s, const int lane, 
     }
 }
 
-template <int NA, int NB, int NC, int ND, int MODE, int JS = 0>
+template <int NA, int NB, int NC, int ND, int MODE>
 __device__ __forceinline__ void digest(const double* f, const double s, const int lane, const int p0, const int nlp,
                                        const int q0, const int nlq, const int r0, const int nlr, const int s0,
-                                       const int nls, const MolDev& m, const double cjw, const double ckw,
-                                       double* jacc = nullptr)
+                                       const int nls, const MolDev& m, const double cjw, const double ckw)
 {
-    digest_t<NA, NB, NC, ND, MODE, double, JS>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, m.D, m.F, m.nao,
-                                               cjw, ckw, jacc);
+    digest_t<NA, NB, NC, ND, MODE, double>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, m.D, m.F, m.nao, cjw, ckw);
 }
 
-// End of a work item with item-level F_PQ accumulation (element e of the
-// lane's part at jl[JS e]): sum each element over the lanes and add it once
-// (and its transpose for a general density).
-template <int NA, int NB, int JS>
-__device__ __forceinline__ void flush_jpq(const double* jl, const int lane, const int mode, const int p0,
-                                          const int nlp, const int q0, const int nlq, const MolDev& m)
+// ---- row items: the lanes keep their ket pair RS and the bra pairs PQ of one
+// second shell Q pass by, so the terms that do not involve P stay with the
+// lane: F_QR, F_QS and F_RS are summed in `acc` over the item and added to F
+// once (flush_row), and the elements D_QR, D_QS, D_RS are read once into `dc`.
+// Per step remain the gathers of D_PR and D_PS, the additions to F_PR and
+// F_PS, and one warp reduction of F_PQ.
+// Layout of both: [QR: NB NC | QS: NB ND | RS: NC ND], and for a general
+// density (GEN) the transposes of the first two [RQ | SQ] behind; RS then
+// stands for both orientations (D_RS + D_SR, equal additions).
+// AS, DS: element stride (1: registers, 32: the lane's column of a per-warp
+// shared-memory array; DS 0: no copy, read from D).
+template <int NB, int NC, int ND, bool GEN>
+struct RowLayout {
+    static constexpr int QS = NB * NC, RS = QS + NB * ND, T = RS + NC * ND, N = GEN ? T + RS : T;
+};
+
+template <bool TR>
+__device__ __forceinline__ double ldT(const MolDev& m, const int r, const int c)
 {
-    __syncwarp();
+    return TR ? ldD(m.D, m.nao, c, r) : ldD(m.D, m.nao, r, c);
+}
+
+template <bool TR>
+__device__ __forceinline__ void addT(const MolDev& m, const int r, const int c, const double v)
+{
+    if (TR)
+        addF(m.F, m.nao, c, r, v);
+    else
+        addF(m.F, m.nao, r, c, v);
+}
+
+// The AO indices of component 0 and the component strides of the four shells.
+struct QuartetAO {
+    int p0, q0, r0, s0, nlp, nlq, nlr, nls;
+    __device__ __forceinline__ int p(int i) const { return p0 + i * nlp; }
+    __device__ __forceinline__ int q(int j) const { return q0 + j * nlq; }
+    __device__ __forceinline__ int r(int k) const { return r0 + k * nlr; }
+    __device__ __forceinline__ int s(int l) const { return s0 + l * nls; }
+};
+
+// Exchange part of one step; TR: the transposed elements of a general density.
+template <int NA, int NB, int NC, int ND, bool TR, int AS, int DS>
+__device__ __forceinline__ void digest_row_k(const double* f, const double ck, const QuartetAO& o, const MolDev& m,
+                                             double* acc, const double* dc)
+{
+    using L = RowLayout<NB, NC, ND, TR>;
+    constexpr int base = TR ? L::T : 0;
+    {
+        double d[NA * ND];
 #pragma unroll
-    for (int e = 0; e < NA * NB; e++) {
-        const double v = warp_sum(jl[JS * e]);
-        if (lane == (e & 31)) {
-            const int i = e / NB, j = e % NB;
-            addF(m.F, m.nao, p0 + i * nlp, q0 + j * nlq, v);
-            if ((mode & 3) == MODE_FOCK_GEN) addF(m.F, m.nao, q0 + j * nlq, p0 + i * nlp, v);
+        for (int i = 0; i < NA; i++)
+#pragma unroll
+            for (int l = 0; l < ND; l++) d[i * ND + l] = ck * ldT<TR>(m, o.p(i), o.s(l));
+#pragma unroll
+        for (int j = 0; j < NB; j++)
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+                double x = acc[AS * (base + j * NC + k)];
+#pragma unroll
+                for (int i = 0; i < NA; i++)
+#pragma unroll
+                    for (int l = 0; l < ND; l++) x = fma(f[((i * NB + j) * NC + k) * ND + l], d[i * ND + l], x);
+                acc[AS * (base + j * NC + k)] = x;
+            }
+    }
+    {
+        double d[NA * NC];
+#pragma unroll
+        for (int i = 0; i < NA; i++)
+#pragma unroll
+            for (int k = 0; k < NC; k++) d[i * NC + k] = ck * ldT<TR>(m, o.p(i), o.r(k));
+#pragma unroll
+        for (int j = 0; j < NB; j++)
+#pragma unroll
+            for (int l = 0; l < ND; l++) {
+                double x = acc[AS * (base + L::QS + j * ND + l)];
+#pragma unroll
+                for (int i = 0; i < NA; i++)
+#pragma unroll
+                    for (int k = 0; k < NC; k++) x = fma(f[((i * NB + j) * NC + k) * ND + l], d[i * NC + k], x);
+                acc[AS * (base + L::QS + j * ND + l)] = x;
+            }
+    }
+    {
+        double x[NA * NC];
+#pragma unroll
+        for (int e = 0; e < NA * NC; e++) x[e] = 0.0;
+#pragma unroll
+        for (int j = 0; j < NB; j++)
+#pragma unroll
+            for (int l = 0; l < ND; l++) {
+                const double d = DS ? dc[DS * (base + L::QS + j * ND + l)] : ldT<TR>(m, o.q(j), o.s(l));
+#pragma unroll
+                for (int i = 0; i < NA; i++)
+#pragma unroll
+                    for (int k = 0; k < NC; k++)
+                        x[i * NC + k] = fma(f[((i * NB + j) * NC + k) * ND + l], d, x[i * NC + k]);
+            }
+        if (ck != 0.0) {
+#pragma unroll
+            for (int i = 0; i < NA; i++)
+#pragma unroll
+                for (int k = 0; k < NC; k++) addT<TR>(m, o.p(i), o.r(k), ck * x[i * NC + k]);
         }
     }
-    __syncwarp();
+    {
+        double x[NA * ND];
+#pragma unroll
+        for (int e = 0; e < NA * ND; e++) x[e] = 0.0;
+#pragma unroll
+        for (int j = 0; j < NB; j++)
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+                const double d = DS ? dc[DS * (base + j * NC + k)] : ldT<TR>(m, o.q(j), o.r(k));
+#pragma unroll
+                for (int i = 0; i < NA; i++)
+#pragma unroll
+                    for (int l = 0; l < ND; l++)
+                        x[i * ND + l] = fma(f[((i * NB + j) * NC + k) * ND + l], d, x[i * ND + l]);
+            }
+        if (ck != 0.0) {
+#pragma unroll
+            for (int i = 0; i < NA; i++)
+#pragma unroll
+                for (int l = 0; l < ND; l++) addT<TR>(m, o.p(i), o.s(l), ck * x[i * ND + l]);
+        }
+    }
+}
+
+// s: the permutational weight of the lane's quartet, 0 on an idle lane.
+template <int NA, int NB, int NC, int ND, bool GEN, int AS, int DS>
+__device__ __forceinline__ void digest_row(const double* f, const double s, const int lane, const QuartetAO& o,
+                                           const MolDev& m, const double cjw, const double ckw, double* acc,
+                                           const double* dc)
+{
+    using L = RowLayout<NB, NC, ND, GEN>;
+    if (cjw != 0.0) {
+        const double cj = cjw * s;
+        double d[NC * ND > NA * NB ? NC * ND : NA * NB];
+#pragma unroll
+        for (int k = 0; k < NC; k++)
+#pragma unroll
+            for (int l = 0; l < ND; l++) {
+                double x = DS ? dc[DS * (L::RS + k * ND + l)] : ldD(m.D, m.nao, o.r(k), o.s(l));
+                if (GEN && !DS) x += ldD(m.D, m.nao, o.s(l), o.r(k));
+                d[k * ND + l] = cj * x;
+            }
+        // F_PQ: chunks of up to 32 elements, each reduced over the lanes
+        constexpr int NPQ = NA * NB, NCH = (NPQ + 31) / 32, CH = (NPQ + NCH - 1) / NCH;
+#pragma unroll
+        for (int c = 0; c < NCH; c++) {
+            double v[CH];
+#pragma unroll
+            for (int e = 0; e < CH; e++) {
+                v[e] = 0.0;
+                if (c * CH + e < NPQ) {
+#pragma unroll
+                    for (int kl = 0; kl < NC * ND; kl++) v[e] = fma(f[(c * CH + e) * NC * ND + kl], d[kl], v[e]);
+                }
+            }
+            const int e = warp_sums<CH>(v, lane) + c * CH;
+            if (e >= c * CH && e < NPQ) {
+                addF(m.F, m.nao, o.p(e / NB), o.q(e % NB), v[0]);
+                if (GEN) addF(m.F, m.nao, o.q(e % NB), o.p(e / NB), v[0]);
+            }
+        }
+        // F_RS
+#pragma unroll
+        for (int i = 0; i < NA; i++)
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                double x = ldD(m.D, m.nao, o.p(i), o.q(j));
+                if (GEN) x += ldD(m.D, m.nao, o.q(j), o.p(i));
+                d[i * NB + j] = cj * x;
+            }
+#pragma unroll
+        for (int kl = 0; kl < NC * ND; kl++) {
+            double x = acc[AS * (L::RS + kl)];
+#pragma unroll
+            for (int ij = 0; ij < NA * NB; ij++) x = fma(f[ij * NC * ND + kl], d[ij], x);
+            acc[AS * (L::RS + kl)] = x;
+        }
+    }
+    if (ckw != 0.0) {
+        digest_row_k<NA, NB, NC, ND, false, AS, DS>(f, ckw * s, o, m, acc, dc);
+        if (GEN) digest_row_k<NA, NB, NC, ND, true, AS, DS>(f, ckw * s, o, m, acc, dc);
+    }
+}
+
+// Start of a row item: clears the lane's accumulators and reads its elements
+// of D (the lanes without a ket pair read a valid one's).
+template <int NB, int NC, int ND, bool TR, int DS>
+__device__ __forceinline__ void read_row_k(const QuartetAO& o, const MolDev& m, double* dc)
+{
+    using L = RowLayout<NB, NC, ND, TR>;
+    constexpr int base = TR ? L::T : 0;
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+#pragma unroll
+        for (int k = 0; k < NC; k++) dc[DS * (base + j * NC + k)] = ldT<TR>(m, o.q(j), o.r(k));
+#pragma unroll
+        for (int l = 0; l < ND; l++) dc[DS * (base + L::QS + j * ND + l)] = ldT<TR>(m, o.q(j), o.s(l));
+    }
+}
+
+template <int NB, int NC, int ND, bool GEN, int AS, int DS>
+__device__ __forceinline__ void begin_row(const QuartetAO& o, const MolDev& m, const double cj, const double ck,
+                                          double* acc, double* dc)
+{
+    using L = RowLayout<NB, NC, ND, GEN>;
+#pragma unroll
+    for (int e = 0; e < L::N; e++) acc[AS * e] = 0.0;
+    if constexpr (DS != 0) {
+        if (ck != 0.0) {
+            read_row_k<NB, NC, ND, false, DS>(o, m, dc);
+            if (GEN) read_row_k<NB, NC, ND, true, DS>(o, m, dc);
+        }
+        if (cj != 0.0) {
+#pragma unroll
+            for (int k = 0; k < NC; k++)
+#pragma unroll
+                for (int l = 0; l < ND; l++) {
+                    double x = ldD(m.D, m.nao, o.r(k), o.s(l));
+                    if (GEN) x += ldD(m.D, m.nao, o.s(l), o.r(k));
+                    dc[DS * (L::RS + k * ND + l)] = x;
+                }
+        }
+    }
+}
+
+// End of a row item: the lane's accumulators into F.
+template <int NB, int NC, int ND, bool TR, int AS>
+__device__ __forceinline__ void flush_row_k(const QuartetAO& o, const MolDev& m, const double* acc)
+{
+    using L = RowLayout<NB, NC, ND, TR>;
+    constexpr int base = TR ? L::T : 0;
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+#pragma unroll
+        for (int k = 0; k < NC; k++) addT<TR>(m, o.q(j), o.r(k), acc[AS * (base + j * NC + k)]);
+#pragma unroll
+        for (int l = 0; l < ND; l++) addT<TR>(m, o.q(j), o.s(l), acc[AS * (base + L::QS + j * ND + l)]);
+    }
+}
+
+template <int NB, int NC, int ND, bool GEN, int AS>
+__device__ __forceinline__ void flush_row(const QuartetAO& o, const MolDev& m, const double cj, const double ck,
+                                          const double* acc)
+{
+    using L = RowLayout<NB, NC, ND, GEN>;
+    if (ck != 0.0) {
+        flush_row_k<NB, NC, ND, false, AS>(o, m, acc);
+        if (GEN) flush_row_k<NB, NC, ND, true, AS>(o, m, acc);
+    }
+    if (cj != 0.0) {
+#pragma unroll
+        for (int k = 0; k < NC; k++)
+#pragma unroll
+            for (int l = 0; l < ND; l++) {
+                const double v = acc[AS * (L::RS + k * ND + l)];
+                addF(m.F, m.nao, o.r(k), o.s(l), v);
+                if (GEN) addF(m.F, m.nao, o.s(l), o.r(k), v);
+            }
+    }
 }
 
 // Scatter one unique spherical quartet into the dense ERI tensor (all eight
@@ -234,43 +507,89 @@ __device__ __forceinline__ void scatter_eri(const double* f, const int p0, const
 constexpr int kWarpsPerBlock = 4;
 
 // Per-class tuning traits, specialised in each class's generated unit from the
-// tables of gen_eri.py (BLOCKS_HINT, STAGE_BRA), so that tuning one class
-// recompiles only that unit:
-//   BlocksHint::value  minimum resident 128-thread blocks per SM the class's
-//                      register allocation must allow (0: no minimum);
-//   StageBra::value    stage the bra primitive records in shared memory per
-//                      work item (PairViewS);
-//   AccumulateJ::value where the plain kernel sums the F_PQ (J) elements of
-//                      a work item: 0 per step (warp sum and atomic add per
-//                      step), 1 per work item in registers, 2 per work item in
-//                      a per-warp shared-memory array.
-template <int LA, int LB, int LC, int LD>
+// tables of gen_eri.py (BLOCKS_HINT, STAGE_BRA, ROW_STORE), so that tuning one
+// class recompiles only that unit:
+//   BlocksHint::value  minimum resident 128-thread blocks per SM the register
+//                      allocation of a kernel variant must allow (0: no minimum);
+//   StageBra::value    the pair-item kernel stages the bra primitive records
+//                      in shared memory per work item (PairViewS);
+//   RowStore::acc, ::dc where the row-item kernels keep an item's accumulators
+//                      and elements of D (digest_row): 1 registers, 2 a
+//                      per-warp shared-memory array, 0 nowhere (acc 0: every
+//                      step is digested by itself; dc 0: read from D).
+template <int LA, int LB, int LC, int LD, int V>
 struct BlocksHint;
 template <int LA, int LB, int LC, int LD>
 struct StageBra;
-template <int LA, int LB, int LC, int LD>
-struct AccumulateJ;
+template <int LA, int LB, int LC, int LD, bool GEN>
+struct RowStore;
+
+// The Boys coefficients of the one order a class needs (the lower orders
+// follow by recursion), staged once per persistent block: the per-lane table
+// lookups then gather from shared memory instead of L1/L2.
+template <typename R>
+constexpr int boys_stride = sizeof(R) == sizeof(float) ? BOYS_STRIDE_F : BOYS_STRIDE;
+
+template <int L, typename R>
+__device__ __forceinline__ void stage_boys(const FockArgs& a, R* sboys)
+{
+    const R* tab;
+    if constexpr (sizeof(R) == sizeof(float))
+        tab = a.boys_f;
+    else
+        tab = a.boys;
+    for (int i = threadIdx.x; i < boys_stride<R>; i += blockDim.x) sboys[i] = __ldg(tab + L * boys_stride<R> + i);
+    __syncthreads();
+}
+
+// The class's integrals of one quartet, in FP64 or FP32.
+template <class C, class Bra, class Ket>
+__device__ __forceinline__ void eri_compute(const Bra& bra, const Ket& ket, const double* tab, const double omega2,
+                                            double* f)
+{
+    C::compute(bra, ket, tab, omega2, f);
+}
+template <class C, class Bra, class Ket>
+__device__ __forceinline__ void eri_compute(const Bra& bra, const Ket& ket, const float* tab, const double omega2,
+                                            float* f)
+{
+    C::compute_f32(bra, ket, tab, (float)omega2, f);
+}
+__device__ __forceinline__ PairView make_view(const PairBlockDev& b, int i, int kuse, double)
+{
+    return {b.prim + prim_offset(b.kprim, i), b.ab + ab_offset(i), kuse};
+}
+__device__ __forceinline__ PairViewF make_view(const PairBlockDev& b, int i, int kuse, float)
+{
+    return {b.primf + prim_offset(b.kprim, i), b.abf + ab_offset(i), kuse};
+}
+__device__ __forceinline__ PairViewR<double> make_row_view(const PairBlockDev& b, int q, int kuse, double)
+{
+    return {b.rprim + (size_t)q * b.kprim * 10, b.rab + 4 * (size_t)q, kuse};
+}
+__device__ __forceinline__ PairViewR<float> make_row_view(const PairBlockDev& b, int q, int kuse, float)
+{
+    return {b.rprimf + (size_t)q * b.kprim * 10, b.rabf + 4 * (size_t)q, kuse};
+}
 
 // One step of a work item: lane evaluates ket pair jj of kb against the bra
 // pair (act = false: an idle lane, which computes and contributes nothing)
 // and digests the spherical block.
-// EXT = false: the plain build (one density, the reference's screening);
-// EXT = true adds the per-quartet density screening, multi-density digestion
-// and the device quartet counters, in a separate instantiation so that the
-// plain kernels keep their code and registers.
-template <int LA, int LB, int LC, int LD, bool EXT>
-__device__ __forceinline__ void quartet_step(const FockArgs& a, const int mode, const bool f32, const int lane,
+// With the per-quartet density screening, multi-density digestion and the
+// device quartet counters; the plain builds take row_body.
+template <int LA, int LB, int LC, int LD, bool GEN, typename R>
+__device__ __forceinline__ void quartet_step(const FockArgs& a, const int mode, const int lane,
                                              const PairBlockDev& bb, const PairBlockDev& kb, const int bbi,
-                                             const int kbi, const WorkItem& w, const PairView& bra, const MolDev& m,
-                                             const int p0, const int q0, const double s_bra, const int jj,
-                                             const bool act, const double* sboys, const void* sbra,
-                                             double* jacc = nullptr)
+                                             const int kbi, const WorkItem& w, const PairViewT<R>& bra,
+                                             const MolDev& m, const int p0, const int q0, const double s_bra,
+                                             const int jj, const bool act, const R* sboys, const R* sbra)
 {
     using C = EriClass<LA, LB, LC, LD>;
+    constexpr bool f32 = sizeof(R) == sizeof(float);
     constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1, NC = 2 * LC + 1, ND = 2 * LD + 1;
     const int nlp = m.nl[LA], nlq = m.nl[LB], nlr = m.nl[LC], nls = m.nl[LD];
-    const PairView ket = make_view(kb, jj);
-    if (EXT && a.qstat) {
+    const PairViewT<R> ket = make_view(kb, jj, __ldg(kb.nuse + jj), R());
+    if (a.qstat) {
         const unsigned n = __popc(__ballot_sync(0xffffffffu, act));
         const unsigned pq = __reduce_add_sync(0xffffffffu, act ? (unsigned)(bra.kuse * ket.kuse) : 0u);
         if (lane == 0) {
@@ -278,72 +597,40 @@ __device__ __forceinline__ void quartet_step(const FockArgs& a, const int mode, 
             atomicAdd(a.qstat + 1, (unsigned long long)pq);
         }
     }
-    double f[C::NSPH];
-    if (f32) {
-        float g[C::NSPH];
-        const PairViewF ketf = make_view_f(kb, jj, ket.kuse);
-        if (StageBra<LA, LB, LC, LD>::value && sbra) {
-            PairViewS<float> bs;
-            bs.s = static_cast<const float*>(sbra);
-            bs.ab = bb.primf + 9 * (size_t)bb.kprim * bb.npairs;
-            bs.npairs = bb.npairs;
-            bs.kuse = bra.kuse;
-            bs.i = w.bra;
-            C::compute_f32(bs, ketf, reinterpret_cast<const float*>(sboys), (float)a.omega2, g);
-        } else {
-            const PairViewF braf = make_view_f(bb, w.bra, bra.kuse);
-            C::compute_f32(braf, ketf, reinterpret_cast<const float*>(sboys), (float)a.omega2, g);
-        }
-        if constexpr (EXT) {
-            // density-screened build with an FP32 accumulator: the FP32
-            // quartets (each contribution below the FP32 cutoff) are digested
-            // in FP32 against the FP32 copy of D
-            if (a.F32 != nullptr && (mode & 3) != MODE_ERI) {
-                const int r0 = __ldg(kb.ao + jj), s0 = __ldg(kb.ao + kb.npairs + jj);
-                float s = act ? (float)s_bra : 0.0f;
-                if (r0 == s0) s *= 0.5f;
-                if (bbi == kbi && jj == w.bra) s *= 0.5f;
-                if ((mode & 3) == MODE_FOCK_SYM)
-                    digest_t<NA, NB, NC, ND, MODE_FOCK_SYM, float>(g, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls,
-                                                                   a.D32, a.F32, m.nao, (float)a.cj, (float)a.ck);
-                else
-                    digest_t<NA, NB, NC, ND, MODE_FOCK_GEN, float>(g, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls,
-                                                                   a.D32, a.F32, m.nao, (float)a.cj, (float)a.ck);
-                return;
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];
-    } else if (StageBra<LA, LB, LC, LD>::value && sbra) {
-        PairViewS<double> bs;
-        bs.s = static_cast<const double*>(sbra);
-        bs.ab = bb.ab;
-        bs.npairs = bb.npairs;
+    R g[C::NSPH];
+    if (StageBra<LA, LB, LC, LD>::value && sbra) {
+        PairViewS<R> bs;
+        bs.s = sbra;
+        bs.ab = bra.ab;
         bs.kuse = bra.kuse;
-        bs.i = w.bra;
-        C::compute(bs, ket, sboys, a.omega2, f);
+        eri_compute<C>(bs, ket, sboys, a.omega2, g);
     } else {
-        C::compute(bra, ket, sboys, a.omega2, f);
+        eri_compute<C>(bra, ket, sboys, a.omega2, g);
     }
+    if constexpr (f32) {
+        // density-screened build with an FP32 accumulator: the FP32 quartets
+        // (each contribution below the FP32 cutoff) are digested in FP32
+        // against the FP32 copy of D
+        if (a.F32 != nullptr && (mode & 3) != MODE_ERI) {
+            const int r0 = __ldg(kb.ao + jj), s0 = __ldg(kb.ao + kb.npairs + jj);
+            float s = act ? (float)s_bra : 0.0f;
+            if (r0 == s0) s *= 0.5f;
+            if (bbi == kbi && jj == w.bra) s *= 0.5f;
+            digest_t<NA, NB, NC, ND, GEN ? MODE_FOCK_GEN : MODE_FOCK_SYM, float>(
+                g, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, a.D32, a.F32, m.nao, (float)a.cj, (float)a.ck);
+            return;
+        }
+    }
+    double f[C::NSPH];
+#pragma unroll
+    for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];
     const int r0 = __ldg(kb.ao + jj), s0 = __ldg(kb.ao + kb.npairs + jj);
-    const int dmode = mode & 3;
-    if (dmode == MODE_ERI) {
+    if (GEN && (mode & 3) == MODE_ERI) {
         if (act) scatter_eri<NA, NB, NC, ND>(f, p0, nlp, q0, nlq, r0, nlr, s0, nls, a.eri, m.nao);
     } else {
         double s = act ? s_bra : 0.0;
         if (r0 == s0) s *= 0.5;
         if (bbi == kbi && jj == w.bra) s *= 0.5;
-        if constexpr (!EXT) {
-            constexpr int acc = AccumulateJ<LA, LB, LC, LD>::value;
-            constexpr int js = acc == 1 ? 1 : (acc == 2 ? 32 : 0);
-            if (dmode == MODE_FOCK_SYM)
-                digest<NA, NB, NC, ND, MODE_FOCK_SYM, js>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, m, a.cj,
-                                                          a.ck, jacc);
-            else
-                digest<NA, NB, NC, ND, MODE_FOCK_GEN, js>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, m, a.cj,
-                                                          a.ck, jacc);
-            return;
-        }
         // one density, or each density of a multi-density build in turn
         const int nd = a.dens.n > 0 ? a.dens.n : 1;
 #pragma unroll 1
@@ -356,39 +643,22 @@ __device__ __forceinline__ void quartet_step(const FockArgs& a, const int mode, 
                 cj = a.dens.cj[d];
                 ck = a.dens.ck[d];
             }
-            if (dmode == MODE_FOCK_SYM)
-                digest<NA, NB, NC, ND, MODE_FOCK_SYM>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, md, cj, ck);
-            else
-                digest<NA, NB, NC, ND, MODE_FOCK_GEN>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls, md, cj, ck);
+            digest<NA, NB, NC, ND, GEN ? MODE_FOCK_GEN : MODE_FOCK_SYM>(f, s, lane, p0, nlp, q0, nlq, r0, nlr, s0, nls,
+                                                                        md, cj, ck);
         }
     }
 }
 
-template <int LA, int LB, int LC, int LD, bool EXT>
+// Pair items.
+template <int LA, int LB, int LC, int LD, bool GEN, typename R>
 __device__ __forceinline__ void quartet_body(const FockArgs& a, const int mode)
 {
-    constexpr int L = LA + LB + LC + LD;
+    constexpr bool f32 = sizeof(R) == sizeof(float);
     const int lane = threadIdx.x & 31;
-    // the Boys coefficients of the one order the class needs (the lower orders
-    // follow by recursion), staged once per persistent block: the per-lane
-    // table lookups then gather from shared memory instead of L1/L2
-    __shared__ double sboys[BOYS_NINT * BOYS_NCOEF];
+    __shared__ __align__(16) R sboys[boys_stride<R>];
     // per warp: the staged bra primitive records of the current work item
-    __shared__ __align__(16) double sbra_all[StageBra<LA, LB, LC, LD>::value ? kWarpsPerBlock * kStageBraMax * 10 : 2];
-    // per warp: the plain kernels' F_PQ accumulator of the current work item
-    // (AccumulateJ 2)
-    constexpr int NAB = (2 * LA + 1) * (2 * LB + 1);
-    __shared__ double sjacc[(!EXT && AccumulateJ<LA, LB, LC, LD>::value == 2) ? kWarpsPerBlock * 32 * NAB : 1];
-    const bool f32 = (mode & MODE_F32) != 0;
-    if (f32) {
-        float* sf = reinterpret_cast<float*>(sboys);
-        for (int i = threadIdx.x; i < BOYS_NINT * BOYS_NCOEF; i += blockDim.x)
-            sf[i] = __ldg(a.boys_f + L * BOYS_NINT * BOYS_NCOEF + i);
-    } else {
-        for (int i = threadIdx.x; i < BOYS_NINT * BOYS_NCOEF; i += blockDim.x)
-            sboys[i] = __ldg(a.boys + L * BOYS_NINT * BOYS_NCOEF + i);
-    }
-    __syncthreads();
+    __shared__ __align__(16) R sbra_all[StageBra<LA, LB, LC, LD>::value ? kWarpsPerBlock * kStageBraMax * 10 : 2];
+    stage_boys<LA + LB + LC + LD>(a, sboys);
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(a.counter, 1);
@@ -399,50 +669,20 @@ __device__ __forceinline__ void quartet_body(const FockArgs& a, const int mode)
         const PairBlockDev bb = a.blocks[bbi];
         const PairBlockDev kb = a.blocks[kbi];
         const MolDev m = a.mols ? a.mols[bb.mol] : a.mol;
-        const PairView bra = make_view(bb, w.bra);
+        const PairViewT<R> bra = make_view(bb, w.bra, __ldg(bb.nuse + w.bra), R());
         const int p0 = __ldg(bb.ao + w.bra), q0 = __ldg(bb.ao + bb.npairs + w.bra);
         const double s_bra = (p0 == q0) ? 0.5 : 1.0;
-        const void* sbra = nullptr;
+        const R* sbra = nullptr;
         if constexpr (StageBra<LA, LB, LC, LD>::value) {
             if (bra.kuse <= kStageBraMax) {
-                double* s = sbra_all + (threadIdx.x >> 5) * kStageBraMax * 10;
+                R* s = sbra_all + (threadIdx.x >> 5) * kStageBraMax * 10;
                 __syncwarp();  // the previous item's reads are done
-                if (f32)
-                    stage_bra(reinterpret_cast<float*>(s), bb.primf, bb.npairs, bb.kprim, w.bra, bra.kuse, lane);
-                else
-                    stage_bra(s, bb.prim, bb.npairs, bb.kprim, w.bra, bra.kuse, lane);
+                stage_bra(s, bra, lane);
                 __syncwarp();
                 sbra = s;
             }
         }
         int k0, k1;
-        if constexpr (!EXT) {
-            item_range(a, bb, kb, w, f32, k0, k1);
-            // the lane's part of the item's F_PQ accumulator when the item
-            // digests J into a Fock matrix (AccumulateJ)
-            constexpr int acc = AccumulateJ<LA, LB, LC, LD>::value;
-            double jreg[acc == 1 ? NAB : 1];
-            double* jl = nullptr;
-            if constexpr (acc != 0) {
-                if ((mode & 3) != MODE_ERI && a.cj != 0.0 && k0 < k1) {
-                    jl = (acc == 1) ? jreg : sjacc + (threadIdx.x >> 5) * (32 * NAB) + lane;
-#pragma unroll
-                    for (int e = 0; e < NAB; e++) jl[(acc == 1 ? 1 : 32) * e] = 0.0;
-                }
-            }
-            for (int j0 = k0; j0 < k1; j0 += 32) {
-                const int j = j0 + lane;
-                const bool act = j < k1;
-                quartet_step<LA, LB, LC, LD, false>(a, mode, f32, lane, bb, kb, bbi, kbi, w, bra, m, p0, q0, s_bra,
-                                                    act ? j : (k1 - 1), act, sboys, sbra, jl);
-            }
-            if constexpr (acc != 0) {
-                if (jl)
-                    flush_jpq<2 * LA + 1, 2 * LB + 1, (acc == 1 ? 1 : 32)>(jl, lane, mode, p0, m.nl[LA], q0,
-                                                                          m.nl[LB], m);
-            }
-            continue;
-        }
         // per warp: kets that passed the density screening, waiting for a full step
         __shared__ int squeue[kWarpsPerBlock][64];
         int* queue = squeue[threadIdx.x >> 5];
@@ -488,40 +728,193 @@ __device__ __forceinline__ void quartet_body(const FockArgs& a, const int mode)
                 n = max(n - 32, 0);
                 __syncwarp();
             }
-            quartet_step<LA, LB, LC, LD, true>(a, mode, f32, lane, bb, kb, bbi, kbi, w, bra, m, p0, q0, s_bra, jj,
-                                               act, sboys, sbra);
+            quartet_step<LA, LB, LC, LD, GEN, R>(a, mode, lane, bb, kb, bbi, kbi, w, bra, m, p0, q0, s_bra, jj, act, sboys,
+                                         sbra);
         }
     }
 }
 
-template <int LA, int LB, int LC, int LD, bool EXT>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) quartet_kernel(const FockArgs a, const int mode)
+// Row items (plain builds): lane j holds ket pair kbeg + j for the whole item
+// and the bra pairs of one second shell Q pass by (see digest_row).
+// Dynamic shared memory: the Boys order, then the accumulators and elements of
+// D that RowStore keeps there.
+template <int LA, int LB, int LC, int LD, bool GEN>
+constexpr int row_elements = RowLayout<2 * LB + 1, 2 * LC + 1, 2 * LD + 1, GEN>::N;
+
+template <int LA, int LB, int LC, int LD, bool GEN, typename R>
+constexpr int row_shared_bytes()
 {
-    quartet_body<LA, LB, LC, LD, EXT>(a, mode);
+    using Store = RowStore<LA, LB, LC, LD, GEN>;
+    return (boys_stride<R> * (int)sizeof(R) + 15) / 16 * 16 +
+           ((Store::acc == 2) + (Store::dc == 2)) * kWarpsPerBlock * 32 * row_elements<LA, LB, LC, LD, GEN> * 8;
 }
 
-template <int MB, int LA, int LB, int LC, int LD, bool EXT>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, MB) quartet_kernel_mb(const FockArgs a, const int mode)
+template <int LA, int LB, int LC, int LD, bool GEN, typename R>
+__device__ __forceinline__ void row_body(const FockArgs& a)
 {
-    quartet_body<LA, LB, LC, LD, EXT>(a, mode);
+    using C = EriClass<LA, LB, LC, LD>;
+    using Store = RowStore<LA, LB, LC, LD, GEN>;
+    constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1, NC = 2 * LC + 1, ND = 2 * LD + 1;
+    constexpr int NROW = row_elements<LA, LB, LC, LD, GEN>;
+    constexpr int AS = Store::acc == 2 ? 32 : 1, DS = Store::dc == 2 ? 32 : (Store::dc == 1 ? 1 : 0);
+    constexpr bool f32 = sizeof(R) == sizeof(float);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    extern __shared__ __align__(16) char shared[];
+    R* sboys = reinterpret_cast<R*>(shared);
+    double* sacc = reinterpret_cast<double*>(shared + (boys_stride<R> * (int)sizeof(R) + 15) / 16 * 16);
+    double* sdc = sacc + (Store::acc == 2 ? kWarpsPerBlock * 32 * NROW : 0);
+    double racc[Store::acc == 1 ? NROW : 1], rdc[Store::dc == 1 ? NROW : 1];
+    double* acc = Store::acc == 2 ? sacc + warp * (32 * NROW) + lane : racc;
+    double* dc = Store::dc == 2 ? sdc + warp * (32 * NROW) + lane : rdc;
+    stage_boys<LA + LB + LC + LD>(a, sboys);
+#pragma unroll 1
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(a.counter, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= a.nitems) return;
+        const WorkItem w = a.items[it];
+        const bool diag = (w.blocks & 0xffff) == (w.blocks >> 16);
+        const PairBlockDev& bb = a.blocks[w.blocks & 0xffff];
+        const PairBlockDev& kb = a.blocks[w.blocks >> 16];
+        const MolDev m = a.mols ? a.mols[bb.mol] : a.mol;
+        const int kl = w.kbeg + lane, jj = min(kl, kb.npairs - 1);
+        int4 head = __ldg(bb.rhead + w.bra);
+        QuartetAO o;
+        o.nlp = m.nl[LA];
+        o.nlq = m.nl[LB];
+        o.nlr = m.nl[LC];
+        o.nls = m.nl[LD];
+        o.q0 = head.z;
+        o.r0 = __ldg(kb.ao + jj);
+        o.s0 = __ldg(kb.ao + kb.npairs + jj);
+        const double s_ket = (o.r0 == o.s0) ? 0.5 : 1.0;
+        const PairViewT<R> ket = make_view(kb, jj, __ldg(kb.nuse + jj), R());
+        if constexpr (Store::acc != 0) begin_row<NB, NC, ND, GEN, AS, DS>(o, m, a.cj, a.ck, acc, dc);
+        bool any = false;
+#pragma unroll 1
+        for (int q = w.bra; q < w.kend; q++) {
+            const int4 h = head;  // the next pair's header is read a step ahead
+            if (q + 1 < w.kend) head = __ldg(bb.rhead + q + 1);
+            const int bx = h.w >> 16;
+            // the kets this launch admits for the bra pair (see item_range)
+            int k0 = diag ? h.x : 0, k1 = 0;
+            if (a.ith >= bx) k1 = __ldg(kb.bin_off + min(a.ith - bx, 15) + 1);
+            if (k1 <= w.kbeg) break;  // ascending bins: nor any later pair's
+            if (a.ith32 >= 0) {
+                const int kmid = (a.ith32 <= bx) ? 0 : __ldg(kb.bin_off + min(a.ith32 - bx, 16));
+                if (f32)
+                    k0 = max(k0, kmid);
+                else
+                    k1 = min(k1, kmid);
+            }
+            if (max(k0, w.kbeg) >= min(k1, w.kbeg + 32)) continue;
+            const bool act = kl >= k0 && kl < k1;
+            any = any || act;
+            o.p0 = h.y;
+            R g[C::NSPH];
+            eri_compute<C>(make_row_view(bb, q, h.w & 0xffff, R()), ket, sboys, a.omega2, g);
+            double f[C::NSPH];
+#pragma unroll
+            for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];
+            double s = act ? s_ket : 0.0;
+            if (o.p0 == o.q0) s *= 0.5;
+            if (diag && kl == h.x) s *= 0.5;
+            if constexpr (Store::acc != 0)
+                digest_row<NA, NB, NC, ND, GEN, AS, DS>(f, s, lane, o, m, a.cj, a.ck, acc, dc);
+            else
+                digest<NA, NB, NC, ND, GEN ? MODE_FOCK_GEN : MODE_FOCK_SYM>(f, s, lane, o.p0, o.nlp, o.q0, o.nlq, o.r0,
+                                                                            o.nlr, o.s0, o.nls, m, a.cj, a.ck);
+        }
+        if constexpr (Store::acc != 0) {
+            if (any) flush_row<NB, NC, ND, GEN, AS>(o, m, a.cj, a.ck, acc);
+        }
+    }
 }
 
-// the kernel variant of a class
-template <int LA, int LB, int LC, int LD, bool EXT>
+// Kernel variants of a class: row items (plain builds) and pair items (extended
+// builds), each for symmetric and general densities; the ERI tensor is with the
+// general pair items.  Each is a kernel of its own, so that it has only its own
+// live values.
+enum KernelVariant { ROWS_SYM = 0, ROWS_GEN = 1, PAIRS_SYM = 2, PAIRS_GEN = 3 };
+constexpr int kNumVariants = 4;
+
+template <int LA, int LB, int LC, int LD, int V, typename R>
+__device__ __forceinline__ void kernel_body(const FockArgs& a, const int mode)
+{
+    if constexpr (V >= PAIRS_SYM)
+        quartet_body<LA, LB, LC, LD, V == PAIRS_GEN, R>(a, mode);
+    else
+        row_body<LA, LB, LC, LD, V == ROWS_GEN, R>(a);
+}
+
+template <int MB, int LA, int LB, int LC, int LD, int V, typename R>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, MB) quartet_kernel(const FockArgs a, const int mode)
+{
+    kernel_body<LA, LB, LC, LD, V, R>(a, mode);
+}
+
+// without a minimum of resident blocks (a minimum of 1 is not the same: it lets
+// the compiler take far more registers)
+template <int LA, int LB, int LC, int LD, int V, typename R>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) quartet_kernel_free(const FockArgs a, const int mode)
+{
+    kernel_body<LA, LB, LC, LD, V, R>(a, mode);
+}
+
+// the kernel of a class, variant and precision, and its dynamic shared memory
+template <int LA, int LB, int LC, int LD, int V, typename R>
 constexpr auto quartet_kernel_of()
 {
-    constexpr int mb = BlocksHint<LA, LB, LC, LD>::value;
+    constexpr int mb = BlocksHint<LA, LB, LC, LD, V>::value;
     if constexpr (mb > 0)
-        return &quartet_kernel_mb<(mb > 0 ? mb : 1), LA, LB, LC, LD, EXT>;
+        return &quartet_kernel<(mb > 0 ? mb : 1), LA, LB, LC, LD, V, R>;
     else
-        return &quartet_kernel<LA, LB, LC, LD, EXT>;
+        return &quartet_kernel_free<LA, LB, LC, LD, V, R>;
 }
 
-// whether a launch needs the extended kernel (density screening,
-// multi-density digestion or quartet counters)
-__host__ __device__ __forceinline__ bool needs_ext(const FockArgs& a)
+template <int LA, int LB, int LC, int LD, int V, typename R>
+constexpr int quartet_shared_bytes()
 {
-    return a.dsh != nullptr || a.dens.n > 0 || a.qstat != nullptr;
+    if constexpr (V >= PAIRS_SYM)
+        return 0;
+    else
+        return row_shared_bytes<LA, LB, LC, LD, V == ROWS_GEN, R>();
+}
+
+template <int LA, int LB, int LC, int LD, int V, typename R>
+void launch_quartet_as(int mode, const FockArgs& a, int grid, cudaStream_t st)
+{
+    quartet_kernel_of<LA, LB, LC, LD, V, R>()<<<grid, 32 * kWarpsPerBlock,
+                                               quartet_shared_bytes<LA, LB, LC, LD, V, R>(), st>>>(a, mode);
+}
+
+template <int LA, int LB, int LC, int LD, int V>
+void launch_quartet(int mode, const FockArgs& a, int grid, cudaStream_t st)
+{
+    if (mode & MODE_F32)
+        launch_quartet_as<LA, LB, LC, LD, V, float>(mode, a, grid, st);
+    else
+        launch_quartet_as<LA, LB, LC, LD, V, double>(mode, a, grid, st);
+}
+
+// Resident blocks per SM (also sets the kernel's limit of dynamic shared
+// memory on the current device: called before its first launch there).
+template <int LA, int LB, int LC, int LD, int V, typename R>
+int occupancy_quartet_as()
+{
+    constexpr int bytes = quartet_shared_bytes<LA, LB, LC, LD, V, R>();
+    const auto kernel = quartet_kernel_of<LA, LB, LC, LD, V, R>();
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 32 * kWarpsPerBlock, bytes);
+    return n;
+}
+
+template <int LA, int LB, int LC, int LD, int V>
+int occupancy_quartet(bool f32)
+{
+    return f32 ? occupancy_quartet_as<LA, LB, LC, LD, V, float>() : occupancy_quartet_as<LA, LB, LC, LD, V, double>();
 }
 
 // max over all spherical components of (ab|ab) per pair (T4CScreener::partition)
@@ -535,7 +928,7 @@ __global__ void __launch_bounds__(64) schwarz_kernel(const PairBlockDev* blocks,
     if (i >= b.npairs) return;
     const PairView v = make_view(b, i);
     double f[C::NSPH];
-    C::compute(v, v, boys + (size_t)(2 * (LA + LB)) * BOYS_NINT * BOYS_NCOEF, 0.0, f);
+    C::compute(v, v, boys + (size_t)(2 * (LA + LB)) * BOYS_STRIDE, 0.0, f);
     double mx = 0.0;
     for (int t = 0; t < C::NSPH; t++) mx = (f[t] > mx) ? f[t] : mx;
     maxv[i] = mx;

@@ -57,9 +57,9 @@ __device__ __forceinline__ void cart_comp(int l, int c, int& x, int& y, int& z)
 __device__ void boys_all(const int M, const double T, double* F, const double* __restrict__ tab)
 {
     if (T < (double)BOYS_TMAX) {
-        const int it = (int)(T * (double)BOYS_INV_H);
-        const double x = fma(2.0 * BOYS_INV_H, T, -(double)(2 * it + 1));
-        const double* c = tab + ((size_t)(M * BOYS_NINT + it)) * BOYS_NCOEF;
+        const int it = (int)(T * (double)BOYS_INV_H + 0.5);
+        const double x = fma(2.0 * BOYS_INV_H, T, -(double)(2 * it));
+        const double* c = tab + M * BOYS_STRIDE + it * BOYS_NCOEF;
         double p = __ldg(c + BOYS_NCOEF - 1);
         for (int j = BOYS_NCOEF - 2; j >= 0; j--) p = fma(p, x, __ldg(c + j));
         F[M] = p;

@@ -1,16 +1,23 @@
 // Types shared by the host orchestration (vlx_host.cu) and the device kernels.
 #pragma once
 
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 // Boys-function Chebyshev table: orders 0..BOYS_MMAX, intervals of width
-// 1 / BOYS_INV_H on [0, BOYS_TMAX), BOYS_NCOEF coefficients per (order,
-// interval); degree 9 on half-unit intervals keeps ~3e-15 relative accuracy.
+// 1 / BOYS_INV_H centred at k / BOYS_INV_H, k = 0..BOYS_NINT - 1 (the nearest
+// integer of BOYS_INV_H T picks the interval), BOYS_NCOEF coefficients per
+// (order, interval); degree 9 on half-unit intervals keeps the rounding error.
+// Behind an order's coefficients stand e^(-k / BOYS_INV_H), k = 0..BOYS_NINT - 1.
+// The FP32 table has the same form with polynomials of degree 7 (error ~1e-12).
 #define BOYS_MMAX 16
 #define BOYS_TMAX 40
 #define BOYS_INV_H 2
-#define BOYS_NINT (BOYS_TMAX * BOYS_INV_H)
+#define BOYS_NINT (BOYS_TMAX * BOYS_INV_H + 1)
 #define BOYS_NCOEF 10
+#define BOYS_NCOEF_F 8
+#define BOYS_STRIDE (BOYS_NINT * BOYS_NCOEF + BOYS_NINT + 1)
+#define BOYS_STRIDE_F (BOYS_NINT * BOYS_NCOEF_F + BOYS_NINT + 3)
 
 // Primitive pairs whose prefactor N_a N_b S_ab sqrt(zeta) (2/sqrt(pi))^{1/2}
 // is below this bound are skipped: a primitive quartet contributes at most the
@@ -28,27 +35,43 @@ namespace vlx {
 // One pair block (shell pairs of GTO blocks (la, Ka) x (lb, Kb)), pairs sorted
 // by Schwarz bin.  Arrays live in one device allocation owned by the screener.
 struct PairBlockDev {
-    const double* prim;  // [9][kprim][npairs], per pair sorted by |kfac| descending
-    const double* ab;    // [3][npairs]  B - A
-    const float* primf;  // [9][kprim][npairs] prim rounded to FP32, then [3][npairs] ab (mixed-precision kernels)
+    // tiles of 32 pairs (the last one padded): a warp's lanes read consecutive
+    // values at offsets that are known at compile time
+    const double* prim;  // [tile][kprim][9][32], per pair sorted by |kfac| descending
+    const double* ab;    // [tile][3][32]  B - A
+    const float* primf;  // both rounded to FP32 (mixed-precision kernels)
+    const float* abf;
     const int* ao;       // [2][npairs]  AO index of component 0 of A and of B
     const int* nuse;     // [npairs]     primitive pairs with |kfac| >= VLX_PRIM_CUTOFF
     const int* bin;      // [npairs]     Schwarz bin of the pair (pairs sorted by bin)
     const int* bin_off;  // [17]         first pair of bin b (pairs with bin <= b end at bin_off[b + 1])
     const int* sh;       // [2][npairs]  shell index of A and of B (rows / columns of FockArgs::dsh)
     const float* q;      // [npairs]     Schwarz factor sqrt(max (ab|ab)), rounded up
+    // the pairs once more in row order (rows of equal second shell B, ascending
+    // pair index, so ascending bin, within a row), as the bra side of the row
+    // items reads them
+    const int4* rhead;    // [npairs]           {pair index, AO index of component 0 of A, of B, nuse | bin << 16}
+    const double* rab;    // [npairs][4]        B - A, 0
+    const double* rprim;  // [npairs][kprim][10] the 9 primitive fields of the pair, 0
+    const float* rabf;    // both rounded to FP32
+    const float* rprimf;
     int npairs;
     int kprim;
     int la, lb;
     int mol;             // molecule of the block in a batched build (index into FockArgs::mols)
 };
 
-// A run of ket pairs for one bra pair of one (bra block, ket block) job.
+// A unit of the persistent work queue, of one (bra block, ket block) job.
+// Pair item (density-screened and multi-density builds, warp-cooperative
+// classes): the bra pair `bra` against the ket pairs [kbeg, kend).
+// Row item (plain builds of the compiled classes): the bra pairs at the row
+// positions [bra, kend), all of one second shell, against the 32 ket pairs
+// from kbeg on, one per lane.
 struct WorkItem {
     int blocks;  // bra block | (ket block << 16)
-    int bra;     // bra pair index within its block
-    int kbeg;    // ket pair range [kbeg, kend) within the ket block
-    int kend;
+    int bra;     // bra pair index within its block, or first row position
+    int kbeg;    // first ket pair
+    int kend;    // end of the ket pairs, or end of the row positions
 };
 
 enum KernelMode { MODE_FOCK_SYM = 0, MODE_FOCK_GEN = 1, MODE_ERI = 2 };
