@@ -191,20 +191,57 @@ class ClassGen:
                 out.append('%s * hizh * %s' % (_num(t[1]), n[t[2]]))
         return ' + '.join(out)
 
-    def closure(self, keys):
-        """VRR nodes the given nodes depend on (themselves included), in the
-        emission order."""
-        seen, stack = set(), list(keys)
-        while stack:
-            k = stack.pop()
-            if k in seen:
-                continue
-            seen.add(k)
-            for term in self.vrr.nodes[k]:
-                for x in term[2:]:
-                    if isinstance(x, tuple):
-                        stack.append(x)
-        return [k for k in self.vrr.order if k in seen]
+    def _operands(self, key):
+        return [x for term in self.vrr.nodes[key] for x in term[2:] if isinstance(x, tuple)]
+
+    def _depth_first(self, targets, order):
+        """Nodes the targets depend on, operands before their users, in
+        depth-first order from the targets (operands sorted by `order`)."""
+        seen, out = set(), []
+
+        def visit(key):
+            if key not in seen:
+                seen.add(key)
+                for x in sorted(self._operands(key), key=order):
+                    visit(x)
+                out.append(key)
+
+        for key in targets:
+            visit(key)
+        return out
+
+    def _live(self, order):
+        """(largest, mean) number of values live at once when the nodes are
+        evaluated in this order and each target is consumed as it is made."""
+        last, live, most, total = {}, 0, 0, 0
+        for i, key in enumerate(order):
+            for x in self._operands(key):
+                last[x] = i
+        dies = {}
+        for i in last.values():
+            dies[i] = dies.get(i, 0) + 1
+        for i, key in enumerate(order):
+            live += 1
+            most, total = max(most, live), total + live
+            live -= dies.get(i, 0) + (key not in last)
+        return most, total / len(order)
+
+    def schedule(self, targets):
+        """Evaluation order of the nodes the targets need that keeps few values
+        live: of several depth-first orders, the one with the smallest largest
+        number of live values.  In creation order (graph-wide, targets consumed
+        at the end) a group of (pf|pd) kept 100 values and its 80 targets live,
+        which spilled; the best order keeps 56.
+        """
+        def size(key):
+            return -(sum(key[0]) + 1.01 * sum(key[1]) + 0.1 * key[2])
+
+        orders = [self._depth_first(ts, order)
+                  for ts in (targets, targets[::-1], sorted(targets, key=lambda k: (sum(k[1]), k[1], k[0])),
+                             sorted(targets, key=lambda k: (-sum(k[1]), k[1], k[0])),
+                             sorted(targets, key=lambda k: (-sum(k[0]), k[0], -sum(k[1]), k[1])))
+                  for order in (size, lambda k: -k[2], lambda k: k[2])]
+        return min(orders, key=self._live)
 
     def emit(self, real='double', parts=1):
         """parts > 1: the accumulator rows (bra Cartesian targets e) are
@@ -225,9 +262,11 @@ class ClassGen:
         w('template <> struct EriClass<%d, %d, %d, %d> {' % (la, lb, lc, ld))
         w('    static constexpr int NSPH = %d;' % nsph)
         method_start = len(lines)
-        w('    template <class BraT, class KetT>')
+        # the spherical integrals go to sink.put<k, l>(o), one ket component
+        # (k, l) at a time with all bra components o[i nb + j]
+        w('    template <class BraT, class KetT, class Sink>')
         w('    __device__ __forceinline__ static void compute(const BraT& bra, const KetT& ket, const double* __restrict__ btab,')
-        w('                                                   const double om2, double* __restrict__ out)')
+        w('                                                   const double om2, Sink& sink)')
         w('    {')
         groups = [list(range(len(e_t)))[r::parts] for r in range(parts)]
         if parts > 1:
@@ -307,12 +346,11 @@ class ClassGen:
         w('                (void)WPx; (void)WPy; (void)WPz; (void)WQx; (void)WQy; (void)WQz;')
         w('                (void)QDx; (void)QDy; (void)QDz; (void)PBx; (void)PBy; (void)PBz;')
         w('                (void)hiz; (void)hie; (void)hizh; (void)rz; (void)rh;')
-        needed = self.closure([(e_t[ie], f, 0) for ie in group for f in f_t])
-        for key in needed:
+        target = {(e_t[ie], f, 0): 'c_%d_%d' % (ie, jf) for ie in group for jf, f in enumerate(f_t)}
+        for key in self.schedule(list(target)):
             w('                const double %s = %s;' % (self.names[key], self._vrr_expr(key)))
-        for ie in group:
-            for jf, f in enumerate(f_t):
-                w('                c_%d_%d += %s;' % (ie, jf, self.names[(e_t[ie], f, 0)]))
+            if key in target:
+                w('                %s += %s;' % (target[key], self.names[key]))
         w('            }')
         w('        }')
         # ---- ket HRR (per e target) then ket spherical
@@ -397,6 +435,7 @@ class ClassGen:
         for k in range(nc):
             for l in range(nd):
                 names = {}
+                w('        double o%d_%d[%d];' % (k, l, na * nb))
                 for n_, key in enumerate(bra_order):
                     node = bra_nodes[key]
                     nm = 'b%d_%d_%d' % (k, l, n_)
@@ -415,7 +454,8 @@ class ClassGen:
                                 if sph_b[j][jb] == 0.0:
                                     continue
                                 terms.append('%s * %s' % (_num(sph_a[i][ia] * sph_b[j][jb]), names[(a, b)]))
-                        w('        out[%d] = %s;' % (((i * nb + j) * nc + k) * nd + l, ' + '.join(terms)))
+                        w('        o%d_%d[%d] = %s;' % (k, l, i * nb + j, ' + '.join(terms)))
+                w('        sink.template put<%d, %d>(o%d_%d);' % (k, l, k, l))
 
 
 
@@ -581,7 +621,7 @@ def to_f32(method_lines):
     for line in method_lines:
         t = line.replace('static void compute(', 'static void compute_f32(')
         t = t.replace('const double* __restrict__ btab', 'const float* __restrict__ btab')
-        t = t.replace('double* __restrict__ out', 'float* __restrict__ out')
+        t = re.sub(r'\bdouble (o\d+_\d+\[)', r'float \1', t)
         t = t.replace('const double ', 'const float ').replace('double c_', 'float c_').replace('double F[', 'float F[')
         t = t.replace('double h_', 'float h_')
         t = t.replace('boys_scaled<', 'boys_scaled_f<').replace('rsqrt_pos(', 'rsqrtf(')
@@ -649,8 +689,10 @@ def emit_class_file(cls, outdir):
     w('template <> struct StageBra<%d, %d, %d, %d> { static constexpr bool value = %s; };'
       % (cls + ('true' if cls in STAGE_BRA else 'false',)))
     for gen in (0, 1):
-        w('template <> struct RowStore<%d, %d, %d, %d, %s> { static constexpr int acc = %d, dc = %d; };'
-          % (cls + ('true' if gen else 'false',) + row_store(cls, gen)))
+        w('template <> struct RowStore<%d, %d, %d, %d, %s> { static constexpr int acc = %d, dc = %d; '
+          'static constexpr bool stream = %s; };'
+          % (cls + ('true' if gen else 'false',) + row_store(cls, gen) +
+             ('true' if row_store(cls, gen)[0] == 0 and not gen and cls not in ROW_ARRAY else 'false',)))
     w(g.emit(parts=class_parts(cls)))
     w('}  // namespace vlx')
     write_if_changed(outdir / ('class_%s.inc' % nm), '\n'.join(body) + '\n')
@@ -716,7 +758,13 @@ STAGE_BRA = {(0, 0, 0, 0), (0, 1, 0, 0), (1, 1, 0, 0), (0, 2, 0, 0), (2, 2, 1, 2
 
 # Where the row-item kernels keep an item's accumulators and elements of D
 # (RowStore in vlx_kernels.cuh) for the classes that differ from row_store's
-# rule: class -> (acc, dc), for symmetric and general densities.
+# rule: class -> (acc, dc), for symmetric and general densities.  The rule, both
+# in shared memory up to 39 elements (two blocks of 80 KB per SM), is from
+# timings of the s, p and d classes on the (H2O)32 / def2-SVP build: registers
+# instead 35.7 ms, accumulators only 38.0, neither 49, both 34.2; classes of more
+# elements lose more to the smaller L1 than they gain, and (pd|pp) is fastest
+# with D in registers (2.35 against 2.49 ms).  Register caps (BLOCKS_HINT) were
+# slower for every class.
 ROW_STORE = ({(1, 2, 1, 1): (2, 1)}, {})
 
 
@@ -726,6 +774,13 @@ def row_store(cls, gen):
     nb, nc, nd = (2 * l + 1 for l in cls[1:])
     n = nb * (nc + nd) * (2 if gen else 1) + nc * nd
     return (2, 2) if n <= 39 else (0, 0)
+
+
+# Classes whose row-item kernel (symmetric density) keeps the block of integrals
+# of a step in an array although it has no row accumulators: measured faster
+# than streaming the block through the digestion (StreamSink) on the
+# (H2O)27 / def2-TZVP build, by 3 to 20%.
+ROW_ARRAY = {(0, 3, 1, 1), (0, 3, 1, 2), (1, 3, 1, 1), (0, 3, 0, 2), (0, 3, 0, 3), (1, 3, 0, 2)}
 
 
 def class_parts(cls):

@@ -433,6 +433,7 @@ struct PairBlock {
     std::vector<int> nuse_ref;               // reference order: significant primitive pairs
     std::vector<int> nuse;                   // sorted order: significant primitive pairs
     std::vector<long long> nuse_prefix;      // sorted order: prefix sums of nuse
+    int nuse_max = 0;
     // the sorted pairs by rows of equal second shell (ascending sorted position
     // within a row): sorted position per row position, row starts, and per row
     // the number of pairs of bin <= b
@@ -468,6 +469,7 @@ struct ClassTasks {
     std::vector<WorkItem> items;
     bool rows = false;                        // row items (else pair items)
     std::vector<std::pair<int, int>> jobs;    // (bra block, ket block) of the class; complete when nodes == 1
+    double step_cost = 0.0;                   // operations of one quartet of its most contracted pairs
     size_t offset = 0;  // first item in the task set's device array
     long long quartets = 0, prim_quartets = 0;  // at the task set's threshold
 };
@@ -487,7 +489,7 @@ struct TaskSet {
 // Streams beside a build's own for its class launches (enqueue_ctx), made on
 // first use and owned by a screener or a batch.
 struct SideStreams {
-    static constexpr int kCount = 16;
+    static constexpr int kCount = 24;
     cudaStream_t s[kCount] = {};
     cudaEvent_t fork = nullptr, join[kCount] = {};
     bool ready = false;
@@ -767,6 +769,7 @@ int upload_pairs(vlx_b200_screener* s, const RawPairs& raw)
             ao[i] = s->shells[pb.pairs[ref].first].ao0;
             ao[n + i] = s->shells[pb.pairs[ref].second].ao0;
             nuse[i] = pb.nuse[i] = pb.nuse_ref[ref];
+            pb.nuse_max = std::max(pb.nuse_max, nuse[i]);
             pb.nuse_prefix[i + 1] = pb.nuse_prefix[i] + pb.nuse[i];
             bins[i] = pb.bin[ref];
             shl[i] = pb.pairs[ref].first;
@@ -999,6 +1002,9 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
             ct.jobs.push_back({(int)bra, (int)ket});
         }
     for (ClassTasks& ct : ts.classes) {
+        for (const auto& j : ct.jobs)
+            ct.step_cost = std::max(ct.step_cost, class_flops(s, ct, 1, (long long)s->blocks[j.first].nuse_max *
+                                                                            s->blocks[j.second].nuse_max));
         // work-item length in ket pairs: a compiled-class item feeds 32 lanes
         // per step; a cooperative-class item is walked one quartet at a time by
         // one warp, so it stays short
@@ -1228,13 +1234,15 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
     const int warps_per_block = vlx::kWarpsPerBlock;
     const int nsm = L.glob->nsm;
     // One launch per class and precision, spread over the side streams, the
-    // slowest steps (highest angular momentum) first.  A single step of the
-    // large classes takes 0.1 to 0.5 ms, so a class of few quartets lasts that
-    // long with most SMs idle, and every class ends in a nearly empty last wave;
-    // beside each other they fill the chip, and kernels of different register
-    // needs and bounds share the SMs.  One stream against 16: (H2O)1 / def2-SVP
-    // 1.69 -> 0.33 ms, (H2O)32 / def2-SVP 34.2 -> 28.6 ms, (H2O)27 / def2-TZVP
-    // 277 -> 258 ms (8 streams: 0.42 ms for the smallest, 24: the same as 16).
+    // longest steps first.  A single step of the large classes, or of the most
+    // contracted pairs of the small ones, takes 0.1 to 0.5 ms, so a class of few
+    // quartets lasts that long with most SMs idle, and every class ends in a
+    // nearly empty last wave; beside each other they fill the chip, and kernels
+    // of different register needs and bounds share the SMs.  Against one stream:
+    // (H2O)1 / def2-SVP 1.69 -> 0.28 ms, (H2O)32 / def2-SVP 34.2 -> 28.6 ms, (H2O)27 /
+    // def2-TZVP 277 -> 258 ms.  8 streams: 0.42 ms for the smallest, 16: 0.33, 32: as
+    // 24; the same launches replayed as a graph: 0.30 ms, but 0.54 instead of
+    // 0.46 ms for (H2O)4.
     const auto variant = [&](const ClassTasks& ct) {
         const bool sym = mode == vlx::MODE_FOCK_SYM;
         return ct.rows ? (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN) : (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN);
@@ -1267,14 +1275,11 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
             list.push_back({c, f, std::max(1, std::min(want, most)), -1});
         }
     }
-    const auto momentum = [&](const Launch& l) {
-        const ClassTasks& ct = ts->classes[l.c];
-        return ct.la + ct.lb + ct.lc + ct.ld;
-    };
     int nside = 0;
     if (L.side && !events && list.size() > 1) {
-        std::stable_sort(list.begin(), list.end(),
-                         [&](const Launch& x, const Launch& y) { return momentum(x) > momentum(y); });
+        std::stable_sort(list.begin(), list.end(), [&](const Launch& x, const Launch& y) {
+            return ts->classes[x.c].step_cost > ts->classes[y.c].step_cost;
+        });
         const int rc = L.side->open();
         if (rc) return rc;
         nside = std::min<int>((int)list.size(), SideStreams::kCount);
@@ -2512,6 +2517,7 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
                 d.items.push_back(w);
             }
             d.quartets += ct.quartets;
+            d.step_cost = std::max(d.step_cost, ct.step_cost);
             d.prim_quartets += ct.prim_quartets;
         }
         m.quartets += t->quartets;

@@ -516,7 +516,8 @@ constexpr int kWarpsPerBlock = 4;
 //   RowStore::acc, ::dc where the row-item kernels keep an item's accumulators
 //                      and elements of D (digest_row): 1 registers, 2 a
 //                      per-warp shared-memory array, 0 nowhere (acc 0: every
-//                      step is digested by itself; dc 0: read from D).
+//                      step is digested by itself; dc 0: read from D);
+//   RowStore::stream   a step's integrals go through StreamSink.
 template <int LA, int LB, int LC, int LD, int V>
 struct BlocksHint;
 template <int LA, int LB, int LC, int LD>
@@ -542,19 +543,133 @@ __device__ __forceinline__ void stage_boys(const FockArgs& a, R* sboys)
     __syncthreads();
 }
 
-// The class's integrals of one quartet, in FP64 or FP32.
-template <class C, class Bra, class Ket>
+// Takes a quartet's integrals into the array f[((i NB + j) NC + k) ND + l].
+template <int NAB, int NC, int ND, typename R>
+struct ArraySink {
+    R* f;
+    template <int K, int L>
+    __device__ __forceinline__ void put(const R* o)
+    {
+#pragma unroll
+        for (int ij = 0; ij < NAB; ij++) f[(ij * NC + K) * ND + L] = o[ij];
+    }
+};
+
+// The class's integrals of one quartet, in FP64 or FP32 by the type of the
+// Boys table, into a sink.
+template <class C, class Bra, class Ket, class Sink>
 __device__ __forceinline__ void eri_compute(const Bra& bra, const Ket& ket, const double* tab, const double omega2,
-                                            double* f)
+                                            Sink& sink)
 {
-    C::compute(bra, ket, tab, omega2, f);
+    C::compute(bra, ket, tab, omega2, sink);
 }
-template <class C, class Bra, class Ket>
+template <class C, class Bra, class Ket, class Sink>
 __device__ __forceinline__ void eri_compute(const Bra& bra, const Ket& ket, const float* tab, const double omega2,
-                                            float* f)
+                                            Sink& sink)
 {
-    C::compute_f32(bra, ket, tab, (float)omega2, f);
+    C::compute_f32(bra, ket, tab, (float)omega2, sink);
 }
+
+// J/K digestion of one quartet (symmetric density) as its integrals arrive, one
+// ket component (k, l) at a time: the classes whose block f does not fit the
+// registers (up to 49 x 49 values) need no array of it, which a lane would
+// write once and read six times through thread-local memory ((pf|pd) of the
+// (H2O)27 / def2-TZVP build 15.0 -> 12.4 ms, (pd|pd) 7.5 -> 6.4, the build
+// 246 -> 237).
+// s: the permutational weight, 0 on an idle lane.
+template <int NA, int NB, int NC, int ND, typename R>
+struct StreamSink {
+    const QuartetAO& o;
+    const MolDev& m;
+    const double cj, ck;  // weights of the label times s
+    const bool j_on, k_on;
+    double pq[NA * NB], qr[NB], pr[NA], qs[NB * ND], ps[NA * ND];
+
+    __device__ __forceinline__ StreamSink(const QuartetAO& ao, const MolDev& mol, const double cjw, const double ckw,
+                                          const double s)
+        : o(ao), m(mol), cj(cjw * s), ck(ckw * s), j_on(cjw != 0.0), k_on(ckw != 0.0)
+    {
+#pragma unroll
+        for (int e = 0; e < NA * NB; e++) pq[e] = 0.0;
+#pragma unroll
+        for (int e = 0; e < NB * ND; e++) qs[e] = 0.0;
+#pragma unroll
+        for (int e = 0; e < NA * ND; e++) ps[e] = 0.0;
+    }
+
+    template <int K, int L>
+    __device__ __forceinline__ void put(const R* f)
+    {
+        if (j_on) {
+            const double d = cj * ldD(m.D, m.nao, o.r(K), o.s(L));
+            double x = 0.0;
+#pragma unroll
+            for (int i = 0; i < NA; i++)
+#pragma unroll
+                for (int j = 0; j < NB; j++) {
+                    const double v = (double)f[i * NB + j];
+                    pq[i * NB + j] = fma(v, d, pq[i * NB + j]);
+                    x = fma(v, ldD(m.D, m.nao, o.p(i), o.q(j)), x);
+                }
+            if (cj != 0.0) addF(m.F, m.nao, o.r(K), o.s(L), cj * x);
+        }
+        if (k_on) {
+            if (L == 0) {
+#pragma unroll
+                for (int j = 0; j < NB; j++) qr[j] = 0.0;
+#pragma unroll
+                for (int i = 0; i < NA; i++) pr[i] = 0.0;
+            }
+            double dqr[NB], dqs[NB];
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                dqr[j] = ldD(m.D, m.nao, o.q(j), o.r(K));
+                dqs[j] = ldD(m.D, m.nao, o.q(j), o.s(L));
+            }
+#pragma unroll
+            for (int i = 0; i < NA; i++) {
+                const double dpr = ldD(m.D, m.nao, o.p(i), o.r(K)), dps = ldD(m.D, m.nao, o.p(i), o.s(L));
+#pragma unroll
+                for (int j = 0; j < NB; j++) {
+                    const double v = (double)f[i * NB + j];
+                    qr[j] = fma(v, dps, qr[j]);
+                    pr[i] = fma(v, dqs[j], pr[i]);
+                    qs[j * ND + L] = fma(v, dpr, qs[j * ND + L]);
+                    ps[i * ND + L] = fma(v, dqr[j], ps[i * ND + L]);
+                }
+            }
+            if (ck != 0.0) {
+                if (L == ND - 1) {
+#pragma unroll
+                    for (int j = 0; j < NB; j++) addF(m.F, m.nao, o.q(j), o.r(K), ck * qr[j]);
+#pragma unroll
+                    for (int i = 0; i < NA; i++) addF(m.F, m.nao, o.p(i), o.r(K), ck * pr[i]);
+                }
+                if (K == NC - 1) {
+#pragma unroll
+                    for (int j = 0; j < NB; j++) addF(m.F, m.nao, o.q(j), o.s(L), ck * qs[j * ND + L]);
+#pragma unroll
+                    for (int i = 0; i < NA; i++) addF(m.F, m.nao, o.p(i), o.s(L), ck * ps[i * ND + L]);
+                }
+            }
+        }
+    }
+
+    // F_PQ over the lanes (all lanes of the warp)
+    __device__ __forceinline__ void finish(const int lane)
+    {
+        if (!j_on) return;
+        constexpr int NPQ = NA * NB, NCH = (NPQ + 31) / 32, CH = (NPQ + NCH - 1) / NCH;
+#pragma unroll
+        for (int c = 0; c < NCH; c++) {
+            double v[CH];
+#pragma unroll
+            for (int e = 0; e < CH; e++) v[e] = (c * CH + e < NPQ) ? pq[c * CH + e] : 0.0;
+            const int e = warp_sums<CH>(v, lane) + c * CH;
+            if (e >= c * CH && e < NPQ) addF(m.F, m.nao, o.p(e / NB), o.q(e % NB), v[0]);
+        }
+    }
+};
 __device__ __forceinline__ PairView make_view(const PairBlockDev& b, int i, int kuse, double)
 {
     return {b.prim + prim_offset(b.kprim, i), b.ab + ab_offset(i), kuse};
@@ -598,14 +713,15 @@ __device__ __forceinline__ void quartet_step(const FockArgs& a, const int mode, 
         }
     }
     R g[C::NSPH];
+    ArraySink<NA * NB, NC, ND, R> sink{g};
     if (StageBra<LA, LB, LC, LD>::value && sbra) {
         PairViewS<R> bs;
         bs.s = sbra;
         bs.ab = bra.ab;
         bs.kuse = bra.kuse;
-        eri_compute<C>(bs, ket, sboys, a.omega2, g);
+        eri_compute<C>(bs, ket, sboys, a.omega2, sink);
     } else {
-        eri_compute<C>(bra, ket, sboys, a.omega2, g);
+        eri_compute<C>(bra, ket, sboys, a.omega2, sink);
     }
     if constexpr (f32) {
         // density-screened build with an FP32 accumulator: the FP32 quartets
@@ -758,6 +874,12 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
     constexpr int NROW = row_elements<LA, LB, LC, LD, GEN>;
     constexpr int AS = Store::acc == 2 ? 32 : 1, DS = Store::dc == 2 ? 32 : (Store::dc == 1 ? 1 : 0);
     constexpr bool f32 = sizeof(R) == sizeof(float);
+    // the straight-line code of a step of the large classes (up to hundreds of
+    // KB) does not fit the instruction caches, least of all beside other
+    // classes' kernels: the warps of a block walk their items in step, so that it
+    // is fetched once for all of them ((H2O)27 / def2-TZVP build 236 -> 228 ms;
+    // each class by itself 3% slower to 18% faster)
+    constexpr bool LOCK = Store::acc == 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     extern __shared__ __align__(16) char shared[];
     R* sboys = reinterpret_cast<R*>(shared);
@@ -769,11 +891,34 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
     stage_boys<LA + LB + LC + LD>(a, sboys);
 #pragma unroll 1
     for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(a.counter, 1);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= a.nitems) return;
-        const WorkItem w = a.items[it];
+        WorkItem w;
+        int steps;
+        if constexpr (LOCK) {
+            // four consecutive items for the block's warps, walked in step
+            __shared__ int first;
+            __syncthreads();
+            if (threadIdx.x == 0) first = atomicAdd(a.counter, kWarpsPerBlock);
+            __syncthreads();
+            const int base = first;
+            if (base >= a.nitems) return;
+            steps = 0;
+            for (int v = 0; v < kWarpsPerBlock; v++) {
+                const int it = min(base + v, a.nitems - 1);
+                const WorkItem x = a.items[it];
+                steps = max(steps, x.kend - x.bra);
+                if (v == warp) {
+                    w = x;
+                    if (base + v >= a.nitems) w.kend = w.bra;  // no item for this warp
+                }
+            }
+        } else {
+            int it = 0;
+            if (lane == 0) it = atomicAdd(a.counter, 1);
+            it = __shfl_sync(0xffffffffu, it, 0);
+            if (it >= a.nitems) return;
+            w = a.items[it];
+            steps = w.kend - w.bra;
+        }
         const bool diag = (w.blocks & 0xffff) == (w.blocks >> 16);
         const PairBlockDev& bb = a.blocks[w.blocks & 0xffff];
         const PairBlockDev& kb = a.blocks[w.blocks >> 16];
@@ -793,14 +938,23 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
         if constexpr (Store::acc != 0) begin_row<NB, NC, ND, GEN, AS, DS>(o, m, a.cj, a.ck, acc, dc);
         bool any = false;
 #pragma unroll 1
-        for (int q = w.bra; q < w.kend; q++) {
+        for (int x = 0; x < steps; x++) {
+            if constexpr (LOCK) {
+                __syncthreads();
+                if (w.bra + x >= w.kend) continue;
+            }
+            const int q = w.bra + x;
             const int4 h = head;  // the next pair's header is read a step ahead
             if (q + 1 < w.kend) head = __ldg(bb.rhead + q + 1);
             const int bx = h.w >> 16;
             // the kets this launch admits for the bra pair (see item_range)
             int k0 = diag ? h.x : 0, k1 = 0;
             if (a.ith >= bx) k1 = __ldg(kb.bin_off + min(a.ith - bx, 15) + 1);
-            if (k1 <= w.kbeg) break;  // ascending bins: nor any later pair's
+            if (k1 <= w.kbeg) {  // ascending bins: nor any later pair's
+                if (!LOCK) break;
+                w.kend = q;
+                continue;
+            }
             if (a.ith32 >= 0) {
                 const int kmid = (a.ith32 <= bx) ? 0 : __ldg(kb.bin_off + min(a.ith32 - bx, 16));
                 if (f32)
@@ -812,19 +966,26 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
             const bool act = kl >= k0 && kl < k1;
             any = any || act;
             o.p0 = h.y;
-            R g[C::NSPH];
-            eri_compute<C>(make_row_view(bb, q, h.w & 0xffff, R()), ket, sboys, a.omega2, g);
-            double f[C::NSPH];
-#pragma unroll
-            for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];
             double s = act ? s_ket : 0.0;
             if (o.p0 == o.q0) s *= 0.5;
             if (diag && kl == h.x) s *= 0.5;
-            if constexpr (Store::acc != 0)
-                digest_row<NA, NB, NC, ND, GEN, AS, DS>(f, s, lane, o, m, a.cj, a.ck, acc, dc);
-            else
-                digest<NA, NB, NC, ND, GEN ? MODE_FOCK_GEN : MODE_FOCK_SYM>(f, s, lane, o.p0, o.nlp, o.q0, o.nlq, o.r0,
-                                                                            o.nlr, o.s0, o.nls, m, a.cj, a.ck);
+            if constexpr (Store::stream) {
+                StreamSink<NA, NB, NC, ND, R> sink(o, m, a.cj, a.ck, s);
+                eri_compute<C>(make_row_view(bb, q, h.w & 0xffff, R()), ket, sboys, a.omega2, sink);
+                sink.finish(lane);
+            } else {
+                R g[C::NSPH];
+                ArraySink<NA * NB, NC, ND, R> sink{g};
+                eri_compute<C>(make_row_view(bb, q, h.w & 0xffff, R()), ket, sboys, a.omega2, sink);
+                double f[C::NSPH];
+#pragma unroll
+                for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];
+                if constexpr (Store::acc != 0)
+                    digest_row<NA, NB, NC, ND, GEN, AS, DS>(f, s, lane, o, m, a.cj, a.ck, acc, dc);
+                else
+                    digest<NA, NB, NC, ND, GEN ? MODE_FOCK_GEN : MODE_FOCK_SYM>(
+                        f, s, lane, o.p0, o.nlp, o.q0, o.nlq, o.r0, o.nlr, o.s0, o.nls, m, a.cj, a.ck);
+            }
         }
         if constexpr (Store::acc != 0) {
             if (any) flush_row<NB, NC, ND, GEN, AS>(o, m, a.cj, a.ck, acc);
@@ -928,7 +1089,9 @@ __global__ void __launch_bounds__(64) schwarz_kernel(const PairBlockDev* blocks,
     if (i >= b.npairs) return;
     const PairView v = make_view(b, i);
     double f[C::NSPH];
-    C::compute(v, v, boys + (size_t)(2 * (LA + LB)) * BOYS_STRIDE, 0.0, f);
+    constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1;
+    ArraySink<NA * NB, NA, NB, double> sink{f};
+    C::compute(v, v, boys + (size_t)(2 * (LA + LB)) * BOYS_STRIDE, 0.0, sink);
     double mx = 0.0;
     for (int t = 0; t < C::NSPH; t++) mx = (f[t] > mx) ? f[t] : mx;
     maxv[i] = mx;
