@@ -369,7 +369,7 @@ __global__ void coop_quartet_kernel(const FockArgs a, const CoopClassDev c, cons
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= a.nitems) return;
         const WorkItem w = a.items[it];
-        const int bbi = w.blocks & 0xffff, kbi = w.blocks >> 16;
+        const int bbi = w.blocks & 0xffff, kbi = (unsigned)w.blocks >> 16;
         const PairBlockDev bb = a.blocks[bbi];
         const PairBlockDev kb = a.blocks[kbi];
         const MolDev m = a.mols ? a.mols[bb.mol] : a.mol;

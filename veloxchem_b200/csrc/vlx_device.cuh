@@ -183,6 +183,9 @@ __device__ __forceinline__ double rsqrt_pos(const double x)
 // the low word: no conversion instructions.
 // tabM: the BOYS_STRIDE values of order M (global or shared memory: the class
 // kernels stage their order in shared memory).
+// Against intervals by truncation, the library's exponential and reciprocal
+// root, and a division beyond BOYS_TMAX: the (H2O)32 / def2-SVP build 43.0 -> 37.5
+// ms (sum of its classes).
 // F[m] = sc F_m(T), m = 0..M: the scale enters the highest order (or F_0) and
 // e^{-T} once, and the recursions carry it to the other orders.
 __device__ __forceinline__ double boys_exp(const double x, const int k, const double* __restrict__ tabM)

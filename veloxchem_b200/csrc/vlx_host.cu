@@ -697,7 +697,7 @@ __global__ void gather_pairs_kernel(const PairBlockDev* __restrict__ raw, const 
     const PairBlockDev b = blocks[blockIdx.y], r = raw[blockIdx.y];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < b.npairs; i += gridDim.x * blockDim.x) {
         const int from = src[blockIdx.y][i], q = pos[blockIdx.y][i];
-        const_cast<int4*>(b.rhead)[q] = make_int4(i, b.ao[i], b.ao[b.npairs + i], b.nuse[i] | (b.bin[i] << 16));
+        const_cast<int4*>(b.rhead)[q] = make_int4(i, b.ao[i], b.ao[b.npairs + i], b.bin[i] | (b.nuse[i] << 4));
         const double* ab = r.ab + vlx::ab_offset(from);
         for (int x = 0; x < 4; x++) {
             const double v = x < 3 ? ab[32 * x] : 0.0;
@@ -902,7 +902,7 @@ void count_pair(const PairBlock& Pb, const PairBlock& Pk, int x, int kbeg, int k
 
 ItemCount count_item(const vlx_b200_screener* s, const WorkItem& w, bool rows, int ith, int ith32)
 {
-    const int bra = w.blocks & 0xffff, ket = w.blocks >> 16;
+    const int bra = w.blocks & 0xffff, ket = (unsigned)w.blocks >> 16;
     const PairBlock& Pb = s->blocks[bra];
     const PairBlock& Pk = s->blocks[ket];
     ItemCount c;
@@ -2512,7 +2512,7 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
             }
             ClassTasks& d = m.classes[it->second];
             for (WorkItem w : ct.items) {
-                const int bb = (w.blocks & 0xffff) + boff, kb = (w.blocks >> 16) + boff;
+                const int bb = (w.blocks & 0xffff) + boff, kb = ((unsigned)w.blocks >> 16) + boff;
                 w.blocks = bb | (kb << 16);
                 d.items.push_back(w);
             }

@@ -1,8 +1,11 @@
-// Kernel templates instantiated once per quartet class by the generated
-// translation units (gen_eri.py).  One warp owns one work item: a bra shell
-// pair (warp-uniform) against a run of ket shell pairs, one ket pair per lane.
-// Work items are pulled from a per-launch queue head with atomicAdd, so the
-// grid is persistent (sized to the resident capacity of the SMs).
+// Kernel templates instantiated once per quartet class and variant by the
+// generated translation units (gen_eri.py).  One warp owns one work item and
+// evaluates one quartet per lane and step: a row item holds 32 ket pairs, one
+// per lane, against the bra pairs of one second shell in turn (plain builds), a
+// pair item one bra pair against a run of ket pairs (density-screened and
+// multi-density builds, the ERI tensor).  Work items are pulled from a
+// per-launch queue head with atomicAdd, so the grid is persistent (sized to the
+// resident capacity of the SMs).
 #pragma once
 
 #include "vlx_device.cuh"
@@ -218,7 +221,11 @@ __device__ __forceinline__ void digest(const double* f, const double s, const in
 // lane: F_QR, F_QS and F_RS are summed in `acc` over the item and added to F
 // once (flush_row), and the elements D_QR, D_QS, D_RS are read once into `dc`.
 // Per step remain the gathers of D_PR and D_PS, the additions to F_PR and
-// F_PS, and one warp reduction of F_PQ.
+// F_PS, and one warp reduction of F_PQ: for (sp|ss) 2 gathers and 2 reductions
+// per quartet where digesting each quartet by itself takes 8 and 9.  The s, p
+// and d classes of the (H2O)32 / def2-SVP build take 34 ms in all with, 49 ms
+// without these sums; (sp|ss) 7.55 -> 5.7 ms, then bound by FP64 and instruction
+// issue (FP64 pipe 46%, issue 57% of the cycles).
 // Layout of both: [QR: NB NC | QS: NB ND | RS: NC ND], and for a general
 // density (GEN) the transposes of the first two [RQ | SQ] behind; RS then
 // stands for both orientations (D_RS + D_SR, equal additions).
@@ -781,7 +788,7 @@ __device__ __forceinline__ void quartet_body(const FockArgs& a, const int mode)
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= a.nitems) return;
         const WorkItem w = a.items[it];
-        const int bbi = w.blocks & 0xffff, kbi = w.blocks >> 16;
+        const int bbi = w.blocks & 0xffff, kbi = (unsigned)w.blocks >> 16;
         const PairBlockDev bb = a.blocks[bbi];
         const PairBlockDev kb = a.blocks[kbi];
         const MolDev m = a.mols ? a.mols[bb.mol] : a.mol;
@@ -919,9 +926,9 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
             w = a.items[it];
             steps = w.kend - w.bra;
         }
-        const bool diag = (w.blocks & 0xffff) == (w.blocks >> 16);
+        const bool diag = (w.blocks & 0xffff) == ((unsigned)w.blocks >> 16);
         const PairBlockDev& bb = a.blocks[w.blocks & 0xffff];
-        const PairBlockDev& kb = a.blocks[w.blocks >> 16];
+        const PairBlockDev& kb = a.blocks[(unsigned)w.blocks >> 16];
         const MolDev m = a.mols ? a.mols[bb.mol] : a.mol;
         const int kl = w.kbeg + lane, jj = min(kl, kb.npairs - 1);
         int4 head = __ldg(bb.rhead + w.bra);
@@ -946,7 +953,7 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
             const int q = w.bra + x;
             const int4 h = head;  // the next pair's header is read a step ahead
             if (q + 1 < w.kend) head = __ldg(bb.rhead + q + 1);
-            const int bx = h.w >> 16;
+            const int bx = h.w & 15;
             // the kets this launch admits for the bra pair (see item_range)
             int k0 = diag ? h.x : 0, k1 = 0;
             if (a.ith >= bx) k1 = __ldg(kb.bin_off + min(a.ith - bx, 15) + 1);
@@ -971,12 +978,12 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
             if (diag && kl == h.x) s *= 0.5;
             if constexpr (Store::stream) {
                 StreamSink<NA, NB, NC, ND, R> sink(o, m, a.cj, a.ck, s);
-                eri_compute<C>(make_row_view(bb, q, h.w & 0xffff, R()), ket, sboys, a.omega2, sink);
+                eri_compute<C>(make_row_view(bb, q, h.w >> 4, R()), ket, sboys, a.omega2, sink);
                 sink.finish(lane);
             } else {
                 R g[C::NSPH];
                 ArraySink<NA * NB, NC, ND, R> sink{g};
-                eri_compute<C>(make_row_view(bb, q, h.w & 0xffff, R()), ket, sboys, a.omega2, sink);
+                eri_compute<C>(make_row_view(bb, q, h.w >> 4, R()), ket, sboys, a.omega2, sink);
                 double f[C::NSPH];
 #pragma unroll
                 for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];

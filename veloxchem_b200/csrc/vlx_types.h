@@ -50,7 +50,7 @@ struct PairBlockDev {
     // the pairs once more in row order (rows of equal second shell B, ascending
     // pair index, so ascending bin, within a row), as the bra side of the row
     // items reads them
-    const int4* rhead;    // [npairs]           {pair index, AO index of component 0 of A, of B, nuse | bin << 16}
+    const int4* rhead;    // [npairs]           {pair index, AO index of component 0 of A, of B, bin | nuse << 4}
     const double* rab;    // [npairs][4]        B - A, 0
     const double* rprim;  // [npairs][kprim][10] the 9 primitive fields of the pair, 0
     const float* rabf;    // both rounded to FP32
