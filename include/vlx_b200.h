@@ -80,8 +80,10 @@ int vlx_b200_screener_npairs(const vlx_b200_screener* screener, int* npairs);
 int vlx_b200_screener_pair_info(const vlx_b200_screener* screener, int* info, double* maxv);
 
 /* Block-size knob of the reference (CFockDriver::set_block_size_factor,
- * src/t4c_func/FockDriver.cpp:356-360): here the number of ket pairs of one
- * GPU work item is 256 / factor, at least 32. */
+ * src/t4c_func/FockDriver.cpp:356-360): here the length of a GPU work item, in
+ * ket pairs, is 256 / factor, at least 32 (an item of a plain build, which
+ * holds 32 ket pairs against several bra pairs, has an eighth of it as bra
+ * pairs). */
 int vlx_b200_set_block_size_factor(vlx_b200_screener* screener, int factor);
 
 /* Work lists of later builds are made for max(ithreshold, ithreshold_base)
@@ -151,8 +153,9 @@ int vlx_b200_fock_build_local_device(vlx_b200_screener* screener, int rank, int 
 
 /* Partition of the work items over ranks for the rank/nodes builds of this
  * screener: 0 (default) deals them round-robin, as the reference's
- * omp::partition_tasks (src/general/OpenMPFunc.hpp:89-112) does, so a rank's
- * share equals the reference's; 1 assigns each item to the rank with the
+ * omp::partition_tasks (src/general/OpenMPFunc.hpp:89-112) deals its tasks (the
+ * items are not the reference's tasks, so the shares differ, their sum does
+ * not); 1 assigns each item to the rank with the
  * least estimated work so far (greedy list scheduling over the items'
  * algorithmic flops), which balances ranks whose round-robin shares differ.
  * The sum over ranks is the full build in both modes. */
@@ -337,7 +340,7 @@ int vlx_b200_mlp_linear_bf16(const float* X, const void* W_bf16, const float* b,
                              int silu, void* stream);
 
 /* Backward of vlx_b200_mlp_linear: from dY[M, N] (and Z when silu != 0, with
- * dZ[M, N] as scratch) writes dW[N, K], db[N] and, when dX != NULL, dX[M, K]. */
+ * dZ[M, N] as scratch, which may stay unwritten) writes dW[N, K], db[N] and, when dX != NULL, dX[M, K]. */
 int vlx_b200_mlp_linear_backward(const float* X, const float* W, const float* Z, const float* dY, float* dZ,
                                  float* dX, float* dW, float* db, int M, int K, int N, int silu, void* stream);
 
