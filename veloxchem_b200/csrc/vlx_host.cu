@@ -75,6 +75,16 @@ int fail(int code, const std::string& msg)
         if (e_ != cudaSuccess) return fail(VLX_B200_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// Host memory to the device, complete on return for every stream: cudaMemcpy from
+// pageable memory returns once the data is staged, its last part may still be on
+// the way, and the streams used here (non-blocking) do not wait for the legacy
+// stream it runs on.
+cudaError_t copy_to_device(void* dst, const void* src, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 // ------------------------------------------------------------------ basis
 // CBasisFunction::normalize / _rescale / _overlap (BasisFunction.cpp:129-260)
 double lnorm(int l)
@@ -190,9 +200,9 @@ int device_globals(int device, DeviceGlobals** out)
         const std::vector<double> tab(t64.begin(), t64.end());
         const std::vector<float> tabf(t32.begin(), t32.end());
         VLX_CUDA(cudaMalloc(&g.boys, tab.size() * sizeof(double)));
-        VLX_CUDA(cudaMemcpy(g.boys, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(g.boys, tab.data(), tab.size() * sizeof(double)));
         VLX_CUDA(cudaMalloc(&g.boys_f, tabf.size() * sizeof(float)));
-        VLX_CUDA(cudaMemcpy(g.boys_f, tabf.data(), tabf.size() * sizeof(float), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(g.boys_f, tabf.data(), tabf.size() * sizeof(float)));
         // warp-cooperative programs (gen_coop.py): magic, count, 16-int headers,
         // 16-byte op records, LIN weights (float64), then the aux int32 stream
         const char* blob = vlx_coop_blob_start;
@@ -221,9 +231,9 @@ int device_globals(int device, DeviceGlobals** out)
         const size_t off_w = (bytes_o + 255) & ~size_t(255), off_a = off_w + ((bytes_w + 255) & ~size_t(255));
         char* dev = nullptr;
         VLX_CUDA(cudaMalloc(&dev, off_a + bytes_a + 64));
-        VLX_CUDA(cudaMemcpy(dev, ops, bytes_o, cudaMemcpyHostToDevice));
-        if (bytes_w) VLX_CUDA(cudaMemcpy(dev + off_w, wts, bytes_w, cudaMemcpyHostToDevice));
-        VLX_CUDA(cudaMemcpy(dev + off_a, aux, bytes_a, cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(dev, ops, bytes_o));
+        if (bytes_w) VLX_CUDA(copy_to_device(dev + off_w, wts, bytes_w));
+        VLX_CUDA(copy_to_device(dev + off_a, aux, bytes_a));
         g.prog = dev;
         const int* daux = reinterpret_cast<const int*>(dev + off_a);
         for (int c = 0; c < ncls; c++) {
@@ -681,8 +691,8 @@ struct RawPairs {
             d.la = pb.la;
             d.lb = pb.lb;
         }
-        VLX_CUDA(cudaMemcpy(dev, host.get(), arena.size, cudaMemcpyHostToDevice));
-        VLX_CUDA(cudaMemcpy(d_blocks, h.data(), nb * sizeof(PairBlockDev), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(dev, host.get(), arena.size));
+        VLX_CUDA(copy_to_device(d_blocks, h.data(), nb * sizeof(PairBlockDev)));
         return VLX_B200_OK;
     }
 };
@@ -806,9 +816,9 @@ int upload_pairs(vlx_b200_screener* s, const RawPairs& raw)
         std::memcpy(host.get() + ptrs + b * sizeof(int*), &sp, sizeof(int*));
         std::memcpy(host.get() + ptrs + (nb + b) * sizeof(int*), &pp, sizeof(int*));
     }
-    VLX_CUDA(cudaMemcpy(dev + idx_at, host.get(), idx.size, cudaMemcpyHostToDevice));
+    VLX_CUDA(copy_to_device(dev + idx_at, host.get(), idx.size));
     VLX_CUDA(cudaMalloc(&s->d_blocks, std::max<size_t>(1, nb) * sizeof(PairBlockDev)));
-    VLX_CUDA(cudaMemcpy(s->d_blocks, s->h_blocks.data(), nb * sizeof(PairBlockDev), cudaMemcpyHostToDevice));
+    VLX_CUDA(copy_to_device(s->d_blocks, s->h_blocks.data(), nb * sizeof(PairBlockDev)));
     if (most > 0) {
         const dim3 grid((unsigned)std::min((most + 127) / 128, 1024), (unsigned)nb);
         const int* const* lists = reinterpret_cast<const int* const*>(dev + idx_at + ptrs);
@@ -1078,7 +1088,7 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
 
         }
         VLX_CUDA(cudaMalloc(&ts.d_items, total * sizeof(WorkItem)));
-        VLX_CUDA(cudaMemcpy(ts.d_items, all.data(), total * sizeof(WorkItem), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(ts.d_items, all.data(), total * sizeof(WorkItem)));
     }
     if (2 * (int)ts.classes.size() > s->ncounters) {
         if (s->d_counters) cudaFree(s->d_counters);
@@ -1330,7 +1340,7 @@ int prepare_dscr(vlx_b200_screener* s, const double* dD, cudaStream_t st)
         std::vector<int2> info(nsh);
         for (int i = 0; i < nsh; i++) info[i] = make_int2(s->shells[i].ao0, s->shells[i].l);
         VLX_CUDA(cudaMalloc(&s->d_shinfo, nsh * sizeof(int2)));
-        VLX_CUDA(cudaMemcpy(s->d_shinfo, info.data(), nsh * sizeof(int2), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(s->d_shinfo, info.data(), nsh * sizeof(int2)));
     }
     const long long n = (long long)nsh * nsh;
     const int4 nl = make_int4(s->nl[0], s->nl[1], s->nl[2], s->nl[3]);
@@ -1616,7 +1626,7 @@ int vlx_b200_screener_create(vlx_b200_screener** out, int device, int natoms, co
             for (int m = 0; m < 2 * sh.l + 1; m++) s->perm[sh.ao0 + m * s->nl[sh.l]] = sh.ao0_ref + m * s->nl[sh.l];
         for (int i = 0; i < s->nao; i++) s->permuted = s->permuted || s->perm[i] != i;
         if (cudaMalloc(&s->d_perm, std::max<size_t>(s->perm.size(), 1) * sizeof(int)) != cudaSuccess ||
-            cudaMemcpy(s->d_perm, s->perm.data(), s->perm.size() * sizeof(int), cudaMemcpyHostToDevice) !=
+            copy_to_device(s->d_perm, s->perm.data(), s->perm.size() * sizeof(int)) !=
                 cudaSuccess)
             return cleanup(fail(VLX_B200_ERR_CUDA, "screener_create: AO permutation upload failed"));
     }
@@ -2082,7 +2092,7 @@ static int one_electron_impl(int device, int which, int natoms, const int* Z, co
     auto up = [&](const void* src, size_t bytes, void** dst) -> int {
         VLX_CUDA(cudaMalloc(dst, std::max<size_t>(bytes, 8)));
         bufs.push_back(*dst);
-        if (bytes) VLX_CUDA(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+        if (bytes) VLX_CUDA(copy_to_device(*dst, src, bytes));
         return VLX_B200_OK;
     };
     auto free_all = [&]() {
@@ -2356,7 +2366,7 @@ int vlx_b200_boys_device(int device, int m, int n, const double* T, double* F)
     double *dT = nullptr, *dF = nullptr;
     VLX_CUDA(cudaMalloc(&dT, n * sizeof(double)));
     VLX_CUDA(cudaMalloc(&dF, n * sizeof(double)));
-    cudaMemcpy(dT, T, n * sizeof(double), cudaMemcpyHostToDevice);
+    copy_to_device(dT, T, n * sizeof(double));
     launch_boys_test<BOYS_MMAX>(m, dT, dF, n, g->boys);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(F, dF, n * sizeof(double), cudaMemcpyDeviceToHost);
@@ -2537,7 +2547,7 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
 
         }
         VLX_CUDA(cudaMalloc(&m.d_items, total * sizeof(WorkItem)));
-        VLX_CUDA(cudaMemcpy(m.d_items, all.data(), total * sizeof(WorkItem), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(m.d_items, all.data(), total * sizeof(WorkItem)));
     }
     if (2 * (int)m.classes.size() > b->ncounters) {
         // the instantiated graph of an earlier threshold launches with the old
@@ -2649,19 +2659,18 @@ int vlx_b200_batch_create(vlx_b200_batch** out, vlx_b200_screener* const* screen
         VLX_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
         VLX_CUDA(cudaMalloc(&b->d_blocks, std::max<size_t>(1, blocks.size()) * sizeof(PairBlockDev)));
         if (!blocks.empty())
-            VLX_CUDA(cudaMemcpy(b->d_blocks, blocks.data(), blocks.size() * sizeof(PairBlockDev),
-                                cudaMemcpyHostToDevice));
+            VLX_CUDA(copy_to_device(b->d_blocks, blocks.data(), blocks.size() * sizeof(PairBlockDev)));
         VLX_CUDA(cudaMalloc(&b->d_mols, n * sizeof(vlx::MolDev)));
         VLX_CUDA(cudaMalloc(&b->d_off, (n + 1) * sizeof(long long)));
-        VLX_CUDA(cudaMemcpy(b->d_off, b->off.data(), (n + 1) * sizeof(long long), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(b->d_off, b->off.data(), (n + 1) * sizeof(long long)));
         VLX_CUDA(cudaMalloc(&b->d_nao, n * sizeof(int)));
-        VLX_CUDA(cudaMemcpy(b->d_nao, nao.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(b->d_nao, nao.data(), n * sizeof(int)));
         VLX_CUDA(cudaMalloc(&b->d_acc, (size_t)std::max<long long>(b->off.back(), 1) * sizeof(double)));
         VLX_CUDA(cudaMalloc(&b->d_aooff, (n + 1) * sizeof(int)));
-        VLX_CUDA(cudaMemcpy(b->d_aooff, aooff.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(b->d_aooff, aooff.data(), (n + 1) * sizeof(int)));
         if (b->permuted) {
             VLX_CUDA(cudaMalloc(&b->d_perm, std::max<size_t>(perm.size(), 1) * sizeof(int)));
-            VLX_CUDA(cudaMemcpy(b->d_perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice));
+            VLX_CUDA(copy_to_device(b->d_perm, perm.data(), perm.size() * sizeof(int)));
             VLX_CUDA(cudaMalloc(&b->d_dint, (size_t)std::max<long long>(b->off.back(), 1) * sizeof(double)));
         }
         return VLX_B200_OK;
@@ -2732,7 +2741,7 @@ int vlx_b200_batch_fock_build(vlx_b200_batch* b, const double* d_densities, int 
             h[k].nao = s->nao;
             for (int l = 0; l <= VLX_LMAX; l++) h[k].nl[l] = s->nl[l];
         }
-        VLX_CUDA(cudaMemcpy(b->d_mols, h.data(), h.size() * sizeof(vlx::MolDev), cudaMemcpyHostToDevice));
+        VLX_CUDA(copy_to_device(b->d_mols, h.data(), h.size() * sizeof(vlx::MolDev)));
         b->mols_D = d_densities;
     }
     long long launches = 0;
