@@ -274,6 +274,15 @@ int vlx_b200_one_electron_device(int device, int which, int natoms, const int* Z
  * (host arrays T[n] in, F[n] out), for validation. */
 int vlx_b200_boys_device(int device, int m, int n, const double* T, double* F);
 
+/* F_0(T) .. F_m(T) (m <= 12) for n arguments as a quartet class of order m
+ * evaluates them, in FP64 or (fp32 != 0, T rounded to float) in FP32 (host
+ * arrays T[n] in, F[n][m + 1] out), for validation. */
+int vlx_b200_boys_orders_device(int device, int m, int fp32, int n, const double* T, double* F);
+
+/* 1 / sqrt(x) for n positive normal x as the FP64 recursions evaluate it (host
+ * arrays), for validation. */
+int vlx_b200_rsqrt_device(int device, int n, const double* x, double* y);
+
 /* Per-class record of a profiled build. */
 typedef struct {
     int la, lb, lc, ld;        /* quartet class (bra la <= lb | ket lc <= ld) */

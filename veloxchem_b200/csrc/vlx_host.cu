@@ -412,6 +412,39 @@ void launch_boys_test(int m, const double* T, double* F, int n, const double* ta
         launch_boys_test<M - 1>(m, T, F, n, tab);
 }
 
+// The Boys functions of orders 0..M as a class of order M evaluates them, and
+// 1 / sqrt(x), for validation.
+template <int M>
+__global__ void boys_orders_test_kernel(const double* T, double* F, int n, const double* tab, const float* tab_f)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (tab_f) {
+        float f[M + 1];
+        vlx::boys_scaled_f<M>((float)T[i], 1.0f, f, tab_f + (size_t)M * BOYS_STRIDE_F);
+        for (int m = 0; m <= M; m++) F[(size_t)i * (M + 1) + m] = f[m];
+    } else {
+        double f[M + 1];
+        vlx::boys_scaled<M>(T[i], 1.0, f, tab + (size_t)M * BOYS_STRIDE);
+        for (int m = 0; m <= M; m++) F[(size_t)i * (M + 1) + m] = f[m];
+    }
+}
+
+template <int M>
+void launch_boys_orders_test(int m, const double* T, double* F, int n, const double* tab, const float* tab_f)
+{
+    if (m == M)
+        boys_orders_test_kernel<M><<<(n + 127) / 128, 128>>>(T, F, n, tab, tab_f);
+    else if constexpr (M > 0)
+        launch_boys_orders_test<M - 1>(m, T, F, n, tab, tab_f);
+}
+
+__global__ void rsqrt_test_kernel(const double* x, double* y, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = vlx::rsqrt_pos(x[i]);
+}
+
 // FP64 throughput probe: 8 independent FMA chains per thread.
 __global__ void fp64_probe_kernel(double* out, int iters, double a, double b)
 {
@@ -2356,6 +2389,30 @@ int vlx_b200_fp64_peak(int device, double* tflops)
     return VLX_B200_OK;
 }
 
+}  // extern "C"
+
+// n values to the device, through `run(in, out)`, and `nout` values back.
+template <class Run>
+static int on_device(int device, int n, const double* in, size_t nout, double* out, Run run)
+{
+    DeviceGlobals* g = nullptr;
+    const int rc = device_globals(device, &g);
+    if (rc) return rc;
+    VLX_CUDA(cudaSetDevice(device));
+    double* buf = nullptr;
+    VLX_CUDA(cudaMalloc(&buf, (n + nout) * sizeof(double)));
+    cudaError_t e = copy_to_device(buf, in, n * sizeof(double));
+    if (e == cudaSuccess) {
+        run(g, buf, buf + n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, buf + n, nout * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(buf);
+    return e == cudaSuccess ? VLX_B200_OK : fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
+}
+
+extern "C" {
+
 int vlx_b200_boys_device(int device, int m, int n, const double* T, double* F)
 {
     if (m < 0 || m > BOYS_MMAX || n < 1 || !T || !F) return fail(VLX_B200_ERR_ARGUMENT, "boys_device: bad args");
@@ -2374,6 +2431,23 @@ int vlx_b200_boys_device(int device, int m, int n, const double* T, double* F)
     cudaFree(dF);
     if (e != cudaSuccess) return fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
     return VLX_B200_OK;
+}
+
+int vlx_b200_boys_orders_device(int device, int m, int fp32, int n, const double* T, double* F)
+{
+    if (m < 0 || m > 4 * VLX_LMAX || n < 1 || !T || !F)
+        return fail(VLX_B200_ERR_ARGUMENT, "boys_orders_device: bad args");
+    return on_device(device, n, T, (size_t)n * (m + 1), F, [=](const DeviceGlobals* g, const double* x, double* y) {
+        launch_boys_orders_test<4 * VLX_LMAX>(m, x, y, n, g->boys, fp32 ? g->boys_f : nullptr);
+    });
+}
+
+int vlx_b200_rsqrt_device(int device, int n, const double* x, double* y)
+{
+    if (n < 1 || !x || !y) return fail(VLX_B200_ERR_ARGUMENT, "rsqrt_device: bad args");
+    return on_device(device, n, x, n, y, [=](const DeviceGlobals*, const double* in, double* out) {
+        rsqrt_test_kernel<<<(n + 127) / 128, 128>>>(in, out, n);
+    });
 }
 
 }  // extern "C"
