@@ -183,7 +183,8 @@ int vlx_b200_set_partition(vlx_b200_screener* screener, int mode);
  * enqueued.  Limits and behaviour:
  *  - nao above VLX_B200_NOALLOC_MAX_NAO is rejected with VLX_B200_ERR_ARGUMENT;
  *  - the screener must already hold the work list of `ithreshold`: one
- *    ordinary build (vlx_b200_fock_build*) with that threshold creates it;
+ *    ordinary build (vlx_b200_fock_build*) with that threshold creates it, and
+ *    loads the kernels for every density, label and precision with it;
  *    otherwise VLX_B200_ERR_ARGUMENT;
  *  - the screener's mixed-precision split (vlx_b200_set_fp32_threshold)
  *    applies as in vlx_b200_fock_build_device;

@@ -6,9 +6,13 @@ keeps the previous call's contents), reject bases above its static limit, and
 refuse to run before the screener has a work list for the threshold."""
 
 import ctypes
+import subprocess
+import sys
 
 import numpy as np
 import pytest
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +98,69 @@ def test_noalloc_honours_mixed_precision():
     scr.set_fp32_threshold(0.0, 0.0)
     assert float((fmix - f64).abs().max()) > 1e-10      # the FP32 quartets changed the matrix
     assert float((fna - fmix).abs().max()) < 1e-10      # ... and the same way in both builds
+
+
+WARM_UP = """
+import ctypes, sys, torch
+from veloxchem_b200 import MolecularBasis, T4CScreener
+from veloxchem_b200 import _native as nat
+from veloxchem_b200.geometry import water_cluster
+mol = water_cluster((2, 1, 1), 3, 2)
+scr = T4CScreener()
+scr.partition(MolecularBasis.read(mol, 'def2-tzvp'), mol, 'eri')
+a = torch.randn(scr.nao, scr.nao, dtype=torch.float64, device='cuda', generator=torch.Generator('cuda').manual_seed(1))
+d, f, ref = (a + a.T) / 2, torch.empty_like(a), torch.empty_like(a)
+stream = torch.cuda.Stream()
+
+def build(entry, out, symmetric):
+    nat.check(getattr(nat.lib(), entry)(scr.handle, ctypes.c_void_p(d.data_ptr()), symmetric, b'2jk', 1.0, 0.0, 12,
+                                        ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(stream.cuda_stream)), entry)
+
+stream.wait_stream(torch.cuda.current_stream())
+build('vlx_b200_fock_build_device', f, 1)  # the warm-up: symmetric, FP64
+build('vlx_b200_fock_build_noalloc', f, 1)
+torch.cuda.synchronize()
+"""
+
+BUILDS = {
+    'general': "symmetric = 0",
+    'fp32': "symmetric = 1\nscr.set_fp32_threshold(1e-3, float(d.abs().max()))",
+    'general, fp32': "symmetric = 0\nscr.set_fp32_threshold(1e-3, float(d.abs().max()))",
+}
+
+
+def _fresh(script):
+    """In a process of its own, where no other test has loaded the kernels."""
+    res = subprocess.run([sys.executable, '-c', script], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+    return res.stdout
+
+
+@pytest.mark.parametrize('build', BUILDS)
+def test_one_warm_up_serves_every_density_and_precision(build):
+    """A build with the work list of a symmetric FP64 one takes no device memory,
+    although it runs other kernels: their code and thread-local memory came with
+    the list."""
+    out = _fresh(WARM_UP + BUILDS[build] + """
+torch.cuda.synchronize()
+before = torch.cuda.mem_get_info()[0]
+build('vlx_b200_fock_build_noalloc', f, symmetric)
+torch.cuda.synchronize()
+print('taken', before - torch.cuda.mem_get_info()[0])
+""")
+    assert out.split()[-1] == '0', out
+
+
+@pytest.mark.parametrize('build', BUILDS)
+def test_one_warm_up_serves_every_captured_build(build):
+    _fresh(WARM_UP + BUILDS[build] + """
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, stream=stream):
+    build('vlx_b200_fock_build_device', f, symmetric)
+f.zero_()
+graph.replay()
+torch.cuda.synchronize()
+build('vlx_b200_fock_build_device', ref, symmetric)
+torch.cuda.synchronize()
+assert float((f - ref).abs().max()) < 1e-11
+""")

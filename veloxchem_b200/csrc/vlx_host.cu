@@ -176,6 +176,11 @@ struct DeviceGlobals {
     // resident blocks per SM of the compiled classes' kernel variants
     // (0: not asked yet; every thread finds the same value)
     std::atomic<int> occupancy[vlx::kNumVariants][2][vlx::kNumQuartetClasses] = {};
+    // classes whose kernels are loaded: compiled ones with row items and with
+    // pair items, warp-cooperative ones
+    static constexpr int kMaxCoop = 64;
+    std::atomic<bool> loaded[2][vlx::kNumQuartetClasses] = {}, loaded_coop[kMaxCoop] = {};
+    int* idle_head = nullptr;  // work-queue head of the launches without items (load_class)
 
     int resident_blocks(int cls, int variant, bool f32)
     {
@@ -184,6 +189,37 @@ struct DeviceGlobals {
         return o.load();
     }
 };
+
+// Loads every kernel that a class's items can reach (symmetric and general
+// densities, FP64 and FP32): a launch without items each, which brings the code
+// and the thread-local memory onto the device.  With the work list, so that no
+// later build on it allocates, whatever its density, label or precision
+// (vlx_b200_fock_build_noalloc, stream capture).
+int load_class(DeviceGlobals& g, int compiled, int coop, bool rows, cudaStream_t st)
+{
+    std::atomic<bool>& loaded = compiled >= 0 ? g.loaded[rows ? 0 : 1][compiled] : g.loaded_coop[coop];
+    if (loaded.load()) return VLX_B200_OK;
+    FockArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.boys = g.boys;
+    a.boys_f = g.boys_f;
+    a.counter = g.idle_head;
+    for (int f = 0; f < 2; f++) {
+        if (compiled < 0) {
+            VLX_CUDA(vlx::launch_coop_quartet(f ? vlx::MODE_F32 : 0, a, g.coop[coop], 1, st));
+            continue;
+        }
+        for (int sym = 0; sym < 2; sym++) {
+            const int variant = rows ? (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN) : (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN);
+            g.resident_blocks(compiled, variant, f != 0);
+            const int mode = sym ? vlx::MODE_FOCK_SYM : vlx::MODE_FOCK_GEN;
+            vlx::kQuartetClasses[compiled].launch[variant](f ? (mode | vlx::MODE_F32) : mode, a, 1, st);
+            VLX_CUDA(cudaGetLastError());
+        }
+    }
+    loaded.store(true);
+    return VLX_B200_OK;
+}
 
 std::mutex g_dev_mutex;
 std::map<int, DeviceGlobals> g_dev;
@@ -211,6 +247,7 @@ int device_globals(int device, DeviceGlobals** out)
         std::memcpy(head, blob, sizeof(head));
         if (head[0] != 0x434F4F51) return fail(VLX_B200_ERR_CUDA, "corrupt cooperative program blob");
         const int ncls = head[1];
+        if (ncls < 0 || ncls > DeviceGlobals::kMaxCoop) return fail(VLX_B200_ERR_CUDA, "corrupt cooperative program blob");
         constexpr int HW = 16;
         std::vector<int> ch((size_t)ncls * HW);
         std::memcpy(ch.data(), blob + 8, ch.size() * sizeof(int));
@@ -264,6 +301,9 @@ int device_globals(int device, DeviceGlobals** out)
             g.coop_post_flops.push_back(h[13]);
         }
         VLX_CUDA(vlx::coop_prepare());
+        VLX_CUDA(cudaMalloc(&g.idle_head, sizeof(int)));
+        const int zero = 0;
+        VLX_CUDA(copy_to_device(g.idle_head, &zero, sizeof(int)));
         g.ready = true;
     }
     *out = &g;
@@ -1037,6 +1077,8 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
                 if (ct.compiled < 0) ct.coop = find_coop(s->glob, Pb.la, Pb.lb, Pk.la, Pk.lb);
                 if (ct.compiled < 0 && ct.coop < 0)
                     return fail(VLX_B200_ERR_UNSUPPORTED, "quartet class not compiled in");
+                const int rc = load_class(*s->glob, ct.compiled, ct.coop, !ext, s->stream);
+                if (rc) return rc;
                 it = cls_index.emplace(key, (int)ts.classes.size()).first;
                 ts.classes.push_back(ct);
             }
