@@ -164,3 +164,32 @@ build('vlx_b200_fock_build_device', ref, symmetric)
 torch.cuda.synchronize()
 assert float((f - ref).abs().max()) < 1e-11
 """)
+
+
+def test_extended_builds_keep_the_plain_work_lists():
+    """Multi-density and batched builds have lists of their own: eight thresholds of
+    them leave the lists of eight plain builds in place."""
+    import torch
+    from veloxchem_b200 import _native as nat
+    from veloxchem_b200.batch import FockBatch
+    mol, bas, scr, dens = _system((2, 2, 2), 2, 3)
+    d = torch.from_numpy(dens).cuda()
+    f, plain = torch.zeros_like(d), torch.zeros_like(d)
+    batch = FockBatch([scr, scr])
+    pair = torch.cat([d.flatten(), d.flatten()])
+    both = torch.zeros_like(pair)
+    out = np.zeros_like(dens)
+    one = ctypes.POINTER(ctypes.c_double) * 1
+    for ith in range(5, 13):
+        nat.check(nat.lib().vlx_b200_fock_build_device(scr.handle, ctypes.c_void_p(d.data_ptr()), 1, b'2jk', 1.0, 0.0, ith,
+                                                       ctypes.c_void_p(plain.data_ptr()), None), 'fock_build_device')
+    for ith in range(5, 13):
+        nat.check(nat.lib().vlx_b200_fock_build_multi(scr.handle, 0, 1, 1, one(nat.dptr(dens)), 1,
+                                                      (ctypes.c_char_p * 1)(b'2jk'), 1.0, 0.0, ith, one(nat.dptr(out)),
+                                                      None), 'fock_build_multi')
+        batch.build_device(pair, both, ithreshold=ith)
+    torch.cuda.synchronize()
+    for ith in (5, 12):
+        nat.check(_noalloc(scr, d, f, ith=ith), 'fock_build_noalloc')
+    torch.cuda.synchronize()
+    assert float((f - plain).abs().max()) < TOL

@@ -1170,10 +1170,14 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
         s->ncounters = std::max<int>(128, 2 * (int)ts.classes.size());
         VLX_CUDA(cudaMalloc(&s->d_counters, s->ncounters * sizeof(int)));
     }
-    // keep the cache small: the SCF changes ithreshold only a few times
-    if (s->tasksets.size() >= 8) {
-        if (s->tasksets.front().d_items) cudaFree(s->tasksets.front().d_items);
-        s->tasksets.erase(s->tasksets.begin());
+    // keep the cache small: the SCF changes ithreshold only a few times.  Eight
+    // lists of each kind, so that extended or batched builds leave the lists of
+    // the plain ones in place (vlx_b200_fock_build_noalloc, captured builds)
+    const auto same_kind = [&](const TaskSet& x) { return x.ext == ts.ext && (x.share > 1) == (ts.share > 1); };
+    if (std::count_if(s->tasksets.begin(), s->tasksets.end(), same_kind) >= 8) {
+        const auto oldest = std::find_if(s->tasksets.begin(), s->tasksets.end(), same_kind);
+        if (oldest->d_items) cudaFree(oldest->d_items);
+        s->tasksets.erase(oldest);
     }
     s->tasksets.push_back(std::move(ts));
     *out = &s->tasksets.back();
