@@ -165,6 +165,28 @@ std::vector<long double> make_boys_table(int stride)
 }
 
 // ------------------------------------------------------------------ per-device globals
+// Streams beside a build's own for its class launches (enqueue_ctx), with the
+// events that tie them to it.  A few sets per device, made with the device's
+// other globals and kept: a set costs 1.4 ms, which every new geometry would pay
+// again in its first build if a screener owned one.  A build has a set while
+// it enqueues; the work of the next one on the same set queues up behind.
+struct SideStreams {
+    static constexpr int kCount = 24;
+    cudaStream_t s[kCount] = {};
+    cudaEvent_t fork = nullptr, join[kCount] = {};
+    std::mutex mutex;
+
+    int open()
+    {
+        if (!fork) VLX_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        for (int i = 0; i < kCount; i++) {
+            if (!s[i]) VLX_CUDA(cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking));
+            if (!join[i]) VLX_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
+        }
+        return VLX_B200_OK;
+    }
+};
+
 struct DeviceGlobals {
     bool ready = false;
     int nsm = 0;
@@ -180,6 +202,11 @@ struct DeviceGlobals {
     // pair items, warp-cooperative ones
     static constexpr int kMaxCoop = 64;
     std::atomic<bool> loaded[2][vlx::kNumQuartetClasses] = {}, loaded_coop[kMaxCoop] = {};
+    // side streams: an owner of builds (screener, batch) has a set of its own as
+    // long as there are few, so that the builds of several run beside each other
+    static constexpr int kSideSets = 4;
+    SideStreams side[kSideSets];
+    std::atomic<unsigned> side_owners = 0;
     int* idle_head = nullptr;  // work-queue head of the launches without items (load_class)
 
     int resident_blocks(int cls, int variant, bool f32)
@@ -187,6 +214,47 @@ struct DeviceGlobals {
         std::atomic<int>& o = occupancy[variant][f32 ? 1 : 0][cls];
         if (o.load() == 0) o.store(std::max(1, vlx::kQuartetClasses[cls].occupancy[variant](f32)));
         return o.load();
+    }
+};
+
+// A set of side streams for one build on `st`, the owner's own one where it is
+// free.  The streams of a set that was forked into a stream capture belong to it
+// until the capture ends, so a set is of use only to builds of the same capture
+// (or of none, when it is in none).
+struct SideLease {
+    SideStreams* set = nullptr;  // null: every set is part of another capture
+    std::unique_lock<std::mutex> lock;
+
+    SideLease() = default;
+    SideLease(DeviceGlobals& g, int own, cudaStream_t st)
+    {
+        const unsigned long long capture = capture_of(st);
+        for (const bool wait : {false, true})
+            for (int i = 0; i < DeviceGlobals::kSideSets && !set; i++) {
+                SideStreams& side = g.side[(own + i) % DeviceGlobals::kSideSets];
+                std::unique_lock<std::mutex> l(side.mutex, std::defer_lock);
+                if (wait)
+                    l.lock();
+                else if (!l.try_lock())
+                    continue;
+                const unsigned long long in = capture_of(side.s[0]);
+                if (in != 0 && in != capture) continue;
+                set = &side;
+                lock = std::move(l);
+            }
+    }
+
+    // id of the capture a stream is part of (0: none)
+    static unsigned long long capture_of(cudaStream_t st)
+    {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+            cudaGetLastError();  // the legacy stream beside another capture: not captured itself
+            return 0;
+        }
+        if (status == cudaStreamCaptureStatusNone) return 0;
+        return status == cudaStreamCaptureStatusActive ? id : ~0ULL;
     }
 };
 
@@ -301,6 +369,10 @@ int device_globals(int device, DeviceGlobals** out)
             g.coop_post_flops.push_back(h[13]);
         }
         VLX_CUDA(vlx::coop_prepare());
+        for (SideStreams& side : g.side) {
+            const int rc = side.open();
+            if (rc) return rc;
+        }
         VLX_CUDA(cudaMalloc(&g.idle_head, sizeof(int)));
         const int zero = 0;
         VLX_CUDA(copy_to_device(g.idle_head, &zero, sizeof(int)));
@@ -569,40 +641,6 @@ struct TaskSet {
     long long quartets = 0, prim_quartets = 0;
 };
 
-// Streams beside a build's own for its class launches (enqueue_ctx), made on
-// first use and owned by a screener or a batch.
-struct SideStreams {
-    static constexpr int kCount = 24;
-    cudaStream_t s[kCount] = {};
-    cudaEvent_t fork = nullptr, join[kCount] = {};
-    bool ready = false;
-
-    int open()
-    {
-        if (ready) return VLX_B200_OK;
-        if (!fork) VLX_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-        for (int i = 0; i < kCount; i++) {
-            if (!s[i]) VLX_CUDA(cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking));
-            if (!join[i]) VLX_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
-        }
-        ready = true;
-        return VLX_B200_OK;
-    }
-
-    void close()
-    {
-        for (int i = 0; i < kCount; i++) {
-            if (s[i]) cudaStreamDestroy(s[i]);
-            if (join[i]) cudaEventDestroy(join[i]);
-            s[i] = nullptr;
-            join[i] = nullptr;
-        }
-        if (fork) cudaEventDestroy(fork);
-        fork = nullptr;
-        ready = false;
-    }
-};
-
 int pair_key(int la, int lb) { return (la + lb) * 16 + lb; }
 
 // ket pairs per work item of a warp-cooperative class
@@ -664,7 +702,7 @@ struct vlx_b200_screener {
     float* d_F32 = nullptr;
     std::vector<TaskSet> tasksets;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    SideStreams side;
+    int side_set = 0;  // its set of DeviceGlobals::side
 };
 
 namespace {
@@ -1216,8 +1254,7 @@ int ensure_buffers(vlx_b200_screener* s)
     if (!s->d_D) VLX_CUDA(cudaMalloc(&s->d_D, std::max<size_t>(bytes, 8)));
     if (!s->d_F) VLX_CUDA(cudaMalloc(&s->d_F, std::max<size_t>(bytes, 8)));
     if (s->permuted && !s->d_Dint) VLX_CUDA(cudaMalloc(&s->d_Dint, std::max<size_t>(bytes, 8)));
-    // with the buffers, so that a later build under stream capture creates nothing
-    return s->side.open();
+    return VLX_B200_OK;
 }
 
 // The density the class kernels read: the caller's dD (caller's AO order)
@@ -1284,7 +1321,8 @@ struct LaunchCtx {
     float* F32 = nullptr;
     const std::map<int, int>* bps = nullptr;  // per-class caps of resident blocks per SM (compiled classes)
     int bps_try = 0;                          // a cap for every compiled class (autotuning; 0: off)
-    SideStreams* side = nullptr;              // the launches run beside each other (null: in turn on the build's stream)
+    int side_set = -1;                        // the launches run beside each other, on this or another set of side
+                                              // streams (-1: in turn on the build's stream)
 };
 
 // Enqueues all class kernels of a task set on `st`; the accumulators must be
@@ -1364,45 +1402,46 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
             list.push_back({c, f, std::max(1, std::min(want, most)), -1});
         }
     }
-    int nside = 0;
-    if (L.side && !events && list.size() > 1) {
+    int nside = 0, rc = VLX_B200_OK;
+    const auto check = [&rc](cudaError_t e) {
+        if (e != cudaSuccess && !rc) rc = fail(VLX_B200_ERR_CUDA, std::string("class launches: ") + cudaGetErrorString(e));
+    };
+    SideLease lease;
+    if (L.side_set >= 0 && !events && list.size() > 1) {
         std::stable_sort(list.begin(), list.end(), [&](const Launch& x, const Launch& y) {
             return ts->classes[x.c].step_cost > ts->classes[y.c].step_cost;
         });
-        const int rc = L.side->open();
-        if (rc) return rc;
+        lease = SideLease(*L.glob, L.side_set, st);
+    }
+    if (lease.set) {
         nside = std::min<int>((int)list.size(), SideStreams::kCount);
-        VLX_CUDA(cudaEventRecord(L.side->fork, st));
-        for (int i = 0; i < nside; i++) VLX_CUDA(cudaStreamWaitEvent(L.side->s[i], L.side->fork, 0));
+        check(cudaEventRecord(lease.set->fork, st));
+        for (int i = 0; i < nside; i++) check(cudaStreamWaitEvent(lease.set->s[i], lease.set->fork, 0));
         for (size_t i = 0; i < list.size(); i++) list[i].side = (int)(i % nside);
     }
-    int rc = VLX_B200_OK;
     for (const Launch& l : list) {
+        if (rc) break;
         const ClassTasks& ct = ts->classes[l.c];
-        cudaStream_t ls = l.side >= 0 ? L.side->s[l.side] : st;
+        cudaStream_t ls = l.side >= 0 ? lease.set->s[l.side] : st;
         FockArgs af = a;
         af.items = ts->d_items + ct.offset;
         af.nitems = (int)ct.items.size();
         af.counter = L.counters + (l.f ? ts->classes.size() : 0) + l.c;
         af.qstat = L.qstat ? L.qstat + (l.c * 2 + l.f) * 2 : nullptr;
         const int fmode = l.f ? (mode | vlx::MODE_F32) : mode;
-        if (events && l.f == 0) VLX_CUDA(cudaEventRecord((*events)[l.c].first, st));
-        if (ct.compiled >= 0) {
+        if (events && l.f == 0) check(cudaEventRecord((*events)[l.c].first, st));
+        if (ct.compiled >= 0)
             vlx::kQuartetClasses[ct.compiled].launch[variant(ct)](fmode, af, l.grid, ls);
-        } else {
-            const cudaError_t e = vlx::launch_coop_quartet(fmode, af, L.glob->coop[ct.coop], l.grid, ls);
-            if (e != cudaSuccess && !rc) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
-        }
+        else
+            check(vlx::launch_coop_quartet(fmode, af, L.glob->coop[ct.coop], l.grid, ls));
         if (launches) (*launches)++;
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess && !rc) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
-        if (events && l.f == nprec - 1) VLX_CUDA(cudaEventRecord((*events)[l.c].second, st));
-        if (rc) break;
+        check(cudaGetLastError());
+        if (events && l.f == nprec - 1) check(cudaEventRecord((*events)[l.c].second, st));
     }
     // `st` waits for the side streams also after a failed launch
     for (int i = 0; i < nside; i++) {
-        VLX_CUDA(cudaEventRecord(L.side->join[i], L.side->s[i]));
-        VLX_CUDA(cudaStreamWaitEvent(st, L.side->join[i], 0));
+        check(cudaEventRecord(lease.set->join[i], lease.set->s[i]));
+        check(cudaStreamWaitEvent(st, lease.set->join[i], 0));
     }
     return rc;
 }
@@ -1450,7 +1489,7 @@ int enqueue_classes(vlx_b200_screener* s, TaskSet* ts, int mode, const double* d
     L.qstat = qstat;
     L.bps = &s->class_bps;
     L.bps_try = s->bps_try;
-    L.side = &s->side;
+    L.side_set = s->side_set;
     if (mode != vlx::MODE_ERI && dscr_active(s)) {
         const int rc = prepare_dscr(s, dD, st);
         if (rc) return rc;
@@ -1659,6 +1698,7 @@ int vlx_b200_screener_create(vlx_b200_screener** out, int device, int natoms, co
     };
     rc = device_globals(device, &s->glob);
     if (rc) return cleanup(rc);
+    s->side_set = (int)(s->glob->side_owners++ % DeviceGlobals::kSideSets);
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) ||
         cudaEventCreate(&s->ev0) || cudaEventCreate(&s->ev1))
         return cleanup(fail(VLX_B200_ERR_CUDA, "screener_create: stream / event creation failed"));
@@ -1809,7 +1849,6 @@ int vlx_b200_screener_destroy(vlx_b200_screener* s)
     if (s->d_Dint) cudaFree(s->d_Dint);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
-    s->side.close();
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return VLX_B200_OK;
@@ -1931,7 +1970,7 @@ int vlx_b200_fock_build_multi(vlx_b200_screener* s, int rank, int nodes, int nde
         L.mol.nao = s->nao;
         for (int l = 0; l <= VLX_LMAX; l++) L.mol.nl[l] = s->nl[l];
         L.dens.n = nd;
-        L.side = &s->side;
+        L.side_set = s->side_set;
         bool chunk_any = false;
         for (int d = 0; d < nd; d++) {
             if (s->permuted) {
@@ -2602,7 +2641,7 @@ struct vlx_b200_batch {
     int run_ith = 0;  // threshold of the build being enqueued
     const double* mols_D = nullptr;  // D of the uploaded per-molecule records
     long long launches = 0;          // kernel launches of one build
-    SideStreams side;
+    int side_set = 0;                // its set of DeviceGlobals::side
 };
 
 namespace {
@@ -2704,7 +2743,7 @@ int batch_enqueue(vlx_b200_batch* b, TaskSet* ts, bool known, int symmetric, dou
         L.glob = b->glob;
         L.counters = b->d_counters;
         L.mols = b->d_mols;
-        L.side = &b->side;
+        L.side_set = b->side_set;
         const int rc = enqueue_ctx(L, ts, symmetric ? vlx::MODE_FOCK_SYM : vlx::MODE_FOCK_GEN, nullptr, cj, ck,
                                    omega2, b->run_ith, -1, st, launches);
         if (rc) return rc;
@@ -2755,6 +2794,7 @@ int vlx_b200_batch_create(vlx_b200_batch** out, vlx_b200_screener* const* screen
     std::unique_ptr<vlx_b200_batch> b(new vlx_b200_batch());
     b->device = screeners[0]->device;
     b->glob = screeners[0]->glob;
+    b->side_set = (int)(b->glob->side_owners++ % DeviceGlobals::kSideSets);
     b->mols.assign(screeners, screeners + n);
     b->off.assign(n + 1, 0);
     std::vector<PairBlockDev> blocks;
@@ -2820,7 +2860,6 @@ int vlx_b200_batch_destroy(vlx_b200_batch* b)
     if (b->d_perm) cudaFree(b->d_perm);
     if (b->d_dint) cudaFree(b->d_dint);
     if (b->d_counters) cudaFree(b->d_counters);
-    b->side.close();
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return VLX_B200_OK;
