@@ -207,7 +207,7 @@ struct DeviceGlobals {
     static constexpr int kSideSets = 4;
     SideStreams side[kSideSets];
     std::atomic<unsigned> side_owners = 0;
-    int* idle_head = nullptr;  // work-queue head of the launches without items (load_class)
+    int* idle_head = nullptr;  // work-queue head of the launches without items (load_kernels)
 
     int resident_blocks(int cls, int variant, bool f32)
     {
@@ -258,37 +258,6 @@ struct SideLease {
     }
 };
 
-// Loads every kernel that a class's items can reach (symmetric and general
-// densities, FP64 and FP32): a launch without items each, which brings the code
-// and the thread-local memory onto the device.  With the work list, so that no
-// later build on it allocates, whatever its density, label or precision
-// (vlx_b200_fock_build_noalloc, stream capture).
-int load_class(DeviceGlobals& g, int compiled, int coop, bool rows, cudaStream_t st)
-{
-    std::atomic<bool>& loaded = compiled >= 0 ? g.loaded[rows ? 0 : 1][compiled] : g.loaded_coop[coop];
-    if (loaded.load()) return VLX_B200_OK;
-    FockArgs a;
-    std::memset(&a, 0, sizeof(a));
-    a.boys = g.boys;
-    a.boys_f = g.boys_f;
-    a.counter = g.idle_head;
-    for (int f = 0; f < 2; f++) {
-        if (compiled < 0) {
-            VLX_CUDA(vlx::launch_coop_quartet(f ? vlx::MODE_F32 : 0, a, g.coop[coop], 1, st));
-            continue;
-        }
-        for (int sym = 0; sym < 2; sym++) {
-            const int variant = rows ? (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN) : (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN);
-            g.resident_blocks(compiled, variant, f != 0);
-            const int mode = sym ? vlx::MODE_FOCK_SYM : vlx::MODE_FOCK_GEN;
-            vlx::kQuartetClasses[compiled].launch[variant](f ? (mode | vlx::MODE_F32) : mode, a, 1, st);
-            VLX_CUDA(cudaGetLastError());
-        }
-    }
-    loaded.store(true);
-    return VLX_B200_OK;
-}
-
 std::mutex g_dev_mutex;
 std::map<int, DeviceGlobals> g_dev;
 
@@ -334,11 +303,15 @@ int device_globals(int device, DeviceGlobals** out)
         if ((size_t)(aux + naux * 4 - blob) > bsize) return fail(VLX_B200_ERR_CUDA, "truncated program blob");
         const size_t bytes_o = nops * 16, bytes_w = nwts * 8, bytes_a = naux * 4;
         const size_t off_w = (bytes_o + 255) & ~size_t(255), off_a = off_w + ((bytes_w + 255) & ~size_t(255));
+        const size_t off_h = off_a + ((bytes_a + 15) & ~size_t(15));
         char* dev = nullptr;
-        VLX_CUDA(cudaMalloc(&dev, off_a + bytes_a + 64));
+        VLX_CUDA(cudaMalloc(&dev, off_h + sizeof(int)));
         VLX_CUDA(copy_to_device(dev, ops, bytes_o));
         if (bytes_w) VLX_CUDA(copy_to_device(dev + off_w, wts, bytes_w));
         VLX_CUDA(copy_to_device(dev + off_a, aux, bytes_a));
+        const int no_item = 0;
+        VLX_CUDA(copy_to_device(dev + off_h, &no_item, sizeof(int)));
+        g.idle_head = reinterpret_cast<int*>(dev + off_h);
         g.prog = dev;
         const int* daux = reinterpret_cast<const int*>(dev + off_a);
         for (int c = 0; c < ncls; c++) {
@@ -373,9 +346,6 @@ int device_globals(int device, DeviceGlobals** out)
             const int rc = side.open();
             if (rc) return rc;
         }
-        VLX_CUDA(cudaMalloc(&g.idle_head, sizeof(int)));
-        const int zero = 0;
-        VLX_CUDA(copy_to_device(g.idle_head, &zero, sizeof(int)));
         g.ready = true;
     }
     *out = &g;
@@ -1074,6 +1044,40 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
     const int part = (nodes > 1) ? s->part : 0;
     for (auto& t : s->tasksets)
         if (t.ith == ith && t.rank == rank && t.nodes == nodes && t.seg == s->seg && t.tune_gen == s->tune_gen &&
+// Loads every kernel that the items of a work list can reach (symmetric and
+// general densities, FP64 and FP32): a launch without items each, which brings the
+// code and the thread-local memory onto the device.  With the list, so that no
+// later build on it allocates, whatever its density, label or precision
+// (vlx_b200_fock_build_noalloc, stream capture).  Variant by variant: the code
+// that runs side by side lies together.
+int load_kernels(DeviceGlobals& g, const std::vector<ClassTasks>& classes, bool ext, cudaStream_t st)
+{
+    const auto loaded = [&](const ClassTasks& ct) -> std::atomic<bool>& {
+        return ct.compiled >= 0 ? g.loaded[ext ? 1 : 0][ct.compiled] : g.loaded_coop[ct.coop];
+    };
+    FockArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.boys = g.boys;
+    a.boys_f = g.boys_f;
+    a.counter = g.idle_head;
+    for (const bool f32 : {false, true})
+        for (const bool sym : {true, false})
+            for (const ClassTasks& ct : classes) {
+                if (loaded(ct).load()) continue;
+                const int mode = (sym ? vlx::MODE_FOCK_SYM : vlx::MODE_FOCK_GEN) | (f32 ? vlx::MODE_F32 : 0);
+                if (ct.compiled >= 0) {
+                    const int variant = ext ? (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN) : (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN);
+                    g.resident_blocks(ct.compiled, variant, f32);
+                    vlx::kQuartetClasses[ct.compiled].launch[variant](mode, a, 1, st);
+                } else {
+                    VLX_CUDA(vlx::launch_coop_quartet(mode, a, g.coop[ct.coop], 1, st));
+                }
+                VLX_CUDA(cudaGetLastError());
+            }
+    for (const ClassTasks& ct : classes) loaded(ct).store(true);
+    return VLX_B200_OK;
+}
+
             t.part == part && t.ext == ext && t.share == share) {
             *out = &t;
             return VLX_B200_OK;
@@ -1115,8 +1119,6 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
                 if (ct.compiled < 0) ct.coop = find_coop(s->glob, Pb.la, Pb.lb, Pk.la, Pk.lb);
                 if (ct.compiled < 0 && ct.coop < 0)
                     return fail(VLX_B200_ERR_UNSUPPORTED, "quartet class not compiled in");
-                const int rc = load_class(*s->glob, ct.compiled, ct.coop, !ext, s->stream);
-                if (rc) return rc;
                 it = cls_index.emplace(key, (int)ts.classes.size()).first;
                 ts.classes.push_back(ct);
             }
@@ -1124,6 +1126,8 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
             ct.rows = ct.compiled >= 0 && !ext;
             ct.jobs.push_back({(int)bra, (int)ket});
         }
+    const int rc = load_kernels(*s->glob, ts.classes, ext, s->stream);
+    if (rc) return rc;
     for (ClassTasks& ct : ts.classes) {
         for (const auto& j : ct.jobs)
             ct.step_cost = std::max(ct.step_cost, class_flops(s, ct, 1, (long long)s->blocks[j.first].nuse_max *
