@@ -305,7 +305,7 @@ int device_globals(int device, DeviceGlobals** out)
         const size_t off_w = (bytes_o + 255) & ~size_t(255), off_a = off_w + ((bytes_w + 255) & ~size_t(255));
         const size_t off_h = off_a + ((bytes_a + 15) & ~size_t(15));
         char* dev = nullptr;
-        VLX_CUDA(cudaMalloc(&dev, off_h + sizeof(int)));
+        VLX_CUDA(cudaMalloc(&dev, off_h + 64));
         VLX_CUDA(copy_to_device(dev, ops, bytes_o));
         if (bytes_w) VLX_CUDA(copy_to_device(dev + off_w, wts, bytes_w));
         VLX_CUDA(copy_to_device(dev + off_a, aux, bytes_a));
@@ -1036,14 +1036,6 @@ void row_items(const PairBlock& Pb, const PairBlock& Pk, int blocks, bool diag, 
     }
 }
 
-// ext: the list of the extended kernels (TaskSet::ext).  share: molecules that
-// share the launches (batched builds), whose items fill the SMs together.
-int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext, TaskSet** out, int share = 1)
-{
-    const int ith = std::max(ith_req, s->ith_base);
-    const int part = (nodes > 1) ? s->part : 0;
-    for (auto& t : s->tasksets)
-        if (t.ith == ith && t.rank == rank && t.nodes == nodes && t.seg == s->seg && t.tune_gen == s->tune_gen &&
 // Loads every kernel that the items of a work list can reach (symmetric and
 // general densities, FP64 and FP32): a launch without items each, which brings the
 // code and the thread-local memory onto the device.  With the list, so that no
@@ -1078,6 +1070,14 @@ int load_kernels(DeviceGlobals& g, const std::vector<ClassTasks>& classes, bool 
     return VLX_B200_OK;
 }
 
+// ext: the list of the extended kernels (TaskSet::ext).  share: molecules that
+// share the launches (batched builds), whose items fill the SMs together.
+int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext, TaskSet** out, int share = 1)
+{
+    const int ith = std::max(ith_req, s->ith_base);
+    const int part = (nodes > 1) ? s->part : 0;
+    for (auto& t : s->tasksets)
+        if (t.ith == ith && t.rank == rank && t.nodes == nodes && t.seg == s->seg && t.tune_gen == s->tune_gen &&
             t.part == part && t.ext == ext && t.share == share) {
             *out = &t;
             return VLX_B200_OK;
