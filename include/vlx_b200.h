@@ -271,6 +271,20 @@ int vlx_b200_one_electron_device(int device, int which, int natoms, const int* Z
                                  const int* ket_l, const int* ket_nprim, const double* ket_exps,
                                  const double* ket_coefs, double* d_out, void* stream);
 
+/* Work items of one quartet class in a work list. */
+typedef struct {
+    int la, lb, lc, ld;  /* quartet class */
+    int rows;            /* 1: row items (plain builds), 0: pair items */
+    long long items;
+    int longest;         /* bra pairs of the longest row item, ket pairs of the longest pair item */
+} vlx_b200_work_class;
+
+/* The work list that the screener's plain (extended = 0) or density-screened
+ * and multi-density (extended != 0) builds at `ithreshold` left behind, up to
+ * max_classes records; VLX_B200_ERR_ARGUMENT without one.  For validation. */
+int vlx_b200_work_list(const vlx_b200_screener* screener, int ithreshold, int extended, int max_classes,
+                       vlx_b200_work_class* out, int* nclasses);
+
 /* Boys function F_m(T) for n arguments as the device evaluates it
  * (host arrays T[n] in, F[n] out), for validation. */
 int vlx_b200_boys_device(int device, int m, int n, const double* T, double* F);

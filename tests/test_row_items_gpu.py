@@ -23,7 +23,7 @@ H 3.8 0.2 -0.1"""
 def _screener(which, basis):
     from veloxchem_b200 import MolecularBasis, Molecule, T4CScreener
     from veloxchem_b200.geometry import water_cluster
-    mol = Molecule.read_str(METHANE_AND_HF) if which == 'mixed' else water_cluster((3, 2, 2), 11, which)
+    mol = Molecule.read_str(METHANE_AND_HF) if which == 'mixed' else water_cluster((3, 2, 2) if which <= 12 else (4, 3, 2), 11, which)
     scr = T4CScreener()
     scr.partition(MolecularBasis.read(mol, basis), mol, 'eri')
     return scr
@@ -69,20 +69,49 @@ def test_row_items_equal_pair_items(which, basis, symmetric):
         assert _close(_rows(scr, d, symmetric, '2jk', ith), _pairs(scr, d, symmetric, '2jk', ith)), ith
 
 
+def _longest_rows(scr, ith):
+    """Longest row of each compiled class of the cached plain list."""
+    from veloxchem_b200 import _native as nat
+    return {c: w.longest for c, w in nat.work_list(scr, ith).items() if w.rows}
+
+
 @pytest.mark.parametrize('symmetric', [1, 0])
 def test_row_lengths_filters_and_shares(symmetric):
-    scr = _screener(7, 'def2-svp')
+    """Rows of up to 32, 8 and 4 bra pairs: a cluster large enough that the work of
+    its s and p classes fills every SM at these lengths."""
+    scr = _screener(24, 'def2-svp')
     d = _density(scr.nao, symmetric, 4)
     ref = {ith: _pairs(scr, d, symmetric, '2jk', ith) for ith in (6, 9, 12)}
-    for factor in (1, 4, 128):  # rows of up to 32, 8 and 4 bra pairs
+    for factor, length in ((1, 32), (4, 8), (128, 4)):
         scr.set_block_size_factor(factor)
         assert _close(_rows(scr, d, symmetric, '2jk', 12), ref[12])
+        longest = _longest_rows(scr, 12)
+        assert max(longest.values()) == length
+        assert all(longest[c] == length for c in ((0, 0, 0, 0), (0, 1, 0, 0), (0, 1, 0, 1), (1, 1, 0, 1))), longest
+    scr.set_block_size_factor(1)
+    scr.set_fp32_threshold(1e-6, float(np.max(np.abs(d))))  # rows of 32 cut at the FP32 boundary
+    assert np.max(np.abs(_rows(scr, d, symmetric, '2jk', 12) - ref[12])) < 1e-8 + 1e-12 * np.max(np.abs(ref[12]))
+    scr.set_fp32_threshold(0.0, 0.0)
     scr.set_work_threshold(14)  # one list, filtered at run time
     for ith, want in ref.items():
         assert _close(_rows(scr, d, symmetric, '2jk', ith), want)
     for partition in ('round_robin', 'balanced'):
         scr.set_partition(partition)
         assert _close(sum(_rows(scr, d, symmetric, '2jk', 12, rank=r, nodes=3) for r in range(3)), ref[12])
+
+
+@pytest.mark.parametrize('symmetric', [1, 0])
+def test_long_rows_of_large_classes(symmetric):
+    """Rows of several bra pairs of the d and f classes whose blocks walk them in
+    step, whole and cut at the FP32 boundary (tolerance as below)."""
+    scr = _screener(24, 'def2-tzvp')
+    d = _density(scr.nao, symmetric, 6)
+    want = _pairs(scr, d, symmetric, '2jk', 12)
+    assert _close(_rows(scr, d, symmetric, '2jk', 12), want)
+    longest = _longest_rows(scr, 12)
+    assert longest[0, 3, 1, 2] >= 8 and longest[1, 3, 0, 2] >= 8 and longest[1, 2, 1, 2] >= 4, longest
+    scr.set_fp32_threshold(1e-6, float(np.max(np.abs(d))))
+    assert np.max(np.abs(_rows(scr, d, symmetric, '2jk', 12) - want)) < 1e-8 + 1e-12 * np.max(np.abs(want))
 
 
 @pytest.mark.parametrize('which,basis', [(7, 'def2-svp'), (2, 'def2-tzvp')])
@@ -93,8 +122,10 @@ def test_fp32_split_of_rows(which, basis):
     scr = _screener(which, basis)
     d = _density(scr.nao, 1, 2)
     want = _pairs(scr, d, 1, '2jk', 12)
+    fp64 = _rows(scr, d, 1, '2jk', 12)
     for cutoff in (1e-9, 1e-6, 1e-3):
         scr.set_fp32_threshold(cutoff, float(np.max(np.abs(d))))
         got = _rows(scr, d, 1, '2jk', 12)
         assert np.max(np.abs(got - want)) < 1e-2 * cutoff + 1e-12 * np.max(np.abs(want))
-    assert np.any(got != want)
+    # far above what another order of the additions changes
+    assert np.max(np.abs(got - fp64)) > 1e3 * max(np.max(np.abs(fp64 - want)), 1e-13)

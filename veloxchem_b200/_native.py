@@ -47,6 +47,7 @@ SIGNATURES = {
     'vlx_b200_boys_device': (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp]),
     'vlx_b200_boys_orders_device': (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp]),
     'vlx_b200_rsqrt_device': (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _dp, _dp]),
+    'vlx_b200_work_list': (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _ip]),
     'vlx_b200_fock_profile': (ctypes.c_int, [_vp, _vp, ctypes.c_int, ctypes.c_char_p, ctypes.c_double, ctypes.c_int,
                                              _vp, _vp, ctypes.c_int, _vp, _ip]),
     'vlx_b200_fp64_peak': (ctypes.c_int, [ctypes.c_int, _dp]),
@@ -87,6 +88,20 @@ class ClassProfile(ctypes.Structure):
 
     def as_dict(self):
         return {k: getattr(self, k) for k, _ in self._fields_}
+
+
+class WorkClass(ctypes.Structure):
+    _fields_ = [('la', ctypes.c_int), ('lb', ctypes.c_int), ('lc', ctypes.c_int), ('ld', ctypes.c_int),
+                ('rows', ctypes.c_int), ('items', ctypes.c_longlong), ('longest', ctypes.c_int)]
+
+
+def work_list(screener, ithreshold=12, extended=False, max_classes=256):
+    """{class: WorkClass} of the work list that the screener's builds left behind."""
+    arr = (WorkClass * max_classes)()
+    n = ctypes.c_int(0)
+    check(lib().vlx_b200_work_list(screener.handle, int(ithreshold), int(extended), max_classes,
+                                   ctypes.cast(arr, ctypes.c_void_p), ctypes.byref(n)), 'work_list')
+    return {(w.la, w.lb, w.lc, w.ld): w for w in arr[:n.value]}
 
 
 class TuneResult(ctypes.Structure):

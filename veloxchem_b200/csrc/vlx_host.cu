@@ -1902,6 +1902,27 @@ int vlx_b200_set_work_threshold(vlx_b200_screener* s, int ithreshold_base)
     return VLX_B200_OK;
 }
 
+int vlx_b200_work_list(const vlx_b200_screener* s, int ith, int extended, int max_classes, vlx_b200_work_class* out,
+                       int* nclasses)
+{
+    if (!s || !out || !nclasses || max_classes < 1) return fail(VLX_B200_ERR_ARGUMENT, "null argument");
+    const TaskSet* found = nullptr;
+    for (const TaskSet& t : s->tasksets)
+        if (t.ith == std::max(ith, s->ith_base) && t.nodes == 1 && t.share == 1 && t.seg == s->seg &&
+            t.tune_gen == s->tune_gen && t.ext == (extended != 0))
+            found = &t;
+    if (!found) return fail(VLX_B200_ERR_ARGUMENT, "work_list: no such list on this screener");
+    int n = 0;
+    for (const ClassTasks& ct : found->classes) {
+        if (n == max_classes) break;
+        vlx_b200_work_class& w = out[n++];
+        w = {ct.la, ct.lb, ct.lc, ct.ld, ct.rows ? 1 : 0, (long long)ct.items.size(), 0};
+        for (const WorkItem& x : ct.items) w.longest = std::max(w.longest, x.kend - (ct.rows ? x.bra : x.kbeg));
+    }
+    *nclasses = n;
+    return VLX_B200_OK;
+}
+
 int vlx_b200_set_block_size_factor(vlx_b200_screener* s, int factor)
 {
     if (!s || factor < 1) return fail(VLX_B200_ERR_ARGUMENT, "invalid block size factor");
