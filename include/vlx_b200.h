@@ -385,10 +385,14 @@ int vlx_b200_to_bf16(const float* x, void* y_bf16, long long n, void* stream);
  * src/t4c_func/FockDriver.cpp:356-404).  Times every quartet class of a
  * 2J-K build of d_density at `ithreshold` under several ket-run lengths per
  * work item, then, with the chosen lengths, the compiled classes under caps
- * of 1, 2 and 4 resident blocks per SM, and keeps the fastest choice per
- * class for the screener's later builds (all thresholds); synchronises
- * `stream`.  Results are numerically the same
- * builds (only the order of the FP64 atomic additions changes). */
+ * of 1, 2 and 4 resident blocks per SM.  The classes are timed one after
+ * another and builds run them beside each other, so the fastest choices are
+ * kept for the screener's later builds (all thresholds) only if whole builds
+ * are faster with them than with the default values; otherwise the defaults
+ * stay and are reported.  Plain builds and density-screened ones have different
+ * work items and are tuned apart, by the screener's settings at this call;
+ * synchronises `stream`.  Results are numerically the same builds (only the
+ * order of the FP64 atomic additions changes). */
 typedef struct {
     int la, lb, lc, ld;
     int table_driven;   /* 1: warp-cooperative kernel */

@@ -2,6 +2,7 @@
 reference's golden matrices.  Tolerances: J, K and 2J-K to 1e-10 absolute
 (max element), ERI tensors to 1e-12, Schwarz values to 1e-12 relative."""
 
+import ctypes
 import json
 import pickle
 
@@ -412,6 +413,29 @@ def test_autotune_keeps_the_result():
     after = _fock(s, g['density'], '2jk', 1.0, 12)
     assert np.max(np.abs(after - before)) < 1e-12
     assert np.max(np.abs(after - g['f2jk'])) < TOL
+
+
+def test_autotune_keeps_to_its_kind_of_list():
+    """Lengths timed on the row items of plain builds leave the pair items of
+    multi-density and density-screened builds alone."""
+    import torch
+    from veloxchem_b200 import _native as nat
+    g, mol, bas = load_golden('h2o4_svp.npz')
+    s = _screener(mol, bas)
+    d = torch.from_numpy(g['density']).cuda()
+    f = torch.empty_like(d)
+
+    def extended_items():
+        s.set_density_screening(0.0, 1e-13)
+        nat.check(nat.lib().vlx_b200_fock_build_device(s.handle, ctypes.c_void_p(d.data_ptr()), 1, b'2jk', 1.0, 0.0, 12,
+                                                       ctypes.c_void_p(f.data_ptr()), None), 'fock_build_device')
+        torch.cuda.synchronize()
+        s.set_density_screening(0.0, 0.0)
+        return {c: (w.items, w.longest) for c, w in nat.work_list(s, 12, True).items()}
+
+    before = extended_items()
+    nat.autotune(s, d.data_ptr(), 12)
+    assert extended_items() == before
 
 
 def test_shared_work_list_filters_thresholds_at_run_time():

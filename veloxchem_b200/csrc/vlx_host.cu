@@ -611,6 +611,13 @@ struct TaskSet {
     long long quartets = 0, prim_quartets = 0;
 };
 
+// Key of a class's tuned values.  Row items and pair items are tuned apart: a
+// length in ket pairs that suits one says nothing about the other.
+int tune_key(const ClassTasks& ct, bool ext)
+{
+    return ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12) | (ext ? 1 << 16 : 0);
+}
+
 int pair_key(int la, int lb) { return (la + lb) * 16 + lb; }
 
 // ket pairs per work item of a warp-cooperative class
@@ -647,7 +654,7 @@ struct vlx_b200_screener {
     int* d_counters = nullptr;
     int ncounters = 0;
     int seg = 256;
-    // autotuned ket-run length per quartet class (key la | lb << 4 | lc << 8 | ld << 12)
+    // autotuned ket-run length per quartet class and kind of list (tune_key)
     std::map<int, int> class_seg;
     // autotuned cap of resident blocks per SM of a compiled class's persistent
     // launch (same key; absent: the occupancy limit)
@@ -1147,7 +1154,7 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
         if (s->seg_try_compiled > 0) {
             seg = (ct.coop >= 0) ? s->seg_try_coop : s->seg_try_compiled;
         } else {
-            const auto tuned = s->class_seg.find(ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12));
+            const auto tuned = s->class_seg.find(tune_key(ct, ext));
             if (tuned != s->class_seg.end()) seg = tuned->second;
         }
         const auto take = [&](const WorkItem& w) {
@@ -1401,7 +1408,7 @@ int enqueue_ctx(const LaunchCtx& L, TaskSet* ts, int mode, double* eri, double c
                 if (L.bps_try > 0) {
                     occ = std::min(occ, L.bps_try);
                 } else if (L.bps) {
-                    const auto cap = L.bps->find(ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12));
+                    const auto cap = L.bps->find(tune_key(ct, ts->ext));
                     if (cap != L.bps->end()) occ = std::min(occ, cap->second);
                 }
                 most = occ * nsm;
@@ -2984,7 +2991,10 @@ int vlx_b200_batch_fock_build(vlx_b200_batch* b, const double* d_densities, int 
 // Per quartet class the length of the ket run of one work item (the unit of
 // the persistent work queue: long runs amortise the bra set-up, short runs
 // balance the tail of the launch) is picked by timing every class under each
-// candidate length in profiled builds (one CUDA-event pair per class launch).
+// candidate length in profiled builds (one CUDA-event pair per class launch, the
+// launches in turn).  Builds run their classes beside each other, where other
+// lengths may be better, so the choices are kept only if whole builds are faster
+// with them.
 // No counterpart in the reference (its block-size factor is one global knob).
 
 namespace {
@@ -3013,7 +3023,13 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
     if (rc) return rc;
     const int ith32_saved = s->ith32;
     s->ith32 = -1;
-    s->class_seg.clear();
+    // only the choices of the kind of list that the builds use now
+    const bool ext = dscr_active(s);
+    const auto drop_choices = [&] {
+        for (auto* m : {&s->class_seg, &s->class_bps})
+            for (auto it = m->begin(); it != m->end();) it = ((it->first >> 16) != 0) == ext ? m->erase(it) : std::next(it);
+    };
+    drop_choices();
     const int gen0 = ++s->tune_gen;
     const size_t ncand = sizeof(kTuneCandidates) / sizeof(kTuneCandidates[0]);
     std::map<int, std::vector<float>> times;  // class key -> ms per candidate
@@ -3023,7 +3039,7 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
         s->seg_try_coop = kTuneCandidates[k].coop;
         s->tune_gen = gen0 + 1 + (int)k;
         TaskSet* ts = nullptr;
-        rc = build_tasks(s, ith, 0, 1, dscr_active(s), &ts);
+        rc = build_tasks(s, ith, 0, 1, ext, &ts);
         if (rc) break;
         const size_t nc = ts->classes.size();
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev(nc);
@@ -3042,7 +3058,7 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
             if (ct.items.empty()) continue;
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, ev[c].first, ev[c].second);
-            const int key = ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12);
+            const int key = tune_key(ct, ext);
             auto& v = times[key];
             v.resize(ncand, 1e30f);
             v[k] = ms;
@@ -3082,10 +3098,9 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
     // SM of each compiled class's persistent launch (fewer resident threads
     // keep the thread-local frames of the large classes in L2); a cap is kept
     // when it beats the uncapped launch by more than 2%
-    s->class_bps.clear();
     s->tune_gen = gen0 + 1 + (int)ncand;
     TaskSet* tsb = nullptr;
-    rc = build_tasks(s, ith, 0, 1, dscr_active(s), &tsb);
+    rc = build_tasks(s, ith, 0, 1, ext, &tsb);
     for (const int cap : kTuneBlockCaps) {
         if (rc) break;
         s->bps_try = cap;
@@ -3105,7 +3120,7 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
             if (ct.items.empty() || ct.compiled < 0) continue;
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, ev[c].first, ev[c].second);
-            const int key = ct.la | (ct.lb << 4) | (ct.lc << 8) | (ct.ld << 12);
+            const int key = tune_key(ct, ext);
             if (ms < 0.98f * best_ms[key]) {
                 best_ms[key] = ms;
                 s->class_bps[key] = cap;
@@ -3117,6 +3132,35 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
         }
     }
     s->bps_try = 0;
+    // whole builds, by the default values and by the chosen ones in turn
+    const std::map<int, int> seg = s->class_seg, bps = s->class_bps;
+    float whole[2] = {1e30f, 1e30f};
+    const auto use = [&](bool chosen) {
+        s->class_seg = seg;
+        s->class_bps = bps;
+        if (!chosen) drop_choices();
+        s->tune_gen = gen0 + 1 + (int)ncand + (chosen ? 0 : 1);
+    };
+    for (int round = 0; round < 6 && !rc; round++)
+        for (int chosen = 0; chosen < 2 && !rc; chosen++) {
+            use(chosen != 0);
+            TaskSet* ts = nullptr;
+            rc = build_tasks(s, ith, 0, 1, ext, &ts);
+            if (rc) break;
+            cudaError_t e = cudaEventRecord(s->ev0, st);
+            if (e == cudaSuccess) e = cudaMemsetAsync(s->d_acc, 0, (size_t)s->nao * s->nao * sizeof(double), st);
+            if (e == cudaSuccess)
+                rc = enqueue_classes(s, ts, vlx::MODE_FOCK_SYM, dI, s->d_acc, nullptr, 4.0, -1.0, 0.0, ith, -1, st, nullptr);
+            if (e == cudaSuccess) e = cudaEventRecord(s->ev1, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (!rc && e != cudaSuccess) rc = fail(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
+            float ms = 0.0f;
+            cudaEventElapsedTime(&ms, s->ev0, s->ev1);
+            if (round > 0) whole[chosen] = std::min(whole[chosen], ms);
+            if (round == 1 && chosen && ms > 200.0f) round = 6;  // long builds hardly vary
+        }
+    const bool keep = !rc && whole[1] < 0.99f * whole[0];
+    use(keep);
     for (auto it = s->tasksets.begin(); it != s->tasksets.end();) {
         if (it->tune_gen >= gen0) {
             if (it->d_items) cudaFree(it->d_items);
@@ -3126,11 +3170,9 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
         }
     }
     s->ith32 = ith32_saved;
-    if (rc) {
-        s->class_bps.clear();
-        s->tune_gen = gen0 + 2 + (int)ncand;
-        return rc;
-    }
+    // later builds make their work lists with the values kept
+    s->tune_gen = gen0 + 3 + (int)ncand;
+    if (rc) return rc;
     int n = 0;
     for (const auto& kv : times) {
         const auto& v = kv.second;
@@ -3141,15 +3183,14 @@ int vlx_b200_autotune(vlx_b200_screener* s, const double* d_density, int ith, vo
             r.lc = (kv.first >> 8) & 15;
             r.ld = (kv.first >> 12) & 15;
             r.table_driven = kind[kv.first] ? 1 : 0;
-            r.segment = s->class_seg[kv.first];
-            r.best_ms = best_ms[kv.first];
+            const auto chosen = s->class_seg.find(kv.first);
+            r.segment = chosen != s->class_seg.end() ? chosen->second : (kind[kv.first] ? kCoopSegment : s->seg);
+            r.best_ms = keep ? best_ms[kv.first] : v[0];
             r.default_ms = v[0];
             const auto cap = s->class_bps.find(kv.first);
             r.blocks_per_sm = (cap == s->class_bps.end()) ? 0 : cap->second;
         }
     }
-    // later builds make their work lists with the chosen lengths
-    s->tune_gen = gen0 + 2 + (int)ncand;
     *nclasses = n;
     return VLX_B200_OK;
 }
