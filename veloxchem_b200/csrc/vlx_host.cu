@@ -198,16 +198,11 @@ struct DeviceGlobals {
     // resident blocks per SM of the compiled classes' kernel variants
     // (0: not asked yet; every thread finds the same value)
     std::atomic<int> occupancy[vlx::kNumVariants][2][vlx::kNumQuartetClasses] = {};
-    // classes whose kernels are loaded: compiled ones with row items and with
-    // pair items, warp-cooperative ones
-    static constexpr int kMaxCoop = 64;
-    std::atomic<bool> loaded[2][vlx::kNumQuartetClasses] = {}, loaded_coop[kMaxCoop] = {};
     // side streams: an owner of builds (screener, batch) has a set of its own as
     // long as there are few, so that the builds of several run beside each other
     static constexpr int kSideSets = 4;
     SideStreams side[kSideSets];
     std::atomic<unsigned> side_owners = 0;
-    int* idle_head = nullptr;  // work-queue head of the launches without items (load_kernels)
 
     int resident_blocks(int cls, int variant, bool f32)
     {
@@ -284,7 +279,6 @@ int device_globals(int device, DeviceGlobals** out)
         std::memcpy(head, blob, sizeof(head));
         if (head[0] != 0x434F4F51) return fail(VLX_B200_ERR_CUDA, "corrupt cooperative program blob");
         const int ncls = head[1];
-        if (ncls < 0 || ncls > DeviceGlobals::kMaxCoop) return fail(VLX_B200_ERR_CUDA, "corrupt cooperative program blob");
         constexpr int HW = 16;
         std::vector<int> ch((size_t)ncls * HW);
         std::memcpy(ch.data(), blob + 8, ch.size() * sizeof(int));
@@ -303,15 +297,11 @@ int device_globals(int device, DeviceGlobals** out)
         if ((size_t)(aux + naux * 4 - blob) > bsize) return fail(VLX_B200_ERR_CUDA, "truncated program blob");
         const size_t bytes_o = nops * 16, bytes_w = nwts * 8, bytes_a = naux * 4;
         const size_t off_w = (bytes_o + 255) & ~size_t(255), off_a = off_w + ((bytes_w + 255) & ~size_t(255));
-        const size_t off_h = off_a + ((bytes_a + 15) & ~size_t(15));
         char* dev = nullptr;
-        VLX_CUDA(cudaMalloc(&dev, off_h + 64));
+        VLX_CUDA(cudaMalloc(&dev, off_a + bytes_a + 64));
         VLX_CUDA(copy_to_device(dev, ops, bytes_o));
         if (bytes_w) VLX_CUDA(copy_to_device(dev + off_w, wts, bytes_w));
         VLX_CUDA(copy_to_device(dev + off_a, aux, bytes_a));
-        const int no_item = 0;
-        VLX_CUDA(copy_to_device(dev + off_h, &no_item, sizeof(int)));
-        g.idle_head = reinterpret_cast<int*>(dev + off_h);
         g.prog = dev;
         const int* daux = reinterpret_cast<const int*>(dev + off_a);
         for (int c = 0; c < ncls; c++) {
@@ -1052,37 +1042,20 @@ void row_items(const PairBlock& Pb, const PairBlock& Pk, int blocks, bool diag, 
 }
 
 // Loads every kernel that the items of a work list can reach (symmetric and
-// general densities, FP64 and FP32): a launch without items each, which brings the
-// code and the thread-local memory onto the device.  With the list, so that no
-// later build on it allocates, whatever its density, label or precision
-// (vlx_b200_fock_build_noalloc, stream capture).  Variant by variant: the code
-// that runs side by side lies together.
-int load_kernels(DeviceGlobals& g, const std::vector<ClassTasks>& classes, bool ext, cudaStream_t st)
+// general densities, FP64 and FP32) by asking for its occupancy, so that no later
+// build on the list brings code onto the device, whatever its density, label or
+// precision (vlx_b200_fock_build_noalloc, stream capture).  Variant by variant: the
+// code that runs side by side lies together.  Not by launches without items: once a
+// general density's kernel has been launched, its larger thread-local frame
+// slows the symmetric builds by 1%, and most users never run one.
+void load_kernels(DeviceGlobals& g, const std::vector<ClassTasks>& classes, bool ext)
 {
-    const auto loaded = [&](const ClassTasks& ct) -> std::atomic<bool>& {
-        return ct.compiled >= 0 ? g.loaded[ext ? 1 : 0][ct.compiled] : g.loaded_coop[ct.coop];
-    };
-    FockArgs a;
-    std::memset(&a, 0, sizeof(a));
-    a.boys = g.boys;
-    a.boys_f = g.boys_f;
-    a.counter = g.idle_head;
     for (const bool f32 : {false, true})
         for (const bool sym : {true, false})
-            for (const ClassTasks& ct : classes) {
-                if (loaded(ct).load()) continue;
-                const int mode = (sym ? vlx::MODE_FOCK_SYM : vlx::MODE_FOCK_GEN) | (f32 ? vlx::MODE_F32 : 0);
-                if (ct.compiled >= 0) {
-                    const int variant = ext ? (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN) : (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN);
-                    g.resident_blocks(ct.compiled, variant, f32);
-                    vlx::kQuartetClasses[ct.compiled].launch[variant](mode, a, 1, st);
-                } else {
-                    VLX_CUDA(vlx::launch_coop_quartet(mode, a, g.coop[ct.coop], 1, st));
-                }
-                VLX_CUDA(cudaGetLastError());
-            }
-    for (const ClassTasks& ct : classes) loaded(ct).store(true);
-    return VLX_B200_OK;
+            for (const ClassTasks& ct : classes)
+                if (ct.compiled >= 0)
+                    g.resident_blocks(ct.compiled,
+                                      ext ? (sym ? vlx::PAIRS_SYM : vlx::PAIRS_GEN) : (sym ? vlx::ROWS_SYM : vlx::ROWS_GEN), f32);
 }
 
 // ext: the list of the extended kernels (TaskSet::ext).  share: molecules that
@@ -1141,8 +1114,7 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
             ct.rows = ct.compiled >= 0 && !ext;
             ct.jobs.push_back({(int)bra, (int)ket});
         }
-    const int rc = load_kernels(*s->glob, ts.classes, ext, s->stream);
-    if (rc) return rc;
+    load_kernels(*s->glob, ts.classes, ext);
     for (ClassTasks& ct : ts.classes) {
         for (const auto& j : ct.jobs)
             ct.step_cost = std::max(ct.step_cost, class_flops(s, ct, 1, (long long)s->blocks[j.first].nuse_max *
