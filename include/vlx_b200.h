@@ -364,7 +364,9 @@ int vlx_b200_mlp_linear_bf16(const float* X, const void* W_bf16, const float* b,
                              int silu, void* stream);
 
 /* Backward of vlx_b200_mlp_linear: from dY[M, N] (and Z when silu != 0, with
- * dZ[M, N] as scratch, which may stay unwritten) writes dW[N, K], db[N] and, when dX != NULL, dX[M, K]. */
+ * dZ[M, N] as scratch) writes dW[N, K], db[N] and, when dX != NULL, dX[M, K].
+ * With silu != 0 the outputs may lie in dY's or Z's memory, which are read only
+ * for dZ, and dZ may be either of these two when no output is. */
 int vlx_b200_mlp_linear_backward(const float* X, const float* W, const float* Z, const float* dY, float* dZ,
                                  float* dX, float* dW, float* db, int M, int K, int N, int silu, void* stream);
 

@@ -30,3 +30,27 @@ def test_split_gradients(m, dims):
         assert torch.equal(dw, dw2) and torch.equal(db, db2)  # the ranges are added in a fixed order
         for got, want in ((dw, ew), (db, eb)):
             assert np.max(np.abs(got.double().cpu().numpy() - want)) < 2e-5 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize('m,n', [(64, 64), (300, 130), (4096, 128)])
+@pytest.mark.parametrize('where', ['dY', 'Z'])
+def test_input_gradient_in_place(m, n, where):
+    """dX in the memory of dY or Z (square layers): equal to dX in its own."""
+    import ctypes
+    import torch
+    from veloxchem_b200 import _native as nat
+    gen = torch.Generator('cuda').manual_seed(m + n)
+    x, z, dy = (torch.randn(m, n, device='cuda', generator=gen) for _ in range(3))
+    w = torch.randn(n, n, device='cuda', generator=gen)
+
+    def backward(dx, z, dy):
+        dz, dw, db = torch.empty_like(dy), torch.empty_like(w), torch.empty(n, device='cuda')
+        p = [ctypes.c_void_p(t.data_ptr()) for t in (x, w, z, dy, dz, dx, dw, db)]
+        nat.check(nat.lib().vlx_b200_mlp_linear_backward(*p, m, n, n, 1,
+                                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), 'backward')
+        return dx, dw, db
+
+    apart = backward(torch.empty_like(x), z, dy)
+    buf = (dy if where == 'dY' else z).clone()
+    inside = backward(buf, buf if where == 'Z' else z, buf if where == 'dY' else dy)
+    assert all(torch.equal(a, b) for a, b in zip(apart, inside))

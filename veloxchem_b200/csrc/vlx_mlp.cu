@@ -25,18 +25,11 @@ constexpr int kTileK = 16; // reduction slice staged in shared memory
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 
-__device__ __forceinline__ float silu_derivative(float z)
-{
-    const float s = 1.0f / (1.0f + expf(-z));
-    return s * (1.0f + z * (1.0f - s));
-}
-
 // C(m, n) = sum_k A(m, k) B(k, n) (+ bias[n]) in FP32; A(m, k) = A[m lda + k]
 // (AK) or A[k lda + m], B(k, n) = B[n ldb + k] (BK) or B[k ldb + n], so the
 // staging loads run along the contiguous index of either operand.  Z (optional)
-// gets the value, Y SiLU of it (act) or the value itself.  PRE (optional, with
-// A's layout): A is multiplied by SiLU'(PRE) as it is staged, which saves the
-// backward pass a separate pass over dY.  SUM (optional): sum_k A(m, k).
+// gets the value, Y SiLU of it (act) or the value itself.  SUM (optional):
+// sum_k A(m, k).
 //
 // 64 x 64 outputs per block of 256 threads, 4 x 4 per thread, slices of 16 in k
 // with the next slice's loads in flight during the products.  The weight
@@ -45,15 +38,15 @@ __device__ __forceinline__ float silu_derivative(float z)
 // tiles through distributed shared memory in rank order (the same sums on every
 // run).  Latency bound: a training step at 4096 samples (134 - 128 - 128 - 196,
 // 8 products) takes 0.38 ms, of which host calls are most; with one block per
-// tile for the gradients, a separate SiLU' pass and the bias sums by one block
-// per 32 columns it took 1.67 ms.
+// tile for the gradients and the bias sums by one block per 32 columns it took
+// 1.67 ms.
 constexpr int kSplitMax = 8;      // portable cluster size
 constexpr int kSplitRows = 128;   // least samples of a split
 
 template <bool AK, bool BK>
 __global__ void __launch_bounds__(256) gemm_kernel(const float* __restrict__ A, const int lda,
-                                                   const float* __restrict__ PRE, const float* __restrict__ B,
-                                                   const int ldb, const float* __restrict__ bias,
+                                                   const float* __restrict__ B, const int ldb,
+                                                   const float* __restrict__ bias,
                                                    float* __restrict__ Z, float* __restrict__ Y,
                                                    float* __restrict__ SUM, const int M, const int N, const int K,
                                                    const int act)
@@ -84,7 +77,6 @@ __global__ void __launch_bounds__(256) gemm_kernel(const float* __restrict__ A, 
             const size_t ia = AK ? (size_t)m * lda + ka : (size_t)ka * lda + m;
             const size_t ib = BK ? (size_t)n * ldb + kb : (size_t)kb * ldb + n;
             ra[x] = (m < M && ka < kend) ? __ldg(A + ia) : 0.0f;
-            if (PRE && m < M && ka < kend) ra[x] *= silu_derivative(__ldg(PRE + ia));
             rb[x] = (n < N && kb < kend) ? __ldg(B + ib) : 0.0f;
         }
     };
@@ -229,6 +221,20 @@ __global__ void __launch_bounds__(128) gemm_bf16_mma_kernel(const float* __restr
             }
 }
 
+// dZ = dY SiLU'(Z), SiLU'(z) = s (1 + z (1 - s)), s = 1 / (1 + e^-z); dZ may be dY
+// or Z.  A pass of its own: as a factor of the products' staging loads it was
+// evaluated again for every 64 columns of the output, in their critical path (dW
+// and dX of 64 / 4096 / 30000 samples with 128 inputs and outputs 31 / 84 / 521 us
+// against 24 / 55 / 285 with this pass), and the products read what they write when
+// dX is dY's buffer.
+__global__ void silu_backward_kernel(const float* dY, const float* Z, float* dZ, const size_t n)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const float z = Z[i], s = 1.0f / (1.0f + expf(-z));
+        dZ[i] = dY[i] * s * (1.0f + z * (1.0f - s));
+    }
+}
+
 // masked squared error: dY = 2 w (Y - T) / count, loss += sum w (Y - T)^2
 __global__ void mse_kernel(const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ W,
                            float* __restrict__ dY, double* __restrict__ loss, const size_t n, const float inv_count)
@@ -292,8 +298,8 @@ int vlx_b200_mlp_linear(const float* X, const float* W, const float* b, float* Z
         return vlx_b200_set_error_internal(VLX_B200_ERR_ARGUMENT, "mlp_linear: bad arguments");
     if (M == 0) return VLX_B200_OK;
     const dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-    gemm_kernel<true, true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(X, K, nullptr, W, K, b, Z, Y, nullptr,
-                                                                                 M, N, K, silu_act);
+    gemm_kernel<true, true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(X, K, W, K, b, Z, Y, nullptr, M, N, K,
+                                                                                 silu_act);
     MLP_CHECK();
     return VLX_B200_OK;
 }
@@ -317,9 +323,14 @@ int vlx_b200_mlp_linear_backward(const float* X, const float* W, const float* Z,
     if (!X || !W || !dY || !dW || !db || (silu_act && (!Z || !dZ)) || M < 1 || K < 1 || N < 1)
         return vlx_b200_set_error_internal(VLX_B200_ERR_ARGUMENT, "mlp_linear_backward: bad arguments");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const float* pre = silu_act ? Z : nullptr;
-    // dW[N, K] = g^T X and db = column sums of g = dY SiLU'(Z): rows n,
-    // reduction over the samples, split over a cluster
+    const float* g = dY;
+    if (silu_act) {
+        const size_t n = (size_t)M * N;
+        silu_backward_kernel<<<grid_1d(n), 256, 0, st>>>(dY, Z, dZ, n);
+        g = dZ;
+    }
+    // dW[N, K] = g^T X and db = column sums of g: rows n, reduction over the
+    // samples, split over a cluster
     int split = 1;
     while (split < kSplitMax && M >= 2 * split * kSplitRows) split *= 2;
     cudaLaunchConfig_t cfg = {};
@@ -331,14 +342,14 @@ int vlx_b200_mlp_linear_backward(const float* X, const float* W, const float* Z,
     attr[0].val.clusterDim = {1, 1, (unsigned)split};
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<false, false>, dY, N, pre, X, K,
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<false, false>, g, N, X, K,
                                              static_cast<const float*>(nullptr), static_cast<float*>(nullptr), dW, db,
                                              N, K, M, 0);
     if (e != cudaSuccess) return vlx_b200_set_error_internal(VLX_B200_ERR_CUDA, cudaGetErrorString(e));
     // dX[M, K] = g W
     if (dX)
         gemm_kernel<true, false><<<dim3((K + kTile - 1) / kTile, (M + kTile - 1) / kTile), 256, 0, st>>>(
-            dY, N, pre, W, K, nullptr, nullptr, dX, nullptr, M, K, N, 0);
+            g, N, W, K, nullptr, nullptr, dX, nullptr, M, K, N, 0);
     MLP_CHECK();
     return VLX_B200_OK;
 }
