@@ -632,12 +632,12 @@ struct vlx_b200_screener {
     // D is permuted into it and F back out of it at the boundary of a build
     std::vector<int> perm;
     bool permuted = false;
-    const int* d_perm = nullptr;  // in d_pairs
+    int* d_perm = nullptr;
     double* d_Dint = nullptr;  // the build's density in the internal order
     std::vector<PairBlock> blocks;
     std::vector<PairBlockDev> h_blocks;
-    const PairBlockDev* d_blocks = nullptr;  // in d_pairs
-    char* d_pairs = nullptr;                 // the pair data, its block table and the AO permutation
+    PairBlockDev* d_blocks = nullptr;
+    char* d_pairs = nullptr;
     double* d_D = nullptr;
     double* d_F = nullptr;
     double* d_acc = nullptr;
@@ -689,15 +689,13 @@ struct Arena {
 // PairBlockDev), computed on the host once, from which the Schwarz diagonals are
 // evaluated and the screened pairs gathered (upload_pairs).
 struct RawPairs {
-    char* dev = nullptr;  // one allocation: the pair data, the block table, the Schwarz maxima
-    const PairBlockDev* d_blocks = nullptr;
-    double* d_max = nullptr;  // block after block, in reference order
-    size_t npairs = 0;
-    std::unique_ptr<char[]> host;  // what is being copied
+    char* dev = nullptr;
+    PairBlockDev* d_blocks = nullptr;
 
     ~RawPairs()
     {
         if (dev) cudaFree(dev);
+        if (d_blocks) cudaFree(d_blocks);
     }
 
     int upload(vlx_b200_screener* s)
@@ -710,15 +708,11 @@ struct RawPairs {
             const size_t n = pb.pairs.size(), tiles = (n + 31) / 32;
             at[b] = {arena.take(tiles * pb.ka * pb.kb * 288 * sizeof(double)), arena.take(tiles * 96 * sizeof(double)),
                      arena.take(n * sizeof(int))};
-            npairs += n;
         }
-        const size_t table = arena.take(nb * sizeof(PairBlockDev)), copied = arena.size;
-        const size_t maxima = arena.take(npairs * sizeof(double));
-        host.reset(new char[copied]);
-        VLX_CUDA(cudaMalloc(&dev, arena.size));
-        d_blocks = reinterpret_cast<const PairBlockDev*>(dev + table);
-        d_max = reinterpret_cast<double*>(dev + maxima);
-        PairBlockDev* h = reinterpret_cast<PairBlockDev*>(host.get() + table);
+        const std::unique_ptr<char[]> host(new char[arena.size + 256]);
+        VLX_CUDA(cudaMalloc(&dev, arena.size + 256));
+        VLX_CUDA(cudaMalloc(&d_blocks, std::max<size_t>(1, nb) * sizeof(PairBlockDev)));
+        std::vector<PairBlockDev> h(nb);
         const double kconst = std::sqrt(2.0 / std::sqrt(M_PI));
         for (size_t b = 0; b < nb; b++) {
             PairBlock& pb = s->blocks[b];
@@ -775,8 +769,8 @@ struct RawPairs {
             d.la = pb.la;
             d.lb = pb.lb;
         }
-        // on the stream of the kernels that read it
-        VLX_CUDA(cudaMemcpyAsync(dev, host.get(), copied, cudaMemcpyHostToDevice, s->stream));
+        VLX_CUDA(copy_to_device(dev, host.get(), arena.size));
+        VLX_CUDA(copy_to_device(d_blocks, h.data(), nb * sizeof(PairBlockDev)));
         return VLX_B200_OK;
     }
 };
@@ -843,10 +837,9 @@ int upload_pairs(vlx_b200_screener* s, const RawPairs& raw)
                  data.take(10 * k * n * sizeof(double)),      data.take(4 * n * sizeof(float)),
                  data.take(10 * k * n * sizeof(float))};
     }
-    const size_t ptrs = idx.take(2 * nb * sizeof(int*)), table = idx.take(nb * sizeof(PairBlockDev));
-    const size_t order = idx.take(s->perm.size() * sizeof(int));
+    const size_t ptrs = idx.take(2 * nb * sizeof(int*));
     const size_t idx_at = data.take(idx.size);
-    VLX_CUDA(cudaMalloc(&s->d_pairs, data.size));
+    VLX_CUDA(cudaMalloc(&s->d_pairs, data.size + 256));
     char* dev = s->d_pairs;
     const std::unique_ptr<char[]> host(new char[idx.size]);
     s->h_blocks.assign(nb, PairBlockDev{});
@@ -901,19 +894,17 @@ int upload_pairs(vlx_b200_screener* s, const RawPairs& raw)
         std::memcpy(host.get() + ptrs + b * sizeof(int*), &sp, sizeof(int*));
         std::memcpy(host.get() + ptrs + (nb + b) * sizeof(int*), &pp, sizeof(int*));
     }
-    std::memcpy(host.get() + table, s->h_blocks.data(), nb * sizeof(PairBlockDev));
-    std::memcpy(host.get() + order, s->perm.data(), s->perm.size() * sizeof(int));
-    s->d_blocks = reinterpret_cast<const PairBlockDev*>(dev + idx_at + table);
-    s->d_perm = reinterpret_cast<const int*>(dev + idx_at + order);
-    VLX_CUDA(cudaMemcpyAsync(dev + idx_at, host.get(), idx.size, cudaMemcpyHostToDevice, s->stream));
+    VLX_CUDA(copy_to_device(dev + idx_at, host.get(), idx.size));
+    VLX_CUDA(cudaMalloc(&s->d_blocks, std::max<size_t>(1, nb) * sizeof(PairBlockDev)));
+    VLX_CUDA(copy_to_device(s->d_blocks, s->h_blocks.data(), nb * sizeof(PairBlockDev)));
     if (most > 0) {
         const dim3 grid((unsigned)std::min((most + 127) / 128, 1024), (unsigned)nb);
         const int* const* lists = reinterpret_cast<const int* const*>(dev + idx_at + ptrs);
         gather_pairs_kernel<<<grid, 128, 0, s->stream>>>(raw.d_blocks, s->d_blocks, lists, lists + nb);
         VLX_CUDA(cudaGetLastError());
+        // builds run on the callers' streams
+        VLX_CUDA(cudaStreamSynchronize(s->stream));
     }
-    // builds run on the callers' streams
-    VLX_CUDA(cudaStreamSynchronize(s->stream));
     return VLX_B200_OK;
 }
 
@@ -935,13 +926,14 @@ int find_coop(const DeviceGlobals* g, int la, int lb, int lc, int ld)
     return -1;
 }
 
-int run_schwarz(vlx_b200_screener* s, const RawPairs& raw, std::vector<std::vector<double>>& maxv)
+int run_schwarz(vlx_b200_screener* s, const PairBlockDev* d_blocks, std::vector<std::vector<double>>& maxv)
 {
-    const PairBlockDev* d_blocks = raw.d_blocks;
-    double* d_max = raw.d_max;
     const size_t nb = s->blocks.size();
     std::vector<size_t> off(nb + 1, 0);
     for (size_t b = 0; b < nb; b++) off[b + 1] = off[b] + s->blocks[b].pairs.size();
+    double* d_max = nullptr;
+    VLX_CUDA(cudaMalloc(&d_max, std::max<size_t>(1, off[nb]) * sizeof(double)));
+    const std::unique_ptr<double, cudaError_t (*)(void*)> owner(d_max, [](void* p) { return cudaFree(p); });
     for (size_t b = 0; b < nb; b++) {
         const PairBlock& pb = s->blocks[b];
         const int n = (int)pb.pairs.size();
@@ -1735,6 +1727,10 @@ int vlx_b200_screener_create(vlx_b200_screener** out, int device, int natoms, co
         for (const Shell& sh : s->shells)
             for (int m = 0; m < 2 * sh.l + 1; m++) s->perm[sh.ao0 + m * s->nl[sh.l]] = sh.ao0_ref + m * s->nl[sh.l];
         for (int i = 0; i < s->nao; i++) s->permuted = s->permuted || s->perm[i] != i;
+        if (cudaMalloc(&s->d_perm, std::max<size_t>(s->perm.size(), 1) * sizeof(int)) != cudaSuccess ||
+            copy_to_device(s->d_perm, s->perm.data(), s->perm.size() * sizeof(int)) !=
+                cudaSuccess)
+            return cleanup(fail(VLX_B200_ERR_CUDA, "screener_create: AO permutation upload failed"));
     }
     // GTO blocks (l ascending, distinct contraction depths ascending)
     std::vector<std::pair<int, int>> gblocks;  // (l, K)
@@ -1778,7 +1774,7 @@ int vlx_b200_screener_create(vlx_b200_screener** out, int device, int natoms, co
     rc = raw.upload(s);
     if (rc) return cleanup(rc);
     std::vector<std::vector<double>> maxv;
-    rc = run_schwarz(s, raw, maxv);
+    rc = run_schwarz(s, raw.d_blocks, maxv);
     if (rc) return cleanup(rc);
     for (size_t b = 0; b < s->blocks.size(); b++) {
         PairBlock& pb = s->blocks[b];
@@ -1820,6 +1816,7 @@ int vlx_b200_screener_destroy(vlx_b200_screener* s)
     for (auto& t : s->tasksets)
         if (t.d_items) cudaFree(t.d_items);
     if (s->d_pairs) cudaFree(s->d_pairs);
+    if (s->d_blocks) cudaFree(s->d_blocks);
     if (s->d_D) cudaFree(s->d_D);
     if (s->d_F) cudaFree(s->d_F);
     if (s->d_acc) cudaFree(s->d_acc);
@@ -1831,6 +1828,7 @@ int vlx_b200_screener_destroy(vlx_b200_screener* s)
     if (s->d_multi) cudaFree(s->d_multi);
     if (s->d_D32) cudaFree(s->d_D32);
     if (s->d_F32) cudaFree(s->d_F32);
+    if (s->d_perm) cudaFree(s->d_perm);
     if (s->d_Dint) cudaFree(s->d_Dint);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
