@@ -102,6 +102,7 @@ def test_scf_energy_against_oracle_driven_scf(guess, incremental, fp32):
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not ref_available(), reason='reference oracle not built')
 @pytest.mark.parametrize('basis', ['def2-svpd', 'def2-tzvp'])
 def test_one_electron_against_reference(basis):
     from conftest import load_golden
@@ -129,6 +130,7 @@ def test_one_electron_device_output_matches_host_output():
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not ref_available(), reason='reference oracle not built')
 def test_mixed_overlap_against_reference():
     from oracle.oracle import RefOracle
     from veloxchem_b200 import MolecularBasis
