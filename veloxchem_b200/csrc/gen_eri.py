@@ -689,10 +689,10 @@ def emit_class_file(cls, outdir):
     w('template <> struct StageBra<%d, %d, %d, %d> { static constexpr bool value = %s; };'
       % (cls + ('true' if cls in STAGE_BRA else 'false',)))
     for gen in (0, 1):
-        w('template <> struct RowStore<%d, %d, %d, %d, %s> { static constexpr int acc = %d, dc = %d; '
-          'static constexpr bool stream = %s; };'
-          % (cls + ('true' if gen else 'false',) + row_store(cls, gen) +
-             ('true' if row_store(cls, gen)[0] == 0 and not gen and cls not in ROW_ARRAY else 'false',)))
+        sums = row_sums(cls, gen)
+        stream = not sums and not gen and cls not in ROW_ARRAY
+        w('template <> struct RowStore<%d, %d, %d, %d, %s> { static constexpr bool sums = %s, d_registers = %s, '
+          'stream = %s; };' % (cls + tuple('true' if x else 'false' for x in (gen, sums, sums and not gen and cls in ROW_D_REGISTERS, stream))))
     w(g.emit(parts=class_parts(cls)))
     w('}  // namespace vlx')
     write_if_changed(outdir / ('class_%s.inc' % nm), '\n'.join(body) + '\n')
@@ -756,24 +756,19 @@ BLOCKS_HINT = ({}, {}, PAIRS_BLOCKS, PAIRS_BLOCKS)
 STAGE_BRA = {(0, 0, 0, 0), (0, 1, 0, 0), (1, 1, 0, 0), (0, 2, 0, 0), (2, 2, 1, 2)}
 
 
-# Where the row-item kernels keep an item's accumulators and elements of D
-# (RowStore in vlx_kernels.cuh) for the classes that differ from row_store's
-# rule: class -> (acc, dc), for symmetric and general densities.  The rule, both
-# in shared memory up to 39 elements (two blocks of 80 KB per SM), is from
-# timings of the s, p and d classes on the (H2O)32 / def2-SVP build: registers
-# instead 35.7 ms, accumulators only 38.0, neither 49, both 34.2; classes of more
-# elements lose more to the smaller L1 than they gain, and (pd|pp) is fastest
-# with D in registers (2.35 against 2.49 ms).  Register caps (BLOCKS_HINT) were
-# slower for every class.
-ROW_STORE = ({(1, 2, 1, 1): (2, 1)}, {})
+# Row-item kernels keep an item's accumulators and elements of D in shared memory
+# up to 39 elements a lane (two blocks of 80 KB per SM), from timings of the s, p
+# and d classes on the (H2O)32 / def2-SVP build: registers instead 35.7 ms,
+# accumulators only 38.0, neither 49, both 34.2; classes of more elements lose more
+# to the smaller L1 than they gain, and (pd|pp) is fastest with D in registers
+# (2.35 against 2.49 ms).  Register caps (BLOCKS_HINT) were slower for every class.
+ROW_D_REGISTERS = {(1, 2, 1, 1)}
+ROW_ELEMENTS = 39
 
 
-def row_store(cls, gen):
-    if tuple(cls) in ROW_STORE[gen]:
-        return ROW_STORE[gen][tuple(cls)]
+def row_sums(cls, gen):
     nb, nc, nd = (2 * l + 1 for l in cls[1:])
-    n = nb * (nc + nd) * (2 if gen else 1) + nc * nd
-    return (2, 2) if n <= 39 else (0, 0)
+    return nb * (nc + nd) * (2 if gen else 1) + nc * nd <= ROW_ELEMENTS
 
 
 # Classes whose row-item kernel (symmetric density) keeps the block of integrals

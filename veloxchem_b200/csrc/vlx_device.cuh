@@ -1,9 +1,10 @@
 // Device-side building blocks of the B200 four-centre Fock build:
-//   * SoA shell-pair views (bra: warp-uniform, ket: one pair per lane),
-//   * the FP64 Boys function from a Chebyshev table,
-//   * J/K digestion of one spherical shell quartet into an FP64 accumulator,
-//   * the persistent work-queue kernels (Fock, ERI tensor, Schwarz diagonal).
-// The per-class recursions (EriClass<la,lb,lc,ld>) are generated by gen_eri.py.
+//   * shell-pair views (ket: one pair per lane; bra: warp-uniform, from the
+//     ket's layout, staged in shared memory, or in row order),
+//   * the FP64 and FP32 Boys functions from Chebyshev tables,
+//   * the ket range of a pair item and the per-quartet density test.
+// The digestion and the work-queue kernels are in vlx_kernels.cuh, the per-class
+// recursions (EriClass<la,lb,lc,ld>) are generated by gen_eri.py.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -229,8 +229,10 @@ __device__ __forceinline__ void digest(const double* f, const double s, const in
 // Layout of both: [QR: NB NC | QS: NB ND | RS: NC ND], and for a general
 // density (GEN) the transposes of the first two [RQ | SQ] behind; RS then
 // stands for both orientations (D_RS + D_SR, equal additions).
-// AS, DS: element stride (1: registers, 32: the lane's column of a per-warp
-// shared-memory array; DS 0: no copy, read from D).
+// acc is the lane's column of a per-warp shared-memory array (element stride
+// kColumn), dc another or, with DS = 1 for its stride, registers.
+constexpr int kColumn = 32;
+
 template <int NB, int NC, int ND, bool GEN>
 struct RowLayout {
     static constexpr int QS = NB * NC, RS = QS + NB * ND, T = RS + NC * ND, N = GEN ? T + RS : T;
@@ -261,7 +263,7 @@ struct QuartetAO {
 };
 
 // Exchange part of one step; TR: the transposed elements of a general density.
-template <int NA, int NB, int NC, int ND, bool TR, int AS, int DS>
+template <int NA, int NB, int NC, int ND, bool TR, int DS>
 __device__ __forceinline__ void digest_row_k(const double* f, const double ck, const QuartetAO& o, const MolDev& m,
                                              double* acc, const double* dc)
 {
@@ -277,12 +279,12 @@ __device__ __forceinline__ void digest_row_k(const double* f, const double ck, c
         for (int j = 0; j < NB; j++)
 #pragma unroll
             for (int k = 0; k < NC; k++) {
-                double x = acc[AS * (base + j * NC + k)];
+                double x = acc[kColumn * (base + j * NC + k)];
 #pragma unroll
                 for (int i = 0; i < NA; i++)
 #pragma unroll
                     for (int l = 0; l < ND; l++) x = fma(f[((i * NB + j) * NC + k) * ND + l], d[i * ND + l], x);
-                acc[AS * (base + j * NC + k)] = x;
+                acc[kColumn * (base + j * NC + k)] = x;
             }
     }
     {
@@ -295,12 +297,12 @@ __device__ __forceinline__ void digest_row_k(const double* f, const double ck, c
         for (int j = 0; j < NB; j++)
 #pragma unroll
             for (int l = 0; l < ND; l++) {
-                double x = acc[AS * (base + L::QS + j * ND + l)];
+                double x = acc[kColumn * (base + L::QS + j * ND + l)];
 #pragma unroll
                 for (int i = 0; i < NA; i++)
 #pragma unroll
                     for (int k = 0; k < NC; k++) x = fma(f[((i * NB + j) * NC + k) * ND + l], d[i * NC + k], x);
-                acc[AS * (base + L::QS + j * ND + l)] = x;
+                acc[kColumn * (base + L::QS + j * ND + l)] = x;
             }
     }
     {
@@ -311,7 +313,7 @@ __device__ __forceinline__ void digest_row_k(const double* f, const double ck, c
         for (int j = 0; j < NB; j++)
 #pragma unroll
             for (int l = 0; l < ND; l++) {
-                const double d = DS ? dc[DS * (base + L::QS + j * ND + l)] : ldT<TR>(m, o.q(j), o.s(l));
+                const double d = dc[DS * (base + L::QS + j * ND + l)];
 #pragma unroll
                 for (int i = 0; i < NA; i++)
 #pragma unroll
@@ -333,7 +335,7 @@ __device__ __forceinline__ void digest_row_k(const double* f, const double ck, c
         for (int j = 0; j < NB; j++)
 #pragma unroll
             for (int k = 0; k < NC; k++) {
-                const double d = DS ? dc[DS * (base + j * NC + k)] : ldT<TR>(m, o.q(j), o.r(k));
+                const double d = dc[DS * (base + j * NC + k)];
 #pragma unroll
                 for (int i = 0; i < NA; i++)
 #pragma unroll
@@ -350,7 +352,7 @@ __device__ __forceinline__ void digest_row_k(const double* f, const double ck, c
 }
 
 // s: the permutational weight of the lane's quartet, 0 on an idle lane.
-template <int NA, int NB, int NC, int ND, bool GEN, int AS, int DS>
+template <int NA, int NB, int NC, int ND, bool GEN, int DS>
 __device__ __forceinline__ void digest_row(const double* f, const double s, const int lane, const QuartetAO& o,
                                            const MolDev& m, const double cjw, const double ckw, double* acc,
                                            const double* dc)
@@ -362,11 +364,7 @@ __device__ __forceinline__ void digest_row(const double* f, const double s, cons
 #pragma unroll
         for (int k = 0; k < NC; k++)
 #pragma unroll
-            for (int l = 0; l < ND; l++) {
-                double x = DS ? dc[DS * (L::RS + k * ND + l)] : ldD(m.D, m.nao, o.r(k), o.s(l));
-                if (GEN && !DS) x += ldD(m.D, m.nao, o.s(l), o.r(k));
-                d[k * ND + l] = cj * x;
-            }
+            for (int l = 0; l < ND; l++) d[k * ND + l] = cj * dc[DS * (L::RS + k * ND + l)];
         // F_PQ: chunks of up to 32 elements, each reduced over the lanes
         constexpr int NPQ = NA * NB, NCH = (NPQ + 31) / 32, CH = (NPQ + NCH - 1) / NCH;
 #pragma unroll
@@ -397,15 +395,15 @@ __device__ __forceinline__ void digest_row(const double* f, const double s, cons
             }
 #pragma unroll
         for (int kl = 0; kl < NC * ND; kl++) {
-            double x = acc[AS * (L::RS + kl)];
+            double x = acc[kColumn * (L::RS + kl)];
 #pragma unroll
             for (int ij = 0; ij < NA * NB; ij++) x = fma(f[ij * NC * ND + kl], d[ij], x);
-            acc[AS * (L::RS + kl)] = x;
+            acc[kColumn * (L::RS + kl)] = x;
         }
     }
     if (ckw != 0.0) {
-        digest_row_k<NA, NB, NC, ND, false, AS, DS>(f, ckw * s, o, m, acc, dc);
-        if (GEN) digest_row_k<NA, NB, NC, ND, true, AS, DS>(f, ckw * s, o, m, acc, dc);
+        digest_row_k<NA, NB, NC, ND, false, DS>(f, ckw * s, o, m, acc, dc);
+        if (GEN) digest_row_k<NA, NB, NC, ND, true, DS>(f, ckw * s, o, m, acc, dc);
     }
 }
 
@@ -425,33 +423,31 @@ __device__ __forceinline__ void read_row_k(const QuartetAO& o, const MolDev& m, 
     }
 }
 
-template <int NB, int NC, int ND, bool GEN, int AS, int DS>
+template <int NB, int NC, int ND, bool GEN, int DS>
 __device__ __forceinline__ void begin_row(const QuartetAO& o, const MolDev& m, const double cj, const double ck,
                                           double* acc, double* dc)
 {
     using L = RowLayout<NB, NC, ND, GEN>;
 #pragma unroll
-    for (int e = 0; e < L::N; e++) acc[AS * e] = 0.0;
-    if constexpr (DS != 0) {
-        if (ck != 0.0) {
-            read_row_k<NB, NC, ND, false, DS>(o, m, dc);
-            if (GEN) read_row_k<NB, NC, ND, true, DS>(o, m, dc);
-        }
-        if (cj != 0.0) {
+    for (int e = 0; e < L::N; e++) acc[kColumn * e] = 0.0;
+    if (ck != 0.0) {
+        read_row_k<NB, NC, ND, false, DS>(o, m, dc);
+        if (GEN) read_row_k<NB, NC, ND, true, DS>(o, m, dc);
+    }
+    if (cj != 0.0) {
 #pragma unroll
-            for (int k = 0; k < NC; k++)
+        for (int k = 0; k < NC; k++)
 #pragma unroll
-                for (int l = 0; l < ND; l++) {
-                    double x = ldD(m.D, m.nao, o.r(k), o.s(l));
-                    if (GEN) x += ldD(m.D, m.nao, o.s(l), o.r(k));
-                    dc[DS * (L::RS + k * ND + l)] = x;
-                }
-        }
+            for (int l = 0; l < ND; l++) {
+                double x = ldD(m.D, m.nao, o.r(k), o.s(l));
+                if (GEN) x += ldD(m.D, m.nao, o.s(l), o.r(k));
+                dc[DS * (L::RS + k * ND + l)] = x;
+            }
     }
 }
 
 // End of a row item: the lane's accumulators into F.
-template <int NB, int NC, int ND, bool TR, int AS>
+template <int NB, int NC, int ND, bool TR>
 __device__ __forceinline__ void flush_row_k(const QuartetAO& o, const MolDev& m, const double* acc)
 {
     using L = RowLayout<NB, NC, ND, TR>;
@@ -459,27 +455,27 @@ __device__ __forceinline__ void flush_row_k(const QuartetAO& o, const MolDev& m,
 #pragma unroll
     for (int j = 0; j < NB; j++) {
 #pragma unroll
-        for (int k = 0; k < NC; k++) addT<TR>(m, o.q(j), o.r(k), acc[AS * (base + j * NC + k)]);
+        for (int k = 0; k < NC; k++) addT<TR>(m, o.q(j), o.r(k), acc[kColumn * (base + j * NC + k)]);
 #pragma unroll
-        for (int l = 0; l < ND; l++) addT<TR>(m, o.q(j), o.s(l), acc[AS * (base + L::QS + j * ND + l)]);
+        for (int l = 0; l < ND; l++) addT<TR>(m, o.q(j), o.s(l), acc[kColumn * (base + L::QS + j * ND + l)]);
     }
 }
 
-template <int NB, int NC, int ND, bool GEN, int AS>
+template <int NB, int NC, int ND, bool GEN>
 __device__ __forceinline__ void flush_row(const QuartetAO& o, const MolDev& m, const double cj, const double ck,
                                           const double* acc)
 {
     using L = RowLayout<NB, NC, ND, GEN>;
     if (ck != 0.0) {
-        flush_row_k<NB, NC, ND, false, AS>(o, m, acc);
-        if (GEN) flush_row_k<NB, NC, ND, true, AS>(o, m, acc);
+        flush_row_k<NB, NC, ND, false>(o, m, acc);
+        if (GEN) flush_row_k<NB, NC, ND, true>(o, m, acc);
     }
     if (cj != 0.0) {
 #pragma unroll
         for (int k = 0; k < NC; k++)
 #pragma unroll
             for (int l = 0; l < ND; l++) {
-                const double v = acc[AS * (L::RS + k * ND + l)];
+                const double v = acc[kColumn * (L::RS + k * ND + l)];
                 addF(m.F, m.nao, o.r(k), o.s(l), v);
                 if (GEN) addF(m.F, m.nao, o.s(l), o.r(k), v);
             }
@@ -514,16 +510,16 @@ __device__ __forceinline__ void scatter_eri(const double* f, const int p0, const
 constexpr int kWarpsPerBlock = 4;
 
 // Per-class tuning traits, specialised in each class's generated unit from the
-// tables of gen_eri.py (BLOCKS_HINT, STAGE_BRA, ROW_STORE), so that tuning one
+// tables of gen_eri.py (BLOCKS_HINT, STAGE_BRA, row_sums), so that tuning one
 // class recompiles only that unit:
 //   BlocksHint::value  minimum resident 128-thread blocks per SM the register
 //                      allocation of a kernel variant must allow (0: no minimum);
 //   StageBra::value    the pair-item kernel stages the bra primitive records
 //                      in shared memory per work item (PairViewS);
-//   RowStore::acc, ::dc where the row-item kernels keep an item's accumulators
-//                      and elements of D (digest_row): 1 registers, 2 a
-//                      per-warp shared-memory array, 0 nowhere (acc 0: every
-//                      step is digested by itself; dc 0: read from D);
+//   RowStore::sums     the row-item kernels keep an item's accumulators and
+//                      elements of D in per-warp shared-memory arrays
+//                      (digest_row), ::d_registers the latter in registers;
+//                      without sums every step is digested by itself;
 //   RowStore::stream   a step's integrals go through StreamSink.
 template <int LA, int LB, int LC, int LD, int V>
 struct BlocksHint;
@@ -869,7 +865,8 @@ constexpr int row_shared_bytes()
 {
     using Store = RowStore<LA, LB, LC, LD, GEN>;
     return (boys_stride<R> * (int)sizeof(R) + 15) / 16 * 16 +
-           ((Store::acc == 2) + (Store::dc == 2)) * kWarpsPerBlock * 32 * row_elements<LA, LB, LC, LD, GEN> * 8;
+           (Store::sums + (Store::sums && !Store::d_registers)) * kWarpsPerBlock * kColumn *
+               row_elements<LA, LB, LC, LD, GEN> * 8;
 }
 
 template <int LA, int LB, int LC, int LD, bool GEN, typename R>
@@ -879,22 +876,21 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
     using Store = RowStore<LA, LB, LC, LD, GEN>;
     constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1, NC = 2 * LC + 1, ND = 2 * LD + 1;
     constexpr int NROW = row_elements<LA, LB, LC, LD, GEN>;
-    constexpr int AS = Store::acc == 2 ? 32 : 1, DS = Store::dc == 2 ? 32 : (Store::dc == 1 ? 1 : 0);
+    constexpr int DS = Store::d_registers ? 1 : kColumn;
     constexpr bool f32 = sizeof(R) == sizeof(float);
     // the straight-line code of a step of the large classes (up to hundreds of
     // KB) does not fit the instruction caches, least of all beside other
     // classes' kernels: the warps of a block walk their items in step, so that it
     // is fetched once for all of them ((H2O)27 / def2-TZVP build 236 -> 228 ms;
     // each class by itself 3% slower to 18% faster)
-    constexpr bool LOCK = Store::acc == 0;
+    constexpr bool LOCK = !Store::sums;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     extern __shared__ __align__(16) char shared[];
     R* sboys = reinterpret_cast<R*>(shared);
     double* sacc = reinterpret_cast<double*>(shared + (boys_stride<R> * (int)sizeof(R) + 15) / 16 * 16);
-    double* sdc = sacc + (Store::acc == 2 ? kWarpsPerBlock * 32 * NROW : 0);
-    double racc[Store::acc == 1 ? NROW : 1], rdc[Store::dc == 1 ? NROW : 1];
-    double* acc = Store::acc == 2 ? sacc + warp * (32 * NROW) + lane : racc;
-    double* dc = Store::dc == 2 ? sdc + warp * (32 * NROW) + lane : rdc;
+    double* acc = sacc + warp * (kColumn * NROW) + lane;
+    double rdc[Store::d_registers ? NROW : 1];
+    double* dc = Store::d_registers ? rdc : acc + kWarpsPerBlock * kColumn * NROW;
     stage_boys<LA + LB + LC + LD>(a, sboys);
 #pragma unroll 1
     for (;;) {
@@ -942,7 +938,7 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
         o.s0 = __ldg(kb.ao + kb.npairs + jj);
         const double s_ket = (o.r0 == o.s0) ? 0.5 : 1.0;
         const PairViewT<R> ket = make_view(kb, jj, __ldg(kb.nuse + jj), R());
-        if constexpr (Store::acc != 0) begin_row<NB, NC, ND, GEN, AS, DS>(o, m, a.cj, a.ck, acc, dc);
+        if constexpr (Store::sums) begin_row<NB, NC, ND, GEN, DS>(o, m, a.cj, a.ck, acc, dc);
         bool any = false;
 #pragma unroll 1
         for (int x = 0; x < steps; x++) {
@@ -987,15 +983,15 @@ __device__ __forceinline__ void row_body(const FockArgs& a)
                 double f[C::NSPH];
 #pragma unroll
                 for (int t = 0; t < C::NSPH; t++) f[t] = (double)g[t];
-                if constexpr (Store::acc != 0)
-                    digest_row<NA, NB, NC, ND, GEN, AS, DS>(f, s, lane, o, m, a.cj, a.ck, acc, dc);
+                if constexpr (Store::sums)
+                    digest_row<NA, NB, NC, ND, GEN, DS>(f, s, lane, o, m, a.cj, a.ck, acc, dc);
                 else
                     digest<NA, NB, NC, ND, GEN ? MODE_FOCK_GEN : MODE_FOCK_SYM>(
                         f, s, lane, o.p0, o.nlp, o.q0, o.nlq, o.r0, o.nlr, o.s0, o.nls, m, a.cj, a.ck);
             }
         }
-        if constexpr (Store::acc != 0) {
-            if (any) flush_row<NB, NC, ND, GEN, AS>(o, m, a.cj, a.ck, acc);
+        if constexpr (Store::sums) {
+            if (any) flush_row<NB, NC, ND, GEN>(o, m, a.cj, a.ck, acc);
         }
     }
 }

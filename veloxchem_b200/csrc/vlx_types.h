@@ -103,7 +103,7 @@ struct FockArgs {
     int nitems;
     int* counter;             // work-queue head for this launch (zeroed before)
     const double* boys;       // Chebyshev table
-    const float* boys_f;      // the same table rounded to float (mixed precision)
+    const float* boys_f;      // the table of the FP32 kernels (BOYS_NCOEF_F coefficients)
     MolDev mol;               // the molecule of a single build
     const MolDev* mols;       // batched build: per molecule, indexed by PairBlockDev::mol (nullptr: single)
     double* eri;              // MODE_ERI: nao^4 tensor of mol
