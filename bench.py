@@ -127,12 +127,13 @@ class ClockSampler:
 
 
 def _profiled_traffic(cls):
-    """DRAM bytes per launch of a class kernel from its committed ncu summary
-    (profiles/quartet_kernel_<class>_h2o32_svp.md), or None."""
+    """DRAM bytes per launch of a class's plain FP64 kernel (row items, symmetric
+    density) from the committed ncu summary of that kernel
+    (profiles/rows_sym_<class>_h2o32_svp.md), or None."""
     import re
     name = '%d%d%d%d' % (cls['la'], cls['lb'], cls['lc'], cls['ld'])
-    path = ROOT / 'profiles' / ('quartet_kernel_%s_h2o32_svp.md' % name)
-    if not path.exists():
+    path = ROOT / 'profiles' / ('rows_sym_%s_h2o32_svp.md' % name)
+    if cls['table_driven'] or not path.exists():
         return None
     m = re.search(r'dram_bytes_per_launch:\s*(\d+)', path.read_text())
     return int(m.group(1)) if m else None
@@ -275,7 +276,7 @@ def run_ours(args):
                 'traffic_source': 'dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this kernel '
                                   'on this workload, summarised under profiles/ (null: no capture of this kernel)',
                 'kernel': ('coop_quartet_kernel<double,%d,%d,%d,%d>' if top['table_driven'] else
-                           'quartet_kernel<%d,%d,%d,%d>') % (top['la'], top['lb'], top['lc'], top['ld']),
+                           'quartet_kernel<%d,%d,%d,%d,ROWS_SYM,double>') % (top['la'], top['lb'], top['lc'], top['ld']),
                 'kernel_share': top['device_ms'] / tot_prof_ms,
                 'peak_source': 'measured: FP64 FMA-chain probe kernel (vlx_b200_fp64_peak), burst; '
                                'MEASURED_PEAKS.json has no FP64 figure',
