@@ -690,7 +690,7 @@ def emit_class_file(cls, outdir):
       % (cls + ('true' if cls in STAGE_BRA else 'false',)))
     for gen in (0, 1):
         sums = row_sums(cls, gen)
-        stream = not sums and not gen and cls not in ROW_ARRAY
+        stream = not sums and not gen and not row_array(cls)
         w('template <> struct RowStore<%d, %d, %d, %d, %s> { static constexpr bool sums = %s, d_registers = %s, '
           'stream = %s; };' % (cls + tuple('true' if x else 'false' for x in (gen, sums, sums and not gen and cls in ROW_D_REGISTERS, stream))))
     w(g.emit(parts=class_parts(cls)))
@@ -762,6 +762,11 @@ STAGE_BRA = {(0, 0, 0, 0), (0, 1, 0, 0), (1, 1, 0, 0), (0, 2, 0, 0), (2, 2, 1, 2
 # accumulators only 38.0, neither 49, both 34.2; classes of more elements lose more
 # to the smaller L1 than they gain, and (pd|pp) is fastest with D in registers
 # (2.35 against 2.49 ms).  Register caps (BLOCKS_HINT) were slower for every class.
+# The f classes: up to 51 elements for symmetric densities 228.5 -> 230.2 ms on the
+# (H2O)27 / def2-TZVP build.  General densities: up to 27 elements 18.5 -> 18.8 ms for
+# (H2O)8 / def2-TZVP, up to 51 (which adds the (X|sd) and (pp|pp) classes of 43 and
+# 45) 17.7, and 4.00 -> 3.85 ms for k_rs of (H2O)11 / def2-SVP: their line could lie
+# higher.
 ROW_D_REGISTERS = {(1, 2, 1, 1)}
 ROW_ELEMENTS = 39
 
@@ -771,11 +776,16 @@ def row_sums(cls, gen):
     return nb * (nc + nd) * (2 if gen else 1) + nc * nd <= ROW_ELEMENTS
 
 
-# Classes whose row-item kernel (symmetric density) keeps the block of integrals
-# of a step in an array although it has no row accumulators: measured faster
-# than streaming the block through the digestion (StreamSink) on the
-# (H2O)27 / def2-TZVP build, by 3 to 20%.
-ROW_ARRAY = {(0, 3, 1, 1), (0, 3, 1, 2), (1, 3, 1, 1), (0, 3, 0, 2), (0, 3, 0, 3), (1, 3, 0, 2)}
+# Whether the row-item kernel (symmetric density) of a class without row sums keeps
+# the block of integrals of a step in an array instead of streaming it through the
+# digestion (StreamSink): where both the block and the sink's own running sums are
+# few.  Each class measured by itself on the (H2O)27 / def2-TZVP build: the array
+# is faster by 3 to 20% for the classes below the line ((sf|pp) 63 and 39 values
+# to (pf|pp) 189 and 61, (pf|sd) 105 and 81), streaming for those above
+# ((pf|sf) 147 and 101, (df|sd) 175 and 107, (pd|pd) 225 and 63 and larger).
+def row_array(cls):
+    na, nb, nc, nd = (2 * l + 1 for l in cls)
+    return na * nb * nc * nd <= 190 and na * nb + na + nb + (na + nb) * nd <= 81
 
 
 def class_parts(cls):

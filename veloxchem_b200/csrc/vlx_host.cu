@@ -3,15 +3,18 @@
 //  * shells, GTO blocks (l, nprim) and pair blocks in the reference order
 //    (src/orbdata/GtoFunc.cpp:9-18, GtoPairBlockFunc.cpp:16-43,
 //    GtoPairBlock.cpp:49-305);
-//  * per-pair primitive data as SoA device arrays [field][prim][pair];
+//  * per-pair primitive data in tiles of 32 pairs (ket side, bin order) and in row
+//    order (bra side of the row items), in FP64 and FP32;
 //  * Schwarz diagonals on the GPU, decade bins as in
 //    src/orbdata/BlockedGtoPairBlock.cpp:22-42, pairs re-sorted by bin so the
 //    kets admitted for a bra of bin b are a prefix of the ket block;
-//  * work items (bra pair x run of ket pairs) per quartet class, the selection
-//    rule of src/general/OpenMPFunc.cpp:121-259 (bin_bra + bin_ket <= ithreshold,
+//  * work items per quartet class (rows of bra pairs x 32 ket pairs, or a bra pair
+//    x a run of ket pairs), the selection rule of
+//    src/general/OpenMPFunc.cpp:121-259 (bin_bra + bin_ket <= ithreshold,
 //    each unordered pair of pairs once), dealt round-robin over ranks like
 //    omp::partition_tasks (src/general/OpenMPFunc.hpp:89-112);
-//  * one persistent launch per quartet class with a work-queue head, then
+//  * one persistent launch per quartet class and precision with a work-queue head,
+//    beside each other on side streams of the device, then
 //    F = acc + acc^T for symmetric densities (src/math/Matrix.cpp:189-197).
 #include <cuda_runtime.h>
 
@@ -614,9 +617,16 @@ int pair_key(int la, int lb) { return (la + lb) * 16 + lb; }
 constexpr int kCoopSegment = 2;
 
 // Steps (bra pairs against 32 kets) of a row item per ket pair of the
-// work-item length: the default length of 256 ket pairs allows rows of 32.
+// work-item length: the default length of 256 ket pairs allows rows of 32.  Rows
+// of 128 / 64 / 32 / 16: (H2O)32 def2-SVP 28.6 / 28.4 / 28.2 / 28.0 ms, (H2O)27 def2-TZVP
+// 228.5 / 228.1 / 226.8 / 229.1.
 constexpr int kRowShare = 8;
-// Row items per SM that a class is cut into at least, where it has the steps.
+// Row items per SM that a class is cut into at least, where it has the steps:
+// fewer leave SMs idle at the end of a class, more give up the sums and reads that
+// the steps of an item share.  16 / 32 / 64 / 128 / 256: (H2O)8 def2-TZVP 12.5 / 12.6 /
+// 13.0 / 13.7 / 15.0 ms, J (H2O)13 def2-SVP 3.38 / 3.30 / 3.27 / 3.03 / 3.01, k_rs (H2O)11
+// 3.91 / 3.94 / 4.03 / 4.35 / 4.80, (H2O)32 28.7 / 28.3 / 28.2 / 28.4 / 30.1, (H2O)27
+// def2-TZVP 240 / 233 / 226.8 / 224.8 / 227.9, 48 clusters 77.4 / 77.0 / 76.6 / 75.5 / 74.6.
 constexpr int kRowSpread = 64;
 
 }  // namespace
@@ -1181,7 +1191,6 @@ int build_tasks(vlx_b200_screener* s, int ith_req, int rank, int nodes, bool ext
         all.reserve(total);
         for (auto& ct : ts.classes) {
             all.insert(all.end(), ct.items.begin(), ct.items.end());
-
         }
         VLX_CUDA(cudaMalloc(&ts.d_items, total * sizeof(WorkItem)));
         VLX_CUDA(copy_to_device(ts.d_items, all.data(), total * sizeof(WorkItem)));
@@ -2707,7 +2716,6 @@ int batch_tasks(vlx_b200_batch* b, int ith, TaskSet** out)
         all.reserve(total);
         for (auto& ct : m.classes) {
             all.insert(all.end(), ct.items.begin(), ct.items.end());
-
         }
         VLX_CUDA(cudaMalloc(&m.d_items, total * sizeof(WorkItem)));
         VLX_CUDA(copy_to_device(m.d_items, all.data(), total * sizeof(WorkItem)));
